@@ -59,6 +59,14 @@ cudaError_t configure_misc()
 
 void launch_init64(const Launch &L, cudaStream_t st) { init64_kernel<<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); }
 
+void launch_bnd(bool f32, const Job *jobs, const int (&job)[3], int count, cudaStream_t st)
+{
+    if (count < 1) return;
+    const dim3 grid(NBND / 256, (unsigned)count);
+    if (f32) bnd_kernel<float><<<grid, 256, 0, st>>>(jobs, job[0], job[1], job[2]);
+    else bnd_kernel<double><<<grid, 256, 0, st>>>(jobs, job[0], job[1], job[2]);
+}
+
 void launch_code(const Launch &L, cudaStream_t st) { code_kernel<<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); }
 
 void launch_tau(int src, const Launch &L, cudaStream_t st)

@@ -84,6 +84,7 @@ struct Ctx {
     int kMax = 0;
     Scalars *d_slots = nullptr;
     uint32_t *d_cnt = nullptr;
+    char *d_bnd = nullptr;          // domain-face tables of the three primary axes
     Scalars *h_snap[2] = {};        // pinned copies of the slot array, one per chunk in flight
     Scalars *h_init = nullptr;      // pinned staging of new solves' scalars
     Job *h_stage = nullptr;         // pinned staging of job tables (5 regions of kMax)
@@ -247,7 +248,7 @@ int admit(Ctx &C)
         SV(cudaMemcpyAsync(d_mask, A.req.mask.data(), n, cudaMemcpyHostToDevice, C.st));
         Scalars &S0 = C.h_init[fresh.size()];
         int s = build_job(A.job, S0, d_mask, A.req.nx, A.req.ny, A.req.nz, A.req.dir, d_code, C.d_slots + A.slot,
-                          C.d_cnt + A.slot, M, P);
+                          C.d_cnt + A.slot, C.d_bnd + (A.req.dir >> 1) * bnd_bytes(P.precision), M, P);
         if (s != FAST_OK) {
             cudaFreeAsync(A.arena, C.st);
             C.free_slots.push_back(A.slot);
@@ -394,6 +395,7 @@ void destroy(Ctx *C)
         if (d) cudaFreeAsync(d, C->st);
     if (C->d_slots) cudaFreeAsync(C->d_slots, C->st);
     if (C->d_cnt) cudaFreeAsync(C->d_cnt, C->st);
+    if (C->d_bnd) cudaFreeAsync(C->d_bnd, C->st);
     if (C->st) cudaStreamSynchronize(C->st);
     for (Scalars *h : C->h_snap)
         if (h) cudaFreeHost(h);
@@ -448,7 +450,8 @@ int create(const fast_ctx_config &cfg, Ctx **out)
         cudaMallocAsync((void **)&C->d_tmp[1], sizeof(Job) * K, C->st) != cudaSuccess ||
         cudaMallocAsync((void **)&C->d_tmp[2], sizeof(Job) * K, C->st) != cudaSuccess ||
         cudaMallocAsync((void **)&C->groups[0].d_gate, sizeof(uint32_t), C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->groups[1].d_gate, sizeof(uint32_t), C->st) != cudaSuccess)
+        cudaMallocAsync((void **)&C->groups[1].d_gate, sizeof(uint32_t), C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_bnd, 3 * bnd_bytes(cfg.precision), C->st) != cudaSuccess)
         return fin(ft_fail(FAST_NOMEM, "context tables"));
     if (cudaMemsetAsync(C->d_cnt, 0, sizeof(uint32_t) * K, C->st) != cudaSuccess ||
         cudaMemsetAsync(C->groups[0].d_gate, 0, sizeof(uint32_t), C->st) != cudaSuccess ||
@@ -458,6 +461,19 @@ int create(const fast_ctx_config &cfg, Ctx **out)
         cudaMallocHost(&C->h_init, sizeof(Scalars) * K) != cudaSuccess ||
         cudaMallocHost(&C->h_stage, sizeof(Job) * 6 * K) != cudaSuccess)
         return fin(ft_fail(FAST_NOMEM, "context staging"));
+    // The domain-face tables depend on the context's coefficients alone.
+    for (int a = 0; a < 3; a++) {
+        Job &J = C->h_stage[a];
+        memset(&J, 0, sizeof(J));
+        J.dir = 2 * a;
+        J.bnd = C->d_bnd + a * bnd_bytes(cfg.precision);
+        job_coefficients(J, C->P[0]);
+        if (cudaMemcpyAsync(C->d_tmp[a], &J, sizeof(Job), cudaMemcpyHostToDevice, C->st) != cudaSuccess)
+            return fin(ft_fail(FAST_CUDA_ERROR, "context setup"));
+        const int first[3] = {0, 0, 0};
+        launch_bnd(cfg.precision == FAST_PREC_F32, C->d_tmp[a], first, 1, C->st);
+    }
+    if (cudaGetLastError() != cudaSuccess) return fin(ft_fail(FAST_CUDA_ERROR, "context setup"));
     if (cudaStreamSynchronize(C->st) != cudaSuccess) return fin(ft_fail(FAST_CUDA_ERROR, "context setup"));
     for (int k = K - 1; k >= 0; k--) C->free_slots.push_back(k);
     *out = C;

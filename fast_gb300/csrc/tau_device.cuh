@@ -27,9 +27,11 @@ namespace ft {
 // Dirichlet face must double (-D_self: 2*D_self in all).  The count is fixed
 // per thread in x and y for a whole slab and changes only on the first and
 // last plane in z, so the lookup has no branch.  FP64 solves and the
-// reference's FP32 mode keep the coordinate-aware evaluation in the
-// reference's subtraction order for voxels on a domain face (row 2 of the FP32
-// table is the interior diagonal they use).
+// reference's FP32 mode need a domain-face voxel's diagonal in the
+// reference's subtraction order: they read it from a table in global memory
+// (Job::bnd) that bnd_kernel fills once per solve with diag_general, by the
+// voxel's missing neighbours and code (row 2 of the FP32 table is the
+// interior diagonal they use).
 // ---------------------------------------------------------------------------
 constexpr int NBC = 7;  // boundary counts -2..4
 
@@ -72,6 +74,7 @@ struct FF {
 template <typename T>
 struct Coef {
     static constexpr int NB = sizeof(T) == 4 ? NBC : 1;
+    const double2 *bnd;  // Job::bnd
     T face[2][2];      // face coefficient by (self solid, neighbour solid)
     T cell2[2];        // 2*D: the half-cell Dirichlet face (dist = h/2)
     T diag_b[NB][128]; // diagonal by (boundary count + 2, code); FP64: interior row only
@@ -87,6 +90,7 @@ struct Coef {
 template <>
 struct Coef<float> {
     static constexpr int NB = NBC;
+    const float2 *bnd;  // Job::bnd
     float face[2][2];
     float cell2[2];
     float2 di[NBC][128];  // {diag, 1/diag} by (boundary count + 2, code)
@@ -115,6 +119,7 @@ __device__ __forceinline__ void load_face_table(FaceTable &t, const Job &J, int 
 template <typename T>
 __device__ __forceinline__ void load_coef(Coef<T> &C, const Job &J, int tid, int nt = NTHREADS)
 {
+    if (tid == 0) C.bnd = static_cast<decltype(C.bnd)>(J.bnd);
     if constexpr (sizeof(T) == 8) {
         if (tid < 128) {
             C.diag_b[0][tid] = J.ddiag_int[tid];
@@ -228,11 +233,24 @@ __device__ __forceinline__ T diag_general(const Coef<T> &C, const Geo &g, uint32
     return d;
 }
 
+// The missing neighbours of a voxel, bit d = neighbour d (Dir order) outside.
+__device__ __forceinline__ int missing_faces(const Geo &g, int x, int y, int z)
+{
+    return (x == g.nx - 1 ? 1 : 0) | (x == 0 ? 2 : 0) | (y == g.ny - 1 ? 4 : 0) | (y == 0 ? 8 : 0) |
+           (z == g.nz - 1 ? 16 : 0) | (z == 0 ? 32 : 0);
+}
+
+// {diagonal, 1/diagonal} of a voxel on a domain face.
+template <typename T>
+__device__ __forceinline__ auto bnd_entry(const Coef<T> &C, const Geo &g, uint32_t code, const Pos &p)
+{
+    return __ldg(C.bnd + missing_faces(g, p.x, p.y, p.z) * 128 + (code & 127));
+}
+
 // Diagonal and its inverse of the voxel at p.  FAST (the FP32 iterations of
 // a MIXED solve): the boundary-count table, no branch.  Otherwise (FP64 and
-// the reference's FP32 mode): the interior table, or the coordinate-aware
-// evaluation in the reference's subtraction order for a voxel on a domain
-// face (BND_BIT of its code).
+// the reference's FP32 mode): the interior table, or the domain-face table
+// (diag_general's values) for a voxel on a domain face (BND_BIT of its code).
 template <typename T>
 __host__ __device__ constexpr int interior_row() { return Coef<T>::NB == 1 ? 0 : 2; }
 
@@ -258,7 +276,7 @@ __device__ __forceinline__ T diag_of(const Coef<T> &C, const Geo &g, uint32_t co
     if constexpr (FAST) {
         return tab_diag(C, p.bc + 2, code);
     } else {
-        if (code & (1u << BND_BIT)) return diag_general(C, g, code, p.x, p.y, p.z);
+        if (code & (1u << BND_BIT)) return bnd_entry(C, g, code, p).x;
         return tab_diag(C, interior_row<T>(), code);
     }
 }
@@ -278,16 +296,10 @@ __device__ __forceinline__ float2 dinv_of(const Coef<float> &C, const Geo &g, ui
     if constexpr (FAST) {
         return C.di[p.bc + 2][code & 127];
     } else {
-        if (code & (1u << BND_BIT)) {
-            const float d = diag_general(C, g, code, p.x, p.y, p.z);
-            return make_float2(d, 1.0f / d);
-        }
+        if (code & (1u << BND_BIT)) return bnd_entry(C, g, code, p);
         return C.di[interior_row<float>()][code & 127];
     }
 }
-
-template <typename T, bool FAST>
-__device__ __forceinline__ T inv_from_diag(const Coef<T> &C, uint32_t code, const Pos &p, T d);
 
 template <typename T, bool FAST>
 __device__ __forceinline__ void diag_inv(const Coef<T> &C, const Geo &g, uint32_t code, const Pos &p, T &d, T &inv)
@@ -296,9 +308,13 @@ __device__ __forceinline__ void diag_inv(const Coef<T> &C, const Geo &g, uint32_
         const float2 di = dinv_of<FAST>(C, g, code, p);
         d = di.x;
         inv = di.y;
+    } else if (code & (1u << BND_BIT)) {
+        const double2 di = bnd_entry(C, g, code, p);
+        d = di.x;
+        inv = di.y;
     } else {
-        d = diag_of<T, FAST>(C, g, code, p);
-        inv = inv_from_diag<T, FAST>(C, code, p, d);
+        d = tab_diag(C, interior_row<T>(), code);
+        inv = tab_inv(C, interior_row<T>(), code);
     }
 }
 
@@ -308,19 +324,8 @@ __device__ __forceinline__ T inv_of(const Coef<T> &C, const Geo &g, uint32_t cod
     if constexpr (FAST) {
         return tab_inv(C, p.bc + 2, code);
     } else {
-        if (code & (1u << BND_BIT)) return T(1) / diag_general(C, g, code, p.x, p.y, p.z);
+        if (code & (1u << BND_BIT)) return bnd_entry(C, g, code, p).y;
         return tab_inv(C, interior_row<T>(), code);
-    }
-}
-
-// The inverse when the diagonal d of the voxel is already at hand.
-template <typename T, bool FAST>
-__device__ __forceinline__ T inv_from_diag(const Coef<T> &C, uint32_t code, const Pos &p, T d)
-{
-    if constexpr (FAST) {
-        return tab_inv(C, p.bc + 2, code);
-    } else {
-        return (code & (1u << BND_BIT)) ? T(1) / d : tab_inv(C, interior_row<T>(), code);
     }
 }
 

@@ -50,6 +50,8 @@ int64_t row_pitch(int64_t nx);
 // the volume's slab depth) and of a volume's stencil codes.
 size_t job_bytes(int64_t nx, int64_t ny, int64_t nz, int prec, int solver, int zc = 0);
 size_t code_bytes(int64_t nx, int64_t ny, int64_t nz);
+// Device bytes of a domain-face table (Job::bnd).
+size_t bnd_bytes(int prec);
 
 // Bump allocator over one device allocation.
 struct Arena {
@@ -66,10 +68,13 @@ struct Arena {
 // Fills the descriptor and initial scalars of one right-hand side: state
 // vectors carved from `A`, tensor maps, coefficient tables; `d_sc` and
 // `d_counter` are its device scalars and finisher counter; tile_base is left
-// to the caller.  zc = 0: the volume's slab depth.
+// to the caller.  d_bnd: the domain-face table of the job's axis (the caller
+// fills it, launch_bnd).  zc = 0: the volume's slab depth.
 int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, int dir,
-              const uint8_t *d_code, Scalars *d_sc, uint32_t *d_counter, Arena &A, const fast_tau_params &P,
-              int zc = 0);
+              const uint8_t *d_code, Scalars *d_sc, uint32_t *d_counter, const void *d_bnd, Arena &A,
+              const fast_tau_params &P, int zc = 0);
+// The coefficient tables of a job (fill_tables of its parameters).
+void job_coefficients(Job &J, const fast_tau_params &P);
 
 int status_of(int state);
 int check_params(const fast_tau_params *p);

@@ -251,6 +251,8 @@ void fill_tables(Job &J, double d0, double d1, int face_mean)
     J.c_tau[1] = (float)d1;
 }
 
+void job_coefficients(Job &J, const fast_tau_params &P) { fill_tables(J, P.d0, P.d1, P.face_mean); }
+
 Geometry make_geometry(int64_t nx, int64_t ny, int64_t nz, int zc_req)
 {
     Geometry g;
@@ -448,6 +450,8 @@ struct JobSpec {
     int dir;
 };
 
+size_t bnd_bytes(int prec) { return (size_t)NBND * (prec == FAST_PREC_F32 ? 8 : 16); }
+
 size_t code_bytes(int64_t nx, int64_t ny, int64_t nz) { return align_up((size_t)(row_pitch(nx) * ny * nz), 256); }
 
 // Slab depth by size class.  A launch's size class is floor(log2(W)), W its
@@ -563,13 +567,15 @@ size_t solve_bytes(const std::vector<VolSpec> &vols, const std::vector<JobSpec> 
     for (const VolSpec &v : vols) need += code_bytes(v.nx, v.ny, v.nz);
     for (const JobSpec &j : jobs) need += job_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec, solver, zc);
     const size_t nj = jobs.size(), nv = vols.size();
+    need += 3 * bnd_bytes(prec);  // one domain-face table per primary axis
     need += align_up(sizeof(Scalars) * nj, 256) + align_up(sizeof(uint32_t) * nj, 256) +
             align_up(sizeof(Job) * (nj + nv), 256) + 256;  // + the replacement gate word
     return need;
 }
 
 int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, int dir,
-              const uint8_t *d_code, Scalars *d_sc, uint32_t *d_counter, Arena &A, const fast_tau_params &P, int zc)
+              const uint8_t *d_code, Scalars *d_sc, uint32_t *d_counter, const void *d_bnd, Arena &A,
+              const fast_tau_params &P, int zc)
 {
     const int prec = P.precision, solver = P.solver;
     const bool mixed = prec == FAST_PREC_MIXED;
@@ -630,7 +636,8 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
     if (ts != FAST_OK) return ts;
     J.sc = d_sc;
     J.counter = d_counter;
-    fill_tables(J, P.d0, P.d1, P.face_mean);
+    J.bnd = d_bnd;
+    job_coefficients(J, P);
 
     const int64_t maxdim = std::max(nx, std::max(ny, nz));
     const float h = 1.0f / (float)maxdim;  // cellDim = vec3(1.0f / maxDim) (VolumeMeasures.cpp:68)
@@ -718,6 +725,10 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     uint32_t *d_cnt = (uint32_t *)A.take(sizeof(uint32_t) * nj);
     Job *d_jobs = (Job *)A.take(sizeof(Job) * (nj + nv));  // jobs, then one code job per volume
     uint32_t *d_gate = (uint32_t *)A.take(sizeof(uint32_t));  // MIXED replacement gate
+    void *d_bnd[3];
+    for (void *&b : d_bnd) b = A.take(bnd_bytes(prec));
+    int axis_job[3] = {0, 0, 0}, naxes = 0;  // a job of each primary axis in use
+    bool axis_seen[3] = {false, false, false};
     std::vector<uint8_t *> d_code(nv);
     std::vector<int> first_job(nv, -1);
     for (int v = 0; v < nv; v++) {
@@ -734,11 +745,15 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     for (int j = 0; j < nj; j++) {
         const VolSpec &V = vols[jobs[j].vol];
         const int bs = build_job(hj[j], hs[j], V.d_mask, V.nx, V.ny, V.nz, jobs[j].dir, d_code[jobs[j].vol], d_sc + j,
-                                 d_cnt + j, A, P, zc);
+                                 d_cnt + j, d_bnd[jobs[j].dir >> 1], A, P, zc);
         if (bs != FAST_OK) {
             cudaFreeAsync(A.base, st);
             cudaStreamSynchronize(st);
             return bs;
+        }
+        if (!axis_seen[jobs[j].dir >> 1]) {
+            axis_seen[jobs[j].dir >> 1] = true;
+            axis_job[naxes++] = j;
         }
         hj[j].tile_base = tile_base;
         tile_base += hj[j].ntiles;
@@ -771,6 +786,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     Launch LC{d_jobs + nj, nv, 0, code_base, nullptr};
 
     int status = FAST_OK;
+    launch_bnd(prec == FAST_PREC_F32, d_jobs, axis_job, naxes, st);
     launch_counted(FAST_K_CODE, st, [&] { launch_code(LC, st); });
     if (!mixed) {
         void (*fn)(Step, const Launch &, cudaStream_t) = (prec == FAST_PREC_F64) ? dispatch_f64 : dispatch_f32;

@@ -23,6 +23,9 @@ void launch_mixed_inner(Step s, const Launch &L, cudaStream_t st);
 void launch_replace(bool bicg, bool ff, const Launch &L, cudaStream_t st);
 void launch_init64(const Launch &L, cudaStream_t st);
 void launch_code(const Launch &L, cudaStream_t st);
+// Fills the domain-face tables (Job::bnd) of the first `count` of jobs[job[0..2]]
+// (device table): one job per primary axis.
+void launch_bnd(bool f32, const Job *jobs, const int (&job)[3], int count, cudaStream_t st);
 // tau flux sum: src 0 = double x, 1 = float x, 2 = the current MIXED iterate
 // as float-float pairs, 3 = the current MIXED iterate as doubles.
 void launch_tau(int src, const Launch &L, cudaStream_t st);

@@ -771,11 +771,11 @@ struct OpInit {
     __device__ Out apply(const Geo &g, const Coef<T> &C, Shared &, const Own &o, const Pos &ps, T fc,
                          T fxp, T fxm, T fyp, T fym, T fzp, T fzm)
     {
-        const T d = diag_of<T, FB>(C, g, o.code, ps);
+        T d, inv;
+        diag_inv<T, FB>(C, g, o.code, ps, d, inv);
         const T ax = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
         const T b = rhs_at<T>(C, g, o.code, ps.x, ps.y, ps.z);
         const T res = b - ax;
-        const T inv = inv_from_diag<T, FB>(C, o.code, ps, d);
         bb.add_prod(b, b);
         rr.add_prod(res, res);
         rz.add_prod(res, res * inv);

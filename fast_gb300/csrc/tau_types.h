@@ -30,6 +30,10 @@ constexpr int NPART = 4;     // partial sums per block per kernel
 constexpr int SELF_BIT = 6;
 constexpr int BND_BIT = 7;
 
+// Entries of the domain-face table (Job::bnd): {diagonal, 1/diagonal} by the
+// voxel's set of missing neighbours (6 bits, Dir order) and its code (7 bits).
+constexpr int NBND = 64 * 128;
+
 enum SolveState : int32_t {
     RUNNING = 0,
     CONVERGED = 1,
@@ -133,6 +137,8 @@ struct Job {
     float xface[2][2][2];        // [self solid][neighbour solid][hi, lo]
     float xcell2[2][2];          // 2*D by solid bit, [hi, lo]
     float c_tau[2];              // tau cell coefficients (float coeffs of the reference)
+    const void *bnd;             // NBND {diagonal, 1/diagonal} pairs of the voxels on a domain face, in the
+                                 // precision that evaluates them by coordinates (F64 and MIXED: double, F32: float)
     int32_t x64_ff;              // MIXED: 1 = x64 holds float-float pairs, 0 = doubles
     int32_t pad0;
 };
