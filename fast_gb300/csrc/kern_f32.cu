@@ -1,7 +1,7 @@
 // FP32 solver kernels: the reference's `-p float` (float scalars) and the
 // inner iterations of the MIXED solve (double scalars).
 #include "tau_launch.h"
-#include "tau_sweep.cuh"
+#include "tau_pointwise.cuh"
 
 namespace ft {
 
@@ -10,6 +10,11 @@ namespace ft {
 #endif
 // Depth of the TMA stage ring (planes of every operand in flight per block).
 constexpr int kStages = FAST_TAU_STAGES_F32;
+#ifndef FAST_TAU_PW_PLANES
+#define FAST_TAU_PW_PLANES 2
+#endif
+// Planes that a thread of a pointwise step loads ahead.
+constexpr int kPlanes = FAST_TAU_PW_PLANES;
 
 #ifndef FAST_TAU_STAGES_K1
 #define FAST_TAU_STAGES_K1 3
@@ -116,11 +121,17 @@ static void dispatch(Step s, const Launch &L, cudaStream_t st)
     case Step::INIT_BI: go<OpInit<T, ST, true>>(L, st); break;
     case Step::CG1: go<OpCG1<T, ST>>(L, st); break;
     case Step::CG2: go<OpCG2<T, ST>>(L, st); break;
-    case Step::BI_RESTART: go<OpBiRestart<T, ST>>(L, st); break;
-    case Step::BI1: go<OpBi1<T, ST>>(L, st); break;
-    case Step::BI2: go<OpBi2<T, ST>>(L, st); break;
-    case Step::BI3: go<OpBi3<T, ST>>(L, st); break;
     default: break;  // replacement steps are MIXED-only (kern_misc.cu)
+    }
+    if constexpr (std::is_same<ST, float>::value) {  // MIXED BiCGSTAB has its own two sweeps
+        switch (s) {
+        case Step::CG2_Q: pointwise_kernel<PwCG2<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
+        case Step::BI_RESTART: go<OpBiRestart<T, ST>>(L, st); break;
+        case Step::BI1: go<OpBi1<T, ST>>(L, st); break;
+        case Step::BI2: go<OpBi2<T, ST>>(L, st); break;
+        case Step::BI3: pointwise_kernel<PwBi3<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
+        default: break;
+        }
     }
 }
 
@@ -133,10 +144,11 @@ static cudaError_t configure()
     if ((r = cfg<OpInit<T, ST, true>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpCG1<T, ST>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpCG2<T, ST>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBiRestart<T, ST>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi1<T, ST>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi2<T, ST>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi3<T, ST>>()) != cudaSuccess) e = r;
+    if constexpr (std::is_same<ST, float>::value) {
+        if ((r = cfg<OpBiRestart<T, ST>>()) != cudaSuccess) e = r;
+        if ((r = cfg<OpBi1<T, ST>>()) != cudaSuccess) e = r;
+        if ((r = cfg<OpBi2<T, ST>>()) != cudaSuccess) e = r;
+    }
     return e;
 }
 

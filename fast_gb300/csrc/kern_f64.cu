@@ -1,6 +1,6 @@
 // Pure FP64 solver kernels (the reference's `-p double`).
 #include "tau_launch.h"
-#include "tau_sweep.cuh"
+#include "tau_pointwise.cuh"
 
 namespace ft {
 
@@ -9,6 +9,11 @@ namespace ft {
 #endif
 // Depth of the TMA stage ring (planes of every operand in flight per block).
 constexpr int kStages = FAST_TAU_STAGES_F64;
+#ifndef FAST_TAU_PW_PLANES
+#define FAST_TAU_PW_PLANES 2
+#endif
+// Planes that a thread of a pointwise step loads ahead.
+constexpr int kPlanes = FAST_TAU_PW_PLANES;
 
 template <class Op>
 static void go(const Launch &L, cudaStream_t st)
@@ -35,7 +40,8 @@ void launch_pure_f64(Step s, const Launch &L, cudaStream_t st)
     case Step::BI_RESTART: go<OpBiRestart<T, T>>(L, st); break;
     case Step::BI1: go<OpBi1<T, T>>(L, st); break;
     case Step::BI2: go<OpBi2<T, T>>(L, st); break;
-    case Step::BI3: go<OpBi3<T, T>>(L, st); break;
+    case Step::CG2_Q: pointwise_kernel<PwCG2<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
+    case Step::BI3: pointwise_kernel<PwBi3<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
     default: break;  // replacement steps are MIXED-only (kern_misc.cu)
     }
 }
@@ -51,7 +57,6 @@ cudaError_t configure_f64()
     if ((r = cfg<OpBiRestart<T, T>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpBi1<T, T>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpBi2<T, T>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi3<T, T>>()) != cudaSuccess) e = r;
     return e;
 }
 

@@ -156,7 +156,8 @@ int kind_of(Step s)
     case Step::INIT_CG:
     case Step::INIT_BI: return FAST_K_INIT;
     case Step::CG1: return FAST_K_CG1;
-    case Step::CG2: return FAST_K_CG2;
+    case Step::CG2:
+    case Step::CG2_Q: return FAST_K_CG2;
     case Step::BI_RESTART: return FAST_K_BI_RESTART;
     case Step::BI1: return FAST_K_BI1;
     case Step::BI2: return FAST_K_BI2;
@@ -559,11 +560,20 @@ size_t job_bytes(int64_t nx, int64_t ny, int64_t nz, int prec, int solver, int z
            align_up((size_t)G.ntiles * NPART * sizeof(double), 256);
 }
 
+// Device bytes of a CG right-hand side's stored product q.
+size_t q_bytes(int64_t nx, int64_t ny, int64_t nz, int prec)
+{
+    return align_up((size_t)(row_pitch(nx) * ny * nz) * (prec == FAST_PREC_F64 ? 8 : 4), 256);
+}
+
 // Device bytes of a solve: one stencil-code array per volume, the state
 // vectors, partial sums and scalars of every right-hand side.
-size_t solve_bytes(const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs, int prec, int solver, int zc)
+size_t solve_bytes(const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs, int prec, int solver, int zc,
+                   bool store_q)
 {
     size_t need = 4096;
+    if (store_q)
+        for (const JobSpec &j : jobs) need += q_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec);
     for (const VolSpec &v : vols) need += code_bytes(v.nx, v.ny, v.nz);
     for (const JobSpec &j : jobs) need += job_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec, solver, zc);
     const size_t nj = jobs.size(), nv = vols.size();
@@ -688,38 +698,44 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
 
     // --- memory plan (the reference's fit check, VolumeMeasures.cpp:104-125)
     const int zc = launch_slab_depth(vols, jobs, prec, solver);
-    const size_t need = solve_bytes(vols, jobs, prec, solver, zc);
+    size_t need = solve_bytes(vols, jobs, prec, solver, zc, false);
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
 #if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
     // test builds: FAST_TAU_TEST_FREE_BYTES pretends the device has that much
     // free memory and nothing cached, so the fit check can be made to fail
     const char *fake_free = getenv("FAST_TAU_TEST_FREE_BYTES");
-    if (fake_free) {
-        free_b = (size_t)strtoull(fake_free, nullptr, 10);
-        if (need > free_b)
-            return fail(FAST_NOMEM, "Solver will not fit in GPU memory: needs %.3f GB, %.3f GB free", need / 1e9,
-                        free_b / 1e9);
-    }
+    if (fake_free) free_b = (size_t)strtoull(fake_free, nullptr, 10);
 #endif
-    if (need > free_b) {
-        // Memory already cached by the stream-ordered pool counts as available.
-        size_t reserved = 0;
-        cudaMemPool_t pool;
-        if (cudaDeviceGetDefaultMemPool(&pool, E.device) == cudaSuccess) {
-            uint64_t r = 0, u = 0;
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &r);
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &u);
-            reserved = (size_t)(r - u);
-        }
-        if (need > free_b + reserved)
-            return fail(FAST_NOMEM, "Solver will not fit in GPU memory: needs %.3f GB, %.3f GB free", need / 1e9,
-                        (free_b + reserved) / 1e9);
+    // Memory already cached by the stream-ordered pool counts as available.
+    size_t avail = free_b;
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, E.device) == cudaSuccess) {
+        uint64_t r = 0, u = 0;
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &r);
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &u);
+        avail += (size_t)(r - u);
     }
+#if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
+    if (fake_free) avail = free_b;
+#endif
+    if (need > avail)
+        return fail(FAST_NOMEM, "Solver will not fit in GPU memory: needs %.3f GB, %.3f GB free", need / 1e9,
+                    avail / 1e9);
     (void)total_b;
 
+    // F64 / F32 CG keeps q = A p between its steps where the extra vector
+    // fits beside everything else; a volume that fills the GPU evaluates the
+    // product twice instead (the same results).
     Arena A;
-    CU(cudaMallocAsync((void **)&A.base, need, st));
+    bool store_q = !mixed && solver == FAST_SOLVER_CG;
+    if (store_q) {
+        const size_t more = solve_bytes(vols, jobs, prec, solver, zc, true);
+        store_q = more <= avail && cudaMallocAsync((void **)&A.base, more, st) == cudaSuccess;
+        if (store_q) need = more;
+        else cudaGetLastError();
+    }
+    if (!store_q) CU(cudaMallocAsync((void **)&A.base, need, st));
     A.cap = need;
     Scalars *d_sc = (Scalars *)A.take(sizeof(Scalars) * nj);
     uint32_t *d_cnt = (uint32_t *)A.take(sizeof(uint32_t) * nj);
@@ -755,6 +771,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
             axis_seen[jobs[j].dir >> 1] = true;
             axis_job[naxes++] = j;
         }
+        if (store_q) hj[j].q = A.take(q_bytes(V.nx, V.ny, V.nz, prec));
         hj[j].tile_base = tile_base;
         tile_base += hj[j].ntiles;
     }
@@ -792,7 +809,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
         void (*fn)(Step, const Launch &, cudaStream_t) = (prec == FAST_PREC_F64) ? dispatch_f64 : dispatch_f32;
         launch_counted(FAST_K_INIT, st, [&] { fn(solver == FAST_SOLVER_CG ? Step::INIT_CG : Step::INIT_BI, L, st); });
         std::vector<Step> steps;
-        if (solver == FAST_SOLVER_CG) steps = {Step::CG1, Step::CG2};
+        if (solver == FAST_SOLVER_CG) steps = {Step::CG1, store_q ? Step::CG2_Q : Step::CG2};
         else steps = {Step::BI_RESTART, Step::BI1, Step::BI2, Step::BI3};
         status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
     } else {

@@ -7,7 +7,7 @@
 namespace ft {
 
 enum class Step {
-    INIT_CG, INIT_BI, CG1, CG2, BI_RESTART, BI1, BI2, BI3, REPLACE_CG, REPLACE_BI, BI_K1, BI_K2, CG_F,
+    INIT_CG, INIT_BI, CG1, CG2, CG2_Q, BI_RESTART, BI1, BI2, BI3, REPLACE_CG, REPLACE_BI, BI_K1, BI_K2, CG_F,
     REPLACE_CG_FF, REPLACE_BI_FF  // the replacement with a float-float iterate (opt-in)
 };
 

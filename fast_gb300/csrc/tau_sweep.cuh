@@ -915,10 +915,11 @@ struct OpCG1 {
     using Shared = NoShared;
     struct Vals { T r, p; uint32_t code; };
     struct Own { uint32_t code; T d; };
-    struct Out { T p; };
+    struct Out { T p, q; };
     const CUtensorMap *tmap[SL::N];
     Faces<T> F;
     T *pnew;
+    T *qout;   // F64 / F32: q for the pointwise step 2 (null: step 2 evaluates it again)
     T *ezero;  // MIXED: e to zero after a residual replacement, else null
     T beta;
     Acc<T> pap;
@@ -945,6 +946,7 @@ struct OpCG1 {
         tmap[1] = &J.tm[TM_P + par];
         tmap[2] = &J.tm[TM_CODE];
         pnew = (T *)J.p[par ^ 1];
+        qout = FB ? nullptr : (T *)J.q;
         ezero = J.sc->e_reset ? (T *)J.x : nullptr;
         beta = (T)J.sc->beta;
     }
@@ -965,11 +967,14 @@ struct OpCG1 {
     {
         const T q = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, o.d);
         pap.add_prod(fc, q);
-        return Out{fc};
+        return Out{fc, q};
     }
     __device__ void store(int64_t i, const Out &a, const Out &b, bool v0, bool v1)
     {
         store2<T>(pnew, i, a.p, b.p, v0, v1);
+        if constexpr (!FB) {
+            if (qout) store2<T>(qout, i, a.q, b.q, v0, v1);
+        }
         if (ezero) store2<T>(ezero, i, T(0), T(0), v0, v1);
     }
     __device__ void partials(T (&v)[NV]) const { v[0] = pap.hi(); }
@@ -981,7 +986,8 @@ struct OpCG1 {
 };
 
 // ===========================================================================
-// CG step 2: q = A p (recomputed), x += alpha p, r -= alpha q, z = r/diag,
+// CG step 2: q = A p (recomputed; F64 and F32 solves with room for q take the
+// pointwise form of tau_pointwise.cuh), x += alpha p, r -= alpha q, z = r/diag,
 // dots |r|^2 and r.z; convergence, beta and the iteration count.
 // CG.cu:87-154.  Streams: p, x, r, code.
 // ===========================================================================
@@ -1233,8 +1239,9 @@ struct OpBi1 {
 };
 
 // ===========================================================================
-// BiCGSTAB step 2: s = r - alpha v, z = s/diag, t = A z, dots t.s, t.t.
-// BICGSTAB.cu:149-183.  Streams: r, v_new, code.
+// BiCGSTAB step 2: s = r - alpha v, z = s/diag, t = A z (stored), dots t.s,
+// t.t.  BICGSTAB.cu:149-183.  Streams: r, v_new, code.  Step 3 is pointwise
+// (tau_pointwise.cuh).
 // ===========================================================================
 template <typename TT, typename ST>
 struct OpBi2 {
@@ -1245,9 +1252,10 @@ struct OpBi2 {
     using Shared = NoShared;
     struct Vals { T r, v; uint32_t code; };
     struct Own { uint32_t code; T s; };
-    using Out = NoOut;
+    struct Out { T t; };
     const CUtensorMap *tmap[SL::N];
     Faces<T> F;
+    T *tout;  // t for the pointwise step 3, in the v buffer that step 1 read
     T nalpha;
     Acc<T> ts, tt;
 
@@ -1272,6 +1280,7 @@ struct OpBi2 {
         tmap[0] = &J.tm[TM_R + par];
         tmap[1] = &J.tm[TM_V + (par ^ 1)];
         tmap[2] = &J.tm[TM_CODE];
+        tout = (T *)J.v[par];
         nalpha = (T)(-J.sc->alpha);
     }
     __device__ __forceinline__ T sval(const Vals &v) const { return v.r + nalpha * v.v; }  // s = r + (-alpha) v
@@ -1292,128 +1301,17 @@ struct OpBi2 {
         const T t = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
         ts.add_prod(t, o.s);
         tt.add_prod(t, t);
-        return Out{};
+        return Out{t};
     }
-    __device__ void store(int64_t, const Out &, const Out &, bool, bool) {}
+    __device__ void store(int64_t i, const Out &a, const Out &b, bool v0, bool v1)
+    {
+        store2<T>(tout, i, a.t, b.t, v0, v1);
+    }
     __device__ void partials(T (&v_)[NV]) const { v_[0] = ts.hi(); v_[1] = tt.hi(); }
     __device__ static void finish(Scalars &sc, const double (&t)[NV])
     {
         const ST tmp = (ST)t[1];
         sc.omega = (tmp > ST(0)) ? (double)((ST)t[0] / tmp) : 0.0;  // BICGSTAB.cu:175-183
-    }
-};
-
-// ===========================================================================
-// BiCGSTAB step 3: t recomputed, x += alpha y + w z, r = s - w t, dots r0.r and
-// |r|^2; divergence, iteration count, convergence, next rho/beta or a
-// restart.  BICGSTAB.cu:187-212 + the loop head :93-112.
-// Streams: r, v_new, p_new, x, r0, code.
-// ===========================================================================
-template <typename TT, typename ST>
-struct OpBi3 {
-    using T = TT;
-    static constexpr bool FB = sizeof(TT) == 4 && sizeof(ST) == 8;  // MIXED FP32 iterations
-    using SL = Streams<sizeof(TT), sizeof(TT), sizeof(TT), sizeof(TT), sizeof(TT), 1>;
-    static constexpr int NV = 2;
-    using Shared = NoShared;
-    struct Vals { T r, v, p, x, r0; uint32_t code; };
-    struct Own { uint32_t code; T s, x, y, r0; };
-    struct Out { T x, r; };
-    const CUtensorMap *tmap[SL::N];
-    Faces<T> F;
-    T *x, *rnew;
-    T alpha, omega, nalpha, nomega;
-    Acc<T> r0r, rr;
-
-    __device__ static bool active(const Scalars &sc) { return sc.state == RUNNING; }
-    __device__ static void load_shared(Shared &, const Job &, int) {}
-    __device__ static void load2(const unsigned char *st, const Pt &p, Vals &a, Vals &b)
-    {
-        sv2<T, SL, 0>(st, p, a.r, b.r);
-        sv2<T, SL, 1>(st, p, a.v, b.v);
-        sv2<T, SL, 2>(st, p, a.p, b.p);
-        sv2<T, SL, 3>(st, p, a.x, b.x);
-        sv2<T, SL, 4>(st, p, a.r0, b.r0);
-        load_code2<SL, 5>(st, p, a.code, b.code);
-    }
-    __device__ static void load1(const unsigned char *st, const Pt &p, Vals &a)
-    {
-        a.r = sv<T, SL, 0>(st, p);
-        a.v = sv<T, SL, 1>(st, p);
-        a.code = sv<uint8_t, SL, 5>(st, p);
-    }
-    __device__ void init(const Job &J, Shared &)
-    {
-        F = faces_of<T>(J);
-        const int par = (int)(J.sc->iter & 1);
-        tmap[0] = &J.tm[TM_R + par];
-        tmap[1] = &J.tm[TM_V + (par ^ 1)];
-        tmap[2] = &J.tm[TM_P + (par ^ 1)];
-        tmap[3] = &J.tm[TM_X];
-        tmap[4] = &J.tm[TM_R0];
-        tmap[5] = &J.tm[TM_CODE];
-        x = (T *)J.x;
-        rnew = (T *)J.r[par ^ 1];
-        alpha = (T)J.sc->alpha;
-        omega = (T)J.sc->omega;
-        nalpha = -alpha;
-        nomega = -omega;
-    }
-    __device__ __forceinline__ T sval(const Vals &v) const { return v.r + nalpha * v.v; }
-    __device__ T field(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps) const
-    {
-        return sval(v) * inv_of<T, FB>(C, g, v.code, ps);
-    }
-    __device__ Own own(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps, T &f) const
-    {
-        const T s = sval(v);
-        const T inv = inv_of<T, FB>(C, g, v.code, ps);
-        f = s * inv;
-        return Own{v.code, s, v.x, v.p * inv, v.r0};
-    }
-    __device__ Out apply(const Geo &g, const Coef<T> &C, Shared &, const Own &o, const Pos &ps, T fc,
-                         T fxp, T fxm, T fyp, T fym, T fzp, T fzm)
-    {
-        const T d = diag_of<T, FB>(C, g, o.code, ps);
-        const T t = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
-        const T xn = o.x + (alpha * o.y + omega * fc);   // __ABC_BetaGammaKernel: x += a*y + w*z
-        const T rn = o.s + nomega * t;                   // __aPlusBetaBKernel(s, t, r, -w)
-        r0r.add_prod(o.r0, rn);
-        rr.add_prod(rn, rn);
-        return Out{xn, rn};
-    }
-    __device__ void store(int64_t i, const Out &a, const Out &b, bool v0, bool v1)
-    {
-        store2<T>(x, i, a.x, b.x, v0, v1);
-        store2<T>(rnew, i, a.r, b.r, v0, v1);
-    }
-    __device__ void partials(T (&v_)[NV]) const { v_[0] = r0r.hi(); v_[1] = rr.hi(); }
-    __device__ static void finish(Scalars &sc, const double (&t)[NV])
-    {
-        if (sc.inner_mode) {
-            mixed_bicg_finish(sc, t[0], t[1]);
-            return;
-        }
-        const ST rsq = (ST)t[1];
-        sc.rsq = rsq;
-        if (rsq > (ST)sc.div_thresh) {  // BICGSTAB.cu:206-209, before ++i
-            sc.state = DIVERGED;
-            return;
-        }
-        sc.iter += 1;  // BICGSTAB.cu:211
-        if (!(rsq > (ST)sc.tol2)) { sc.state = CONVERGED; return; }
-        if (sc.iter >= sc.max_iter) { sc.state = MAXITER; return; }
-        // Loop head of the next iteration (BICGSTAB.cu:95-112).
-        const ST rho_old = (ST)sc.rho;
-        const ST rho = (ST)t[0];
-        sc.rho_old = rho_old;
-        sc.rho = rho;
-        const ST mag = rho < ST(0) ? -rho : rho;
-        if (mag < (ST)sc.eps2 * (ST)sc.r0_sq) {
-            sc.restart = 1;
-        } else {
-            sc.beta = (double)((rho / rho_old) * ((ST)sc.alpha / (ST)sc.omega));
-        }
     }
 };
 

@@ -116,6 +116,8 @@ struct Job {
     void *r0;                    // BiCGSTAB shadow residual (T)
     void *p[2];                  // search direction ping-pong (T)
     void *v[2];                  // BiCGSTAB v ping-pong (T)
+    void *q;                     // F64 / F32 CG: q = A p, kept from step 1 to the pointwise step 2 (null: no room,
+                                 // step 2 evaluates it again)
     void *t;                     // MIXED BiCGSTAB: t = A s, kept from step 2 to step 1 (FP32)
     void *x64[2];                // MIXED extended-precision iterate ping-pong: double, or float-float
                                  // (hi, lo) pairs when x64_ff is set
