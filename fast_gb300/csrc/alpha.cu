@@ -24,16 +24,18 @@
 //     in double, then over all cells.
 //
 // The engine evaluates all of it in one pass over the volume and, for the
-// per-direction form, over the CCL labels at the same time: each voxel gets
-// a 7-bit code (bit d: its pore component touches face d; bit 6: the voxel
-// is solid), expanded to one 4-bit lane per bit, so adding the eight voxels
-// around a grid point counts all seven fields at once.  A block owns a 32x8
-// column of cells and walks a z-slab, keeping a ring of three expanded voxel
-// planes in shared memory; a cell whose eight corner words are equal has no
-// surface in any field and costs nothing more.  Reductions are per block
-// then in a fixed order, so results are run-to-run identical.
+// per-direction form, over the CCL labels at the same time.  A block owns a
+// brick of 62 x 16 x up to 16 cells and holds the voxels it needs as bits, 64
+// along x in a word, one word array per field (bit set: the voxel's pore
+// component touches face d; the seventh field: the voxel is solid).  Corner
+// counts are sums of eight bits, done for 63 corners at once with word-wide
+// adders, and so are the comparison with the isovalue and the test of which
+// cells the surface cuts: a few instructions per 62 cells.  Only cut cells go
+// further, compacted into a queue.  Fields that are equal over the brick (the
+// face-connected pores, nearly everywhere) share their triangles.  Reductions
+// are per block then in a fixed order, so results are run-to-run identical.
 //
-// The triangulation table is generated here, not copied: for each of the 256
+// The triangulation table is generated at compile time, not copied: for each of the 256
 // corner patterns the cut edges of every cube face are joined in pairs (on a
 // face with four cut edges, the two "below" corners are kept apart), the
 // pairs close into loops, and each loop is fanned from its first edge.  Two
@@ -50,7 +52,6 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "fasttau.h"
@@ -58,12 +59,12 @@
 
 namespace {
 
-// A block is 32 x 8 threads; each thread owns two cells in y (rows ty and
-// ty + 8), so a block covers 32 x 16 cells.
-constexpr int TX = 32, TYT = 8, NT = TX * TYT, CY = 2, TY = TYT * CY;
-constexpr int PW = TX + 2, PH = TY + 2;  // expanded plane tile with a one-voxel rim
-constexpr int NLOAD = (PW * PH + NT - 1) / NT;
-constexpr int kMaxSlab = 32;             // z-slab depth limit (5 bits in a queue item)
+constexpr int NT = 256;
+constexpr int BX = 62, BY = 16, BZ = 16;  // cells of a brick (z: at most)
+constexpr int VY = BY + 2;                // voxel rows of a brick's plane
+constexpr int VROWS = VY * (BZ + 2);      // voxel rows of a brick, 64 bits each
+constexpr int CROWS = (BY + 1) * (BZ + 1);  // rows of grid points
+static_assert(BY * BZ <= NT, "one row of cells per thread");
 constexpr int kMaxTri = 5;
 constexpr int kFields = 7;               // six face-connected pore fields + the solid field
 
@@ -71,7 +72,6 @@ struct McTable {
     uint8_t ntri[256];
     uint8_t edge[256][3 * kMaxTri];
 };
-static_assert(sizeof(McTable) == 4096, "table is copied as 256 x 16 bytes");
 
 // Corner c of a cell sits at offset (c&1 ^ c>>1&1, c>>1&1, c>>2) in the
 // reference's order: 0 (0,0,0) 1 (1,0,0) 2 (1,1,0) 3 (0,1,0), 4..7 the same at
@@ -81,27 +81,23 @@ constexpr int kEdgeA[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
 constexpr int kEdgeB[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
 constexpr int kFaces[6][4] = {{0, 1, 2, 3}, {4, 5, 6, 7}, {0, 1, 5, 4}, {3, 2, 6, 7}, {0, 3, 7, 4}, {1, 2, 6, 5}};
 
-int edge_between(int a, int b)
+constexpr int edge_between(int a, int b)
 {
     for (int e = 0; e < 12; e++)
         if ((kEdgeA[e] == a && kEdgeB[e] == b) || (kEdgeA[e] == b && kEdgeB[e] == a)) return e;
     return -1;
 }
 
-McTable build_table()
+constexpr McTable build_table()
 {
-    McTable T;
-    memset(&T, 0, sizeof(T));
+    McTable T{};
     for (int cs = 0; cs < 256; cs++) {
-        int nb[12][2], deg[12] = {0};
-        auto link = [&](int a, int b) {
-            nb[a][deg[a]++] = b;
-            nb[b][deg[b]++] = a;
-        };
-        for (const auto &f : kFaces) {
-            int E[4];
-            bool cut[4], below[4];
-            int ncut = 0;
+        int nb[12][2] = {}, deg[12] = {};
+        for (int fi = 0; fi < 6; fi++) {
+            const int *f = kFaces[fi];
+            int E[4] = {}, pair[4] = {};
+            bool cut[4] = {}, below[4] = {};
+            int ncut = 0, npair = 0;
             for (int q = 0; q < 4; q++) {
                 E[q] = edge_between(f[q], f[(q + 1) & 3]);
                 below[q] = (cs >> f[q]) & 1;
@@ -111,25 +107,22 @@ McTable build_table()
                 ncut += cut[q];
             }
             if (ncut == 2) {
-                int a = -1, b = -1;
                 for (int q = 0; q < 4; q++)
-                    if (cut[q]) (a < 0 ? a : b) = E[q];
-                link(a, b);
+                    if (cut[q]) pair[npair++] = E[q];
             } else if (ncut == 4) {
-                if (below[0]) {  // corners 0 and 2 below: cut around each
-                    link(E[3], E[0]);
-                    link(E[1], E[2]);
-                } else {         // corners 1 and 3 below
-                    link(E[0], E[1]);
-                    link(E[2], E[3]);
-                }
+                const int first = below[0] ? 3 : 0;  // corners 0 and 2 below: cut around each; else around 1 and 3
+                for (int q = 0; q < 4; q++) pair[npair++] = E[(first + q) & 3];
+            }
+            for (int q = 0; q < npair; q += 2) {
+                nb[pair[q]][deg[pair[q]]++] = pair[q + 1];
+                nb[pair[q + 1]][deg[pair[q + 1]]++] = pair[q];
             }
         }
-        bool seen[12] = {false};
+        bool seen[12] = {};
         int nt = 0;
         for (int e = 0; e < 12; e++) {
             if (deg[e] == 0 || seen[e]) continue;
-            int loop[12], len = 0, prev = e, cur = nb[e][0] < nb[e][1] ? nb[e][0] : nb[e][1];
+            int loop[12] = {}, len = 0, prev = e, cur = nb[e][0] < nb[e][1] ? nb[e][0] : nb[e][1];
             loop[len++] = e;
             seen[e] = true;
             while (cur != e) {
@@ -151,14 +144,86 @@ McTable build_table()
     return T;
 }
 
+// The same by corner pattern in one word, as fans: the edges of a loop's
+// vertices in order, 4 bits each, kRestart before every further loop, and 0
+// bits from the end on (a loop's 12 edges and 3 restarts fit 60 bits; the
+// number of entries is in bits 60..63).
+using PackedCase = uint64_t;
+constexpr int kRestart = 15;
+struct PackedTable {
+    PackedCase at[256];
+};
+
+constexpr PackedTable pack_table(const McTable &T)
+{
+    PackedTable P{};
+    for (int cs = 0; cs < 256; cs++) {
+        int n = 0;
+        for (int t = 0; t < T.ntri[cs]; t++) {
+            const uint8_t *e = &T.edge[cs][3 * t];
+            const bool more = t > 0 && e[0] == e[-3] && e[1] == e[-1];
+            if (!more) {
+                if (t > 0) P.at[cs] |= (PackedCase)kRestart << (4 * n++);
+                P.at[cs] |= (PackedCase)e[0] << (4 * n++);
+                P.at[cs] |= (PackedCase)e[1] << (4 * n++);
+            }
+            P.at[cs] |= (PackedCase)e[2] << (4 * n++);
+        }
+        P.at[cs] |= (PackedCase)n << 60;
+    }
+    return P;
+}
+
+// What a vertex on an edge needs: the corners' counts to pick (a byte
+// selector over the counts of the even then the odd corners), the direction
+// along each axis from its first corner (1, -1, or 0 across the edge) and
+// all-ones where that corner is the cell's high one.
+struct alignas(16) EdgeInfo {
+    float dir[3];
+    uint32_t pick;
+    uint32_t high[3];
+    uint32_t pad;
+};
+struct EdgeTable {
+    EdgeInfo at[12];
+};
+
+constexpr EdgeTable make_edges()
+{
+    EdgeTable E{};
+    for (int e = 0; e < 12; e++) {
+        const int c[2] = {kEdgeA[e], kEdgeB[e]};
+        int at[2][3] = {};
+        for (int k = 0; k < 2; k++) {
+            at[k][0] = (c[k] & 1) ^ ((c[k] >> 1) & 1);
+            at[k][1] = (c[k] >> 1) & 1;
+            at[k][2] = c[k] >> 2;
+        }
+        for (int a = 0; a < 3; a++) {
+            E.at[e].dir[a] = (float)(at[1][a] - at[0][a]);
+            E.at[e].high[a] = at[0][a] ? 0xffffffffu : 0u;
+        }
+        // bytes 0..3: corners 0, 2, 4, 6; bytes 4..7: corners 1, 3, 5, 7;
+        // byte 0 of the result: the second corner, byte 1: the first
+        auto byte_of = [](int q) { return (uint32_t)((q & 1) * 4 + q / 2); };
+        E.at[e].pick = byte_of(c[1]) | byte_of(c[0]) << 4;
+    }
+    return E;
+}
+
+constexpr McTable kTable = build_table();
+__device__ const McTable d_table = kTable;
+__device__ const PackedTable d_cases = pack_table(kTable);
+__device__ const EdgeTable d_edges = make_edges();
+
 struct AlphaArgs {
     const uint8_t *mask;
     const uint32_t *labels;      // nullptr: the solid field alone
     const uint8_t *label_bits;   // per label: bit d = touches face d
-    const McTable *table;
-    double *partials;            // [blocks][kFields]
+    double *partials;            // [kFields][blocks]
     uint32_t *bad;               // set when a voxel is neither 0 nor 255
     int nx, ny, nz, zc, tiles_x, tiles_y;
+    int64_t nblocks;
     float iso, vx, vy, vz;       // isovalue, voxel size 1/n per axis
     int thr;                     // corner below <=> count < thr (count = 8 x value)
 };
@@ -167,70 +232,40 @@ struct AlphaArgs {
 __device__ __forceinline__ int edge_a(int e) { return (int)((0x321076543210ULL >> (4 * e)) & 15u); }
 __device__ __forceinline__ int edge_b(int e) { return (int)((0x765447650321ULL >> (4 * e)) & 15u); }
 
-__device__ __forceinline__ uint32_t spread7(uint32_t c)
-{
-    return (c & 1u) | (c & 2u) << 3 | (c & 4u) << 6 | (c & 8u) << 9 | (c & 16u) << 12 | (c & 32u) << 15 |
-           (c & 64u) << 18;
-}
-
-// One expanded voxel plane into shared memory; off[r] = the clamped (x, y)
-// offset of this thread's r-th tile entry (fixed for the block).
-template <bool LABELS>
-__device__ __forceinline__ void load_plane(const AlphaArgs &A, uint32_t *dst, const int64_t off[NLOAD], int p)
-{
-    const int pz = p < 0 ? 0 : (p >= A.nz ? A.nz - 1 : p);
-    const int64_t base = (int64_t)pz * A.nx * A.ny;
-#pragma unroll
-    for (int r = 0; r < NLOAD; r++) {
-        const int e = threadIdx.x + r * NT;
-        if (e < PW * PH) {
-            const int64_t idx = base + off[r];
-            const uint32_t m = A.mask[idx];
-            if (m != 0 && m != 255) *A.bad = 1;
-            uint32_t code;
-            if (LABELS)
-                code = spread7((m ? 64u : 0u) | A.label_bits[A.labels[idx]]);
-            else
-                code = m ? 1u : 0u;
-            dst[e] = code;
-        }
-    }
-}
-
-// Float arithmetic as the reference's helpers (lerp, cross, length) write it,
-// with no fused multiply-add so that every cell's area is reproducible.
 __device__ __forceinline__ float lerp1(float a, float b, float t) { return __fadd_rn(a, __fmul_rn(t, __fsub_rn(b, a))); }
 
-// Area of triangle `t` of corner pattern `cube` in the cell whose low corner
-// is (px, py, pz) and high corner (qx, qy, qz); cnt = 8 corner counts
-// (4 bits each, corner c at bits 4c).
-__device__ __forceinline__ float triangle_area(const McTable &T, int cube, int t, uint32_t cnt, float iso, float px,
-                                               float py, float pz, float qx, float qy, float qz)
+// What a cell's vertices are made of: its low corner, high corner XOR low
+// corner (as bits) and high - low along each axis, and its corner counts, a
+// byte each, corners 0, 2, 4, 6 and 1, 3, 5, 7.
+struct Cell {
+    uint32_t p[3], x[3];
+    float d[3];
+    uint32_t even, odd;
+};
+
+// t by the counts n0, n1 at an edge's two ends sits at n0 * 256 + n1, the
+// two bytes that a byte permute picks from the cell's counts.
+constexpr int kTSize = 8 * 256 + 9;
+
+// The vertex on an edge, in float arithmetic as the reference's helpers
+// (lerp, cross, length) write it, with no fused multiply-add, so that every
+// cell's area is reproducible: p0 + t (p1 - p0) per axis, where p1 - p0 is
+// plus or minus high - low along the edge and 0 across it.
+__device__ __forceinline__ float3 vertex(const Cell &C, const float *t_of, const EdgeInfo *edges, int e)
 {
-    float v[3][3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        const int e = T.edge[cube][3 * t + q];
-        const int ca = edge_a(e), cb = edge_b(e);
-        const float fa = __fmul_rn((float)((cnt >> (4 * ca)) & 15u), 0.125f);
-        const float fb = __fmul_rn((float)((cnt >> (4 * cb)) & 15u), 0.125f);
-        const int axa = (ca & 1) ^ ((ca >> 1) & 1), aya = (ca >> 1) & 1, aza = ca >> 2;
-        const int axb = (cb & 1) ^ ((cb >> 1) & 1), ayb = (cb >> 1) & 1, azb = cb >> 2;
-        const float x0 = axa ? qx : px, y0 = aya ? qy : py, z0 = aza ? qz : pz;
-        const float x1 = axb ? qx : px, y1 = ayb ? qy : py, z1 = azb ? qz : pz;
-        if (fa == fb) {
-            v[q][0] = x0;
-            v[q][1] = y0;
-            v[q][2] = z0;
-        } else {
-            const float tt = __fdiv_rn(__fsub_rn(iso, fa), __fsub_rn(fb, fa));
-            v[q][0] = lerp1(x0, x1, tt);
-            v[q][1] = lerp1(y0, y1, tt);
-            v[q][2] = lerp1(z0, z1, tt);
-        }
-    }
-    const float ax = __fsub_rn(v[1][0], v[0][0]), ay = __fsub_rn(v[1][1], v[0][1]), az = __fsub_rn(v[1][2], v[0][2]);
-    const float bx = __fsub_rn(v[2][0], v[0][0]), by = __fsub_rn(v[2][1], v[0][1]), bz = __fsub_rn(v[2][2], v[0][2]);
+    const uint4 a = *reinterpret_cast<const uint4 *>(&edges[e].dir[0]);
+    const uint4 b = *reinterpret_cast<const uint4 *>(&edges[e].high[0]);
+    const float t = t_of[__byte_perm(C.even, C.odd, a.w) & 0xffffu];
+    auto axis = [&](int k, uint32_t dir, uint32_t high) {
+        return __fadd_rn(__uint_as_float(C.p[k] ^ (C.x[k] & high)), __fmul_rn(__fmul_rn(t, __uint_as_float(dir)), C.d[k]));
+    };
+    return make_float3(axis(0, a.x, b.x), axis(1, a.y, b.y), axis(2, a.z, b.z));
+}
+
+__device__ __forceinline__ float triangle_area(const float3 &v0, const float3 &v1, const float3 &v2)
+{
+    const float ax = __fsub_rn(v1.x, v0.x), ay = __fsub_rn(v1.y, v0.y), az = __fsub_rn(v1.z, v0.z);
+    const float bx = __fsub_rn(v2.x, v0.x), by = __fsub_rn(v2.y, v0.y), bz = __fsub_rn(v2.z, v0.z);
     const float cx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
     const float cy = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
     const float cz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
@@ -238,252 +273,327 @@ __device__ __forceinline__ float triangle_area(const McTable &T, int cube, int t
     return __fmul_rn(__fsqrt_rn(d), 0.5f);
 }
 
-// Counts of field f at the 8 corners, corner c at bits 4c.
-__device__ __forceinline__ uint32_t field_counts(const uint32_t W[8], int f)
+// A sum of floats as an unevaluated pair (Knuth's two-sum): a thread adds a
+// few dozen areas of a brick, so the pair holds them to about 2^-47; the FP64
+// pipe is narrow enough that adding every area in double would cost more than
+// finding the triangles.
+struct PairSum {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(float a, float ac = 0.f)
+    {
+        const float t = __fadd_rn(s, a);
+        const float b = __fsub_rn(t, s);
+        const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(a, b));
+        s = t;
+        c = __fadd_rn(c, __fadd_rn(e, ac));
+    }
+};
+
+// Full adder of three words: sum and carry.
+__device__ __forceinline__ uint64_t maj3(uint64_t a, uint64_t b, uint64_t c) { return (a & b) | (c & (a | b)); }
+
+// Counts over two neighbouring voxels along x then y, bit c of word b the bit
+// 2^b of the count at grid point c.
+struct Sum2x2 {
+    uint64_t b0, b1, b2;
+};
+
+__device__ __forceinline__ Sum2x2 sum2x2(uint64_t u, uint64_t v)
 {
-    uint32_t c = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) c |= ((W[q] >> (4 * f)) & 15u) << (4 * q);
-    return c;
+    const uint64_t u0 = u ^ (u >> 1), u1 = u & (u >> 1), v0 = v ^ (v >> 1), v1 = v & (v >> 1);
+    const uint64_t k = u0 & v0;
+    return Sum2x2{u0 ^ v0, u1 ^ v1 ^ k, maj3(u1, v1, k)};
 }
 
+// Grid points whose count over both planes is below thr (1..8).
+__device__ __forceinline__ uint64_t below_word(const Sum2x2 &a, const Sum2x2 &b, int thr)
+{
+    const uint64_t t0 = a.b0 ^ b.b0, k0 = a.b0 & b.b0;
+    const uint64_t t1 = a.b1 ^ b.b1 ^ k0, k1 = maj3(a.b1, b.b1, k0);
+    const uint64_t t2 = a.b2 ^ b.b2 ^ k1, t3 = maj3(a.b2, b.b2, k1);
+    uint64_t lt = (thr & 1) ? ~t0 : 0ull;
+    lt = (thr & 2) ? (~t1 | lt) : (~t1 & lt);
+    lt = (thr & 4) ? (~t2 | lt) : (~t2 & lt);
+    return (thr & 8) ? (~t3 | lt) : (~t3 & lt);
+}
+
+// Counts at the eight corners of the cell in row (j, k) whose low corner is
+// grid point c: three bits of each of the nine voxel rows around it.
+__device__ __forceinline__ uint32_t cell_counts(const uint64_t *v, int j, int k, int c)
+{
+    uint32_t p[3][2];
+#pragma unroll
+    for (int dz = 0; dz < 3; dz++) {
+        uint32_t x[3];
+#pragma unroll
+        for (int dy = 0; dy < 3; dy++) {
+            const uint32_t b = (uint32_t)(v[(k + dz) * VY + j + dy] >> c) & 7u;
+            // sums of bits 0, 1 (low nibble) and 1, 2 (high nibble)
+            x[dy] = __byte_perm(0x12110100u, 0x22211110u, b);
+        }
+        p[dz][0] = x[0] + x[1];
+        p[dz][1] = x[1] + x[2];
+    }
+    auto swap = [](uint32_t g) { return ((g & 15u) << 4) | (g >> 4); };  // corners 2, 3 run against x
+    return (p[0][0] + p[1][0]) | swap(p[0][1] + p[1][1]) << 8 | (p[1][0] + p[2][0]) << 16 |
+           swap(p[1][1] + p[2][1]) << 24;
+}
+
+// Corner pattern of eight counts: bit q set when count q < thr (1..8).
 __device__ __forceinline__ int cube_of(uint32_t cnt, int thr)
 {
-    int cube = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) cube |= (int)(((cnt >> (4 * q)) & 15u) < (uint32_t)thr) << q;
-    return cube;
+    uint32_t m = (~(cnt + (uint32_t)(8 - thr) * 0x11111111u) >> 3) & 0x11111111u;
+    m = (m | m >> 3) & 0x03030303u;
+    m = (m | m >> 6) & 0x000f000fu;
+    return (int)((m | m >> 12) & 0xffu);
 }
 
-// Triangles wait in a shared queue so that all lanes compute areas at once:
-// a cell with a surface is rare and has one to five triangles per field, so
-// evaluating them in the cell's own lane would leave most of the warp idle.
-// Queue positions come from a block-wide exclusive scan (fixed order), and
-// item q is always done by thread q mod NT, so the double sums are the same
-// on every run.
-constexpr int QCAP = 2048;
+constexpr int QCAP = 4096;  // cells in the queue at once
 
-// Both passes are held to 64 registers (4 blocks per SM; the seven-field
-// one spills a few hundred bytes): their memory waits want the warps more
-// than the registers (1024^3: seven fields 62.9 ms at 128 registers and 2
-// blocks, 61.3 at 3, 58.7 at 4; one field 16.1 ms at 75 registers and 3
-// blocks, 14.7 at 4, 15.4 at 5).
+// The cut cells go through a shared queue so that all lanes have one: about
+// one cell in seven of a porous volume is cut.  Queue positions come from a
+// block-wide scan and item q is done by thread q mod NT, so every sum has a
+// fixed order.  A cell's triangles are fans: a thread keeps the fan's first
+// and last vertex and makes one new vertex per triangle.
+//
+// Bound by instruction issue (384^3: 74 % of the slots busy, DRAM 6 %); most
+// of it is the cut cells' vertices and areas.  Against summing every cell's
+// corners as one 4-bit lane per field and queueing triangles: 512^3 spheres
+// 7.40 -> 1.03 ms for the seven fields, 1024^3 58.6 -> 8.3; 200 x 181 x 190
+// one field 146 -> 69 us.  U rows in flight hide the loads; more cost
+// registers and so blocks per SM.
 template <bool LABELS>
-__global__ void __launch_bounds__(NT, 4) alpha_kernel(AlphaArgs A)
+__global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
 {
-    __shared__ uint32_t s_w[3][PH * PW];
-    __shared__ McTable s_tab;
-    __shared__ uint2 s_q[QCAP];     // x: corner counts, y: tx | cy << 5 | kk << 9 | fields << 14 | t << 21 | cube << 24
-    __shared__ int s_warp[NT / 32];
-    __shared__ double s_red[kFields][NT / 32];
     constexpr int NF = LABELS ? kFields : 1;
+    __shared__ uint64_t s_v[NF][VROWS];
+    __shared__ uint64_t s_below[CROWS];
+    __shared__ PackedCase s_tab[256];
+    __shared__ float s_t[kTSize];
+    __shared__ EdgeInfo s_edge[12];
+    __shared__ uint16_t s_q[QCAP];  // c | row << 6
+    __shared__ int s_warp[NT / 32];
+    __shared__ float2 s_red[NT / 32];
+    __shared__ uint32_t s_differ;
 
-    reinterpret_cast<uint4 *>(&s_tab)[threadIdx.x] = reinterpret_cast<const uint4 *>(A.table)[threadIdx.x];
-
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tiles_xy = A.tiles_x * A.tiles_y;
     const int bz = blockIdx.x / tiles_xy;
     const int rem = blockIdx.x - bz * tiles_xy;
     const int by = rem / A.tiles_x, bx = rem - by * A.tiles_x;
-    const int i0 = bx * TX, j0 = by * TY, k0 = bz * A.zc;
-    const int k1 = min(k0 + A.zc, A.nz);
-    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    bool active[CY];
-#pragma unroll
-    for (int c = 0; c < CY; c++) active[c] = (i0 + tx) < A.nx && (j0 + ty + TYT * c) < A.ny;
-
-    int64_t off[NLOAD];
-#pragma unroll
-    for (int r = 0; r < NLOAD; r++) {
-        const int e = threadIdx.x + r * NT;
-        const int ly = e / PW, lx = e - ly * PW;
-        int gx = i0 - 1 + lx, gy = j0 - 1 + ly;
-        gx = gx < 0 ? 0 : (gx >= A.nx ? A.nx - 1 : gx);
-        gy = gy < 0 ? 0 : (gy >= A.ny ? A.ny - 1 : gy);
-        off[r] = (int64_t)gy * A.nx + gx;
+    const int i0 = bx * BX, j0 = by * BY, k0 = bz * A.zc;
+    const int nzc = min(A.zc, A.nz - k0);
+    s_tab[tid] = d_cases.at[tid];
+    if (tid < 81) {
+        const float fa = __fmul_rn((float)(tid / 9), 0.125f), fb = __fmul_rn((float)(tid % 9), 0.125f);
+        s_t[tid / 9 * 256 + tid % 9] = __fdiv_rn(__fsub_rn(A.iso, fa), __fsub_rn(fb, fa));
+    } else if (tid >= 128 && tid < 128 + 24) {
+        reinterpret_cast<uint4 *>(s_edge)[tid - 128] = reinterpret_cast<const uint4 *>(d_edges.at)[tid - 128];
     }
+    if (tid == 0) s_differ = 0;
 
-    double acc[NF];
+    // Voxel rows as bits: one warp per row, bit b = the voxel at x = i0 - 1 + b
+    // (clamped to the volume, as y and z).
+    const int rows = VY * (nzc + 2);
+    const int x0 = min(max(i0 - 1 + lane, 0), A.nx - 1), x1 = min(i0 + 31 + lane, A.nx - 1);
+    bool bad = false;
+    constexpr int U = LABELS ? 3 : 6;  // rows in flight per warp
+    for (int r0 = warp; r0 < rows; r0 += (NT / 32) * U) {
+        uint32_t m[U][2], l[U][2];
 #pragma unroll
-    for (int f = 0; f < NF; f++) acc[f] = 0.0;
-
-    auto flush = [&](int n) {
-        __syncthreads();
-        for (int q = threadIdx.x; q < n; q += NT) {
-            const uint2 it = s_q[q];
-            const int ctx = it.y & 31, cy = (it.y >> 5) & 15, kk = (it.y >> 9) & 31;
-            const int fields = (it.y >> 14) & 127, t = (it.y >> 21) & 7, cube = (it.y >> 24) & 255;
-            const float px = __fmul_rn(A.vx, (float)(i0 + ctx)), py = __fmul_rn(A.vy, (float)(j0 + cy));
-            const float pz = __fmul_rn(A.vz, (float)(k0 + kk));
-            const float a = triangle_area(s_tab, cube, t, it.x, A.iso, px, py, pz, __fadd_rn(px, A.vx),
-                                          __fadd_rn(py, A.vy), __fadd_rn(pz, A.vz));
-#pragma unroll
-            for (int g = 0; g < NF; g++)
-                if ((fields >> g) & 1) acc[g] += (double)a;
-        }
-        __syncthreads();
-    };
-
-    load_plane<LABELS>(A, s_w[(k0 + 2) % 3], off, k0 - 1);
-    load_plane<LABELS>(A, s_w[k0 % 3], off, k0);
-    __syncthreads();
-    // S[c][a + 2b] = sum of the 2x2 voxels around grid point (i + a, j + b)
-    // of cell row c, in one plane.
-    auto plane_sums = [&](int p, uint32_t S[CY][4]) {
-        const uint32_t *w = s_w[(p + 3) % 3];
-#pragma unroll
-        for (int c = 0; c < CY; c++) {
-            const int r0 = (ty + TYT * c) * PW + tx;
-#pragma unroll
-            for (int b = 0; b < 2; b++)
-#pragma unroll
-                for (int a = 0; a < 2; a++)
-                    S[c][a + 2 * b] = w[r0 + b * PW + a] + w[r0 + b * PW + a + 1] + w[r0 + (b + 1) * PW + a] +
-                                      w[r0 + (b + 1) * PW + a + 1];
-        }
-    };
-    uint32_t Sp[CY][4], Sc[CY][4], Sn[CY][4];
-    plane_sums(k0 - 1, Sp);
-    plane_sums(k0, Sc);
-
-    int queued = 0;  // block-uniform
-    for (int k = k0; k < k1; k++) {
-        __syncthreads();  // the slot of plane k - 2 is free
-        load_plane<LABELS>(A, s_w[(k + 1) % 3], off, k + 1);
-        __syncthreads();
-        plane_sums(k + 1, Sn);
-        // Corner counts per cell and field; fields with equal counts share
-        // their triangles (queued once with the set of fields they serve).
-        uint32_t cnt[CY][NF];
-        int mine_c[CY];
-        int mine = 0;
-#pragma unroll
-        for (int c = 0; c < CY; c++) {
-            uint32_t W[8];
-            W[0] = Sp[c][0] + Sc[c][0];
-            W[1] = Sp[c][1] + Sc[c][1];
-            W[2] = Sp[c][3] + Sc[c][3];
-            W[3] = Sp[c][2] + Sc[c][2];
-            W[4] = Sc[c][0] + Sn[c][0];
-            W[5] = Sc[c][1] + Sn[c][1];
-            W[6] = Sc[c][3] + Sn[c][3];
-            W[7] = Sc[c][2] + Sn[c][2];
-            bool flat = true;
-#pragma unroll
-            for (int q = 1; q < 8; q++) flat &= W[q] == W[0];
-            mine_c[c] = 0;
-#pragma unroll
-            for (int f = 0; f < NF; f++) cnt[c][f] = 0;
-            if (active[c] && !flat) {
-#pragma unroll
-                for (int f = 0; f < NF; f++) cnt[c][f] = field_counts(W, f);
-#pragma unroll
-                for (int f = 0; f < NF; f++) {
-                    bool dup = false;
-#pragma unroll
-                    for (int g = 0; g < f; g++) dup |= cnt[c][g] == cnt[c][f];
-                    if (!dup) mine_c[c] += s_tab.ntri[cube_of(cnt[c][f], A.thr)];
-                }
+        for (int u = 0; u < U; u++) {
+            const int r = min(r0 + u * (NT / 32), rows - 1);
+            const int zz = r / VY, yy = r - zz * VY;
+            const int gz = min(max(k0 - 1 + zz, 0), A.nz - 1), gy = min(max(j0 - 1 + yy, 0), A.ny - 1);
+            const int64_t base = ((int64_t)gz * A.ny + gy) * A.nx;
+            m[u][0] = __ldg(A.mask + base + x0);
+            m[u][1] = __ldg(A.mask + base + x1);
+            if (LABELS) {
+                l[u][0] = __ldg(A.labels + base + x0);
+                l[u][1] = __ldg(A.labels + base + x1);
             }
-            mine += mine_c[c];
         }
-        // Block-wide exclusive scan of the triangle counts.
-        int inc = mine;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        if (lane == 31) s_warp[warp] = inc;
-        __syncthreads();
-        int before = 0, total = 0;
+        for (int u = 0; u < U; u++) {
+            const int r = min(r0 + u * (NT / 32), rows - 1);
 #pragma unroll
-        for (int w = 0; w < NT / 32; w++) {
-            const int v = s_warp[w];
-            before += w < warp ? v : 0;
-            total += v;
-        }
-        const int off0 = before + inc - mine;
-        for (int base = 0; base < total; base += QCAP) {
-            const int chunk = min(total - base, QCAP);
-            if (queued + chunk > QCAP) {
-                flush(queued);
-                queued = 0;
-            }
-            if (mine && off0 + mine > base && off0 < base + chunk) {
-                int idx = off0;
+            for (int h = 0; h < 2; h++) bad |= m[u][h] != 0 && m[u][h] != 255;
+            const uint32_t s0 = __ballot_sync(0xffffffffu, m[u][0] != 0), s1 = __ballot_sync(0xffffffffu, m[u][1] != 0);
+            uint32_t w0 = s0, w1 = s1;
+            if (LABELS) {
+                const uint32_t c0 = __ldg(A.label_bits + l[u][0]), c1 = __ldg(A.label_bits + l[u][1]);
+                // Nearly every row's labelled voxels belong to components that
+                // touch the same faces: one ballot then serves all of them.
+                const uint32_t q = __reduce_or_sync(0xffffffffu, c0 | c1);
+                if (__all_sync(0xffffffffu, (c0 == 0 || c0 == q) && (c1 == 0 || c1 == q))) {
+                    const uint32_t b0 = __ballot_sync(0xffffffffu, c0 != 0), b1 = __ballot_sync(0xffffffffu, c1 != 0);
+                    if (lane < kFields - 1) {
+                        w0 = (q >> lane) & 1u ? b0 : 0u;
+                        w1 = (q >> lane) & 1u ? b1 : 0u;
+                    }
+                } else {
 #pragma unroll
-                for (int c = 0; c < CY; c++) {
-                    if (!mine_c[c]) continue;
-#pragma unroll
-                    for (int f = 0; f < NF; f++) {
-                        bool dup = false;
-                        uint32_t fields = 0;
-#pragma unroll
-                        for (int g = 0; g < NF; g++) {
-                            dup |= g < f && cnt[c][g] == cnt[c][f];
-                            fields |= (uint32_t)(g >= f && cnt[c][g] == cnt[c][f]) << g;
-                        }
-                        if (dup) continue;
-                        const int cube = cube_of(cnt[c][f], A.thr);
-                        const int nt = s_tab.ntri[cube];
-                        const uint32_t meta = (uint32_t)tx | (uint32_t)(ty + TYT * c) << 5 | (uint32_t)(k - k0) << 9 |
-                                              fields << 14 | (uint32_t)cube << 24;
-                        for (int t = 0; t < nt; t++, idx++) {
-                            if (idx >= base && idx < base + chunk)
-                                s_q[queued + idx - base] = make_uint2(cnt[c][f], meta | (uint32_t)t << 21);
+                    for (int f = 0; f < kFields - 1; f++) {
+                        const uint32_t b0 = __ballot_sync(0xffffffffu, (c0 >> f) & 1u);
+                        const uint32_t b1 = __ballot_sync(0xffffffffu, (c1 >> f) & 1u);
+                        if (lane == f) {
+                            w0 = b0;
+                            w1 = b1;
                         }
                     }
                 }
             }
-            queued += chunk;
+            if (lane < NF) s_v[lane][r] = (uint64_t)w1 << 32 | w0;
         }
-#pragma unroll
-        for (int c = 0; c < CY; c++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                Sp[c][q] = Sc[c][q];
-                Sc[c][q] = Sn[c][q];
-            }
     }
-    flush(queued);
-
-    // Block sums in a fixed order.
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-        double v = acc[f];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) s_red[f][warp] = v;
-    }
+    if (bad) *A.bad = 1;
     __syncthreads();
-    if (threadIdx.x < NF) {
-        double s = 0.0;
-        for (int w = 0; w < NT / 32; w++) s += s_red[threadIdx.x][w];
-        A.partials[(size_t)blockIdx.x * kFields + threadIdx.x] = s;
-    }
-}
 
-// One block sums the per-block partials of every field in a fixed order.
-__global__ void __launch_bounds__(NT) alpha_sum_kernel(const double *partials, int nblocks, double *out)
-{
-    __shared__ double s[NT];
-    for (int f = 0; f < kFields; f++) {
-        double v = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += NT) v += partials[(size_t)b * kFields + f];
-        s[threadIdx.x] = v;
+    // Fields equal to an earlier one over the whole brick.
+    if (LABELS) {
+        uint32_t differ = 0;  // bit of (f, g), f < g
+        for (int r = tid; r < rows; r += NT) {
+            uint64_t w[kFields];
+#pragma unroll
+            for (int f = 0; f < kFields; f++) w[f] = s_v[LABELS ? f : 0][r];
+            int bit = 0;
+#pragma unroll
+            for (int g = 1; g < kFields; g++)
+#pragma unroll
+                for (int f = 0; f < g; f++, bit++) differ |= (uint32_t)(w[f] != w[g]) << bit;
+        }
+        differ = __reduce_or_sync(0xffffffffu, differ);
+        if (lane == 0) atomicOr(&s_differ, differ);
         __syncthreads();
-        for (int w = NT / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    }
+    const uint32_t differ = s_differ;
+    const int bit0[kFields] = {0, 0, 1, 3, 6, 10, 15};  // first bit of the pairs (., g)
+
+    for (int f = 0; f < NF; f++) {
+        bool dup = false;
+        for (int e = 0; e < f; e++) dup |= !((differ >> (bit0[f] + e)) & 1u);
+        if (dup) continue;
+        const uint64_t *v = s_v[f];
+        for (int r = tid; r < (BY + 1) * (nzc + 1); r += NT) {
+            const int z = r / (BY + 1), y = r - z * (BY + 1);
+            const uint64_t *q = v + z * VY + y;
+            s_below[r] = below_word(sum2x2(q[0], q[1]), sum2x2(q[VY], q[VY + 1]), A.thr);
+        }
+        __syncthreads();
+        // One row of cells per thread: those with corners on both sides.
+        const int k = tid / BY, j = tid - k * BY;
+        uint64_t cut = 0;
+        if (k < nzc && j0 + j < A.ny) {
+            const int nc = min(BX, A.nx - i0);
+            uint64_t any = 0, all = ~0ull;
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const uint64_t w = s_below[(k + (h >> 1)) * (BY + 1) + j + (h & 1)];
+                any |= w | w >> 1;
+                all &= w & w >> 1;
+            }
+            cut = any & ~all & ((1ull << nc) - 1);
+        }
+        const int mine = __popcll(cut);
+        int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) s_warp[warp] = inc;
+        __syncthreads();
+        int at = inc - mine, total = 0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++) {
+            const int t = s_warp[w];
+            at += w < warp ? t : 0;
+            total += t;
+        }
+        PairSum acc;
+        for (int base = 0; base < total; base += QCAP) {
+            while (cut && at < base + QCAP) {
+                const int c = __ffsll((long long)cut) - 1;
+                cut &= cut - 1;
+                s_q[at - base] = (uint16_t)(c | tid << 6);
+                at++;
+            }
+            __syncthreads();
+            const int n = min(total - base, QCAP);
+            for (int q = tid; q < n; q += NT) {
+                const int it = s_q[q], c = it & 63, row = it >> 6;
+                const int ck = row / BY, cj = row - ck * BY;
+                const uint32_t cnt = cell_counts(v, cj, ck, c);
+                Cell C;
+                C.even = cnt & 0x0f0f0f0fu;
+                C.odd = (cnt >> 4) & 0x0f0f0f0fu;
+                const float lo[3] = {__fmul_rn(A.vx, (float)(i0 + c)), __fmul_rn(A.vy, (float)(j0 + cj)),
+                                     __fmul_rn(A.vz, (float)(k0 + ck))};
+                const float size[3] = {A.vx, A.vy, A.vz};
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    const float hi = __fadd_rn(lo[a], size[a]);
+                    C.p[a] = __float_as_uint(lo[a]);
+                    C.x[a] = __float_as_uint(lo[a]) ^ __float_as_uint(hi);
+                    C.d[a] = __fsub_rn(hi, lo[a]);
+                }
+                PackedCase pc = s_tab[cube_of(cnt, A.thr)];
+                int left = (int)(pc >> 60) - 2;
+                float3 v0 = vertex(C, s_t, s_edge, (int)pc & 15), v2 = vertex(C, s_t, s_edge, (int)(pc >> 4) & 15);
+                pc >>= 8;
+                for (; left > 0; left--, pc >>= 4) {
+                    int e = (int)pc & 15;
+                    if (e == kRestart) {
+                        v0 = vertex(C, s_t, s_edge, (int)(pc >> 4) & 15);
+                        v2 = vertex(C, s_t, s_edge, (int)(pc >> 8) & 15);
+                        pc >>= 12;
+                        left -= 3;
+                        e = (int)pc & 15;
+                    }
+                    const float3 v1 = v2;
+                    v2 = vertex(C, s_t, s_edge, e);
+                    acc.add(triangle_area(v0, v1, v2));
+                }
+            }
             __syncthreads();
         }
-        if (threadIdx.x == 0) out[f] = s[0];
+        // The brick's sum, in a fixed order.
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float s2 = __shfl_down_sync(0xffffffffu, acc.s, o), c2 = __shfl_down_sync(0xffffffffu, acc.c, o);
+            acc.add(s2, c2);
+        }
+        if (lane == 0) s_red[warp] = make_float2(acc.s, acc.c);
         __syncthreads();
+        if (tid < NF) {  // to every field of the group
+            bool same = tid == f;
+            if (tid > f) same = !((differ >> (bit0[tid] + f)) & 1u);
+            if (same) {
+                double sum = 0.0;
+                for (int w = 0; w < NT / 32; w++) sum += (double)s_red[w].x + (double)s_red[w].y;
+                A.partials[(size_t)tid * A.nblocks + blockIdx.x] = sum;
+            }
+        }
     }
 }
 
-std::once_flag g_table_once;
-McTable g_table;
+// One block per field sums its per-block partials in a fixed order.
+constexpr int NSUM = 1024;
+__global__ void __launch_bounds__(NSUM) alpha_sum_kernel(const double *partials, int nblocks, double *out)
+{
+    __shared__ double s[NSUM];
+    const double *p = partials + (size_t)blockIdx.x * nblocks;
+    double v = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nblocks; b += NSUM) v += p[b];
+    s[threadIdx.x] = v;
+    __syncthreads();
+    for (int w = NSUM / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = s[0];
+}
 
 int check_args(int64_t nx, int64_t ny, int64_t nz, float iso)
 {
@@ -497,7 +607,6 @@ int check_args(int64_t nx, int64_t ny, int64_t nz, float iso)
 int area_device(const uint8_t *d_mask, const uint32_t *d_labels, const uint8_t *d_bits, int64_t nx, int64_t ny,
                 int64_t nz, float iso, double *out, cudaStream_t st)
 {
-    std::call_once(g_table_once, [] { g_table = build_table(); });
     AlphaArgs A;
     memset(&A, 0, sizeof(A));
     A.mask = d_mask;
@@ -506,17 +615,18 @@ int area_device(const uint8_t *d_mask, const uint32_t *d_labels, const uint8_t *
     A.nx = (int)nx;
     A.ny = (int)ny;
     A.nz = (int)nz;
-    A.tiles_x = (int)((nx + TX - 1) / TX);
-    A.tiles_y = (int)((ny + TY - 1) / TY);
-    // z-slabs: 32 deep, halved while the grid has fewer than 8 blocks per SM.
+    A.tiles_x = (int)((nx + BX - 1) / BX);
+    A.tiles_y = (int)((ny + BY - 1) / BY);
+    // Bricks 16 cells deep, halved while the grid has fewer than 8 blocks per SM.
     int sms = 152, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t xy = (int64_t)A.tiles_x * A.tiles_y;
-    int zc = kMaxSlab;
+    int zc = BZ;
     while (zc > 1 && xy * ((nz + zc - 1) / zc) < 8LL * sms) zc /= 2;
     const int64_t nblocks = xy * ((nz + zc - 1) / zc);
     if (nblocks > INT32_MAX) return ft_fail(FAST_BAD_ARG, "volume too large for one area pass");
     A.zc = zc;
+    A.nblocks = nblocks;
     A.iso = iso;
     A.vx = 1.0f / (float)nx;
     A.vy = 1.0f / (float)ny;
@@ -524,29 +634,28 @@ int area_device(const uint8_t *d_mask, const uint32_t *d_labels, const uint8_t *
     A.thr = 9;
     for (int c = 8; c >= 0; c--)
         if ((float)c * 0.125f >= iso) A.thr = c;
+    const bool none = A.thr < 1 || A.thr > 8;  // no corner, or every corner, is below: no surface
+    if (none) A.thr = 8;
 
     const size_t part_bytes = (size_t)nblocks * kFields * sizeof(double);
     char *scratch = nullptr;
-    const size_t need = sizeof(McTable) + 256 + part_bytes + 256 + kFields * sizeof(double) + 256 + 16;
+    const size_t need = part_bytes + 256 + kFields * sizeof(double) + 256 + 16;
     cudaError_t e = cudaMallocAsync((void **)&scratch, need, st);
     if (e != cudaSuccess) return ft_fail(FAST_NOMEM, "area scratch: %s", cudaGetErrorString(e));
-    McTable *d_tab = (McTable *)scratch;
-    double *d_part = (double *)(scratch + sizeof(McTable) + 256);
+    double *d_part = (double *)scratch;
     double *d_out = (double *)((char *)d_part + part_bytes + 256);
     uint32_t *d_bad = (uint32_t *)((char *)d_out + kFields * sizeof(double) + 256);
-    A.table = d_tab;
     A.partials = d_part;
     A.bad = d_bad;
     double h_out[kFields];
     uint32_t h_bad = 0;
-    e = cudaMemcpyAsync(d_tab, &g_table, sizeof(McTable), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_bad, 0, sizeof(uint32_t), st);
+    e = cudaMemsetAsync(d_bad, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) {
         if (d_labels)
             alpha_kernel<true><<<(unsigned)nblocks, NT, 0, st>>>(A);
         else
             alpha_kernel<false><<<(unsigned)nblocks, NT, 0, st>>>(A);
-        alpha_sum_kernel<<<1, NT, 0, st>>>(d_part, (int)nblocks, d_out);
+        alpha_sum_kernel<<<d_labels ? kFields : 1, NSUM, 0, st>>>(d_part, (int)nblocks, d_out);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, d_out, sizeof(h_out), cudaMemcpyDeviceToHost, st);
@@ -556,11 +665,7 @@ int area_device(const uint8_t *d_mask, const uint32_t *d_labels, const uint8_t *
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return ft_fail(FAST_CUDA_ERROR, "area pass: %s", cudaGetErrorString(e));
     if (h_bad) return ft_fail(FAST_BAD_TYPE, "the volume must hold 0 and 255 only");
-    if (!d_labels) {
-        out[0] = h_out[0];
-    } else {
-        for (int f = 0; f < kFields; f++) out[f] = h_out[f];
-    }
+    for (int f = 0; f < (d_labels ? kFields : 1); f++) out[f] = none ? 0.0 : h_out[f];
     return FAST_OK;
 }
 
@@ -640,7 +745,6 @@ constexpr int kMeshBlock = 256;
 
 struct MeshArgs {
     const uint8_t *mask;
-    const McTable *table;
     int nx, ny, nz, thr;
     float iso, vx, vy, vz, dx;
 };
@@ -679,7 +783,7 @@ __global__ void __launch_bounds__(kMeshBlock) mesh_count_kernel(MeshArgs A, int6
     if (cell < ncell) {
         int cube, i, j, k;
         mesh_counts(A, cell, cube, i, j, k);
-        nt = A.table->ntri[cube];
+        nt = d_table.ntri[cube];
     }
     s[threadIdx.x] = nt;
     __syncthreads();
@@ -699,7 +803,7 @@ __global__ void __launch_bounds__(kMeshBlock) mesh_emit_kernel(MeshArgs A, int64
     uint32_t cnt = 0, nt = 0;
     if (cell < ncell) {
         cnt = mesh_counts(A, cell, cube, i, j, k);
-        nt = A.table->ntri[cube];
+        nt = d_table.ntri[cube];
     }
     // exclusive scan of the counts in cell order (Hillis-Steele over the block)
     s[threadIdx.x] = nt;
@@ -720,7 +824,7 @@ __global__ void __launch_bounds__(kMeshBlock) mesh_emit_kernel(MeshArgs A, int64
     for (uint32_t t = 0; t < nt; t++) {
         float v[3][3];
         for (int q = 0; q < 3; q++) {
-            const int e = A.table->edge[cube][3 * t + q];
+            const int e = d_table.edge[cube][3 * t + q];
             const int ca = edge_a(e), cb = edge_b(e);
             const float fa = __fmul_rn((float)((cnt >> (4 * ca)) & 15u), 0.125f);
             const float fb = __fmul_rn((float)((cnt >> (4 * cb)) & 15u), 0.125f);
@@ -754,7 +858,6 @@ __global__ void __launch_bounds__(kMeshBlock) mesh_emit_kernel(MeshArgs A, int64
 int mesh_device(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, float iso, float *out, uint64_t capacity,
                 uint64_t *ntri, cudaStream_t st)
 {
-    std::call_once(g_table_once, [] { g_table = build_table(); });
     const int64_t ncell = nx * ny * nz;
     const int64_t nblocks = (ncell + kMeshBlock - 1) / kMeshBlock;
     if (nblocks > INT32_MAX) return ft_fail(FAST_BAD_ARG, "volume too large for the mesh export");
@@ -770,21 +873,16 @@ int mesh_device(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, float
     const int64_t maxdim = std::max(nx, std::max(ny, nz));
     A.dx = 1.0f / (float)maxdim;
     char *scratch = nullptr;
-    const size_t need = sizeof(McTable) + 256 + (size_t)nblocks * 4 + 256 + (size_t)nblocks * 8;
+    const size_t need = (size_t)nblocks * 4 + 256 + (size_t)nblocks * 8;
     cudaError_t e = cudaMallocAsync((void **)&scratch, need, st);
     if (e != cudaSuccess) return ft_fail(FAST_NOMEM, "mesh scratch: %s", cudaGetErrorString(e));
-    McTable *d_tab = (McTable *)scratch;
-    uint32_t *d_cnt = (uint32_t *)(scratch + sizeof(McTable) + 256);
+    uint32_t *d_cnt = (uint32_t *)scratch;
     uint64_t *d_off = (uint64_t *)((char *)d_cnt + ((size_t)nblocks * 4 + 255) / 256 * 256);
-    A.table = d_tab;
     std::vector<uint32_t> cnt((size_t)nblocks);
     std::vector<uint64_t> off((size_t)nblocks);
     int s = FAST_OK;
-    e = cudaMemcpyAsync(d_tab, &g_table, sizeof(McTable), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
-        mesh_count_kernel<<<(unsigned)nblocks, kMeshBlock, 0, st>>>(A, ncell, d_cnt);
-        e = cudaGetLastError();
-    }
+    mesh_count_kernel<<<(unsigned)nblocks, kMeshBlock, 0, st>>>(A, ncell, d_cnt);
+    e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_cnt, (size_t)nblocks * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     uint64_t total = 0;
