@@ -11,27 +11,37 @@
 //     rows 0..5.
 //
 // The reference gets that numbering from span labels merged by atomicMin and a
-// scan over root spans.  Here it comes from a union-find whose links always
-// point from a larger to a smaller linear index, so the root of every tree is
-// its component's minimum index; roots are then ranked by a two-level scan in
-// linear-index order.  Passes:
-//   1. rows: one warp per (y, z) row seeds parent[i] = first index of the
-//      voxel's x-run (ballot + count-leading-zeros over 32-voxel chunks);
-//   2. union: each foreground voxel joins its y-1 and z-1 neighbours, skipping
-//      a join already implied through the x-1 voxel (both x-1 voxels
-//      foreground); Rem's union with splicing, lock-free (compare-and-swap).
-//      Every stored parent is a run start, so afterwards a voxel points at
-//      a run start (its own or one joined to it);
-//   3. starts: one warp per row; every run start that is a root counts
-//      itself in its 8192-voxel chunk and sets its bit of a root bitmap,
-//      every other run start is pointed straight at its root;
+// scan over root spans.  Here it comes from a union-find over x-runs whose
+// links always point from a larger to a smaller linear index, so the root of
+// every tree is its component's minimum index; roots are then ranked by a
+// two-level scan in linear-index order.  Passes:
+//   1. bricks: one block per 64 x 8 x 8 brick holds its rows as 64-bit words
+//      and joins their runs in shared memory.  A run's node is named by its
+//      row and start in the brick, which order as linear indices do, so the
+//      local root is the run with the smallest index.  Kept in global memory:
+//      the words, every run's local root (16 bits, at slot start / 2 of its
+//      row: runs start at least two voxels apart) and which runs are local
+//      roots;
+//   2. merge: the joins across brick faces, between local roots; Rem's union
+//      with splicing, lock-free (compare-and-swap), on parents kept at the
+//      local roots' places of the label array;
+//   3. flatten: every local root that is a global root counts itself in its
+//      chunk of voxels and sets its bit of a root bitmap, every other one is
+//      pointed straight at its root;
 //   4. scan the chunk counts;
 //   5. rank: one block per chunk numbers the chunk's roots from the bitmap;
-//   6. relabel: labels[i] = label of parent[parent[i]] (the root: the run
-//      start's parent), 0 on the background;
+//   6. relabel: a brick fetches the labels of its local roots, then writes
+//      every voxel's (0 on the background);
 //   7. face bitmaps, 8. the all-faces AND.
 // Every loop terminates: a find follows strictly decreasing indices, and a
 // failed link continues from a strictly smaller index.
+//
+// Joining voxels in global memory was bound by dependent loads: most joins
+// are inside a brick, where shared memory answers in a few dozen cycles, and
+// about one in five is left for pass 2.  768 x 700 x 720 spheres: 5.92 ms of
+// kernels -> 1.30 (pass 1 0.57, issue bound; pass 2 0.25; pass 6 0.37, 4.2 TB/s
+// of labels); 1024^3 17.3 -> 3.7 ms.  Scratch is 1.2 bytes per voxel (4.1
+// with a parent per voxel) for volumes at least 64 voxels wide.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -41,12 +51,56 @@
 namespace ft {
 namespace {
 
-constexpr uint32_t kNone = 0xFFFFFFFFu;  // parent of a background voxel
-constexpr int kChunk = 8192;             // voxels per block in the ranking passes
-constexpr int kRankThreads = 256;        // one root-bitmap word (32 voxels) per thread
-static_assert(kChunk == kRankThreads * 32, "a rank block covers one chunk");
+constexpr int kChunk = 32768;      // voxels per block in the ranking pass
+constexpr int kRankThreads = 256;  // each takes kRankWords root-bitmap words (32 voxels)
+constexpr int kRankWords = 4;
+static_assert(kChunk == kRankThreads * kRankWords * 32, "a rank block covers one chunk");
 
-// Parent reads during the union and starts passes go through L1
+// Bricks: 64 voxels (one word) x RY x RZ rows.
+constexpr int RY = 8, RZ = 8, ROWS = RY * RZ;
+constexpr int kSlots = 32;          // runs of a word at most: slot = start / 2
+constexpr int kBrickThreads = 128;
+static_assert(RY == 8 && RZ == 8, "three join steps in y and in z");
+
+// Geometry of a labelling and its scratch arrays.
+struct Ccl {
+    int nx, ny, nz;
+    int wx, by, bz;    // words per row, bricks in y and z
+    int slots;         // slots kept per word
+    uint8_t bg;
+    const uint8_t *mask;
+    uint64_t *bits;    // [z][y][word]: foreground
+    uint16_t *local;   // [z][y][word][slot]: local root, row * 64 + start
+    uint32_t *roots;   // [z][y][word]: slots that are local roots
+    uint32_t *par;     // the label array: parents at the local roots' places
+    uint32_t *cnt, *root_bits;
+
+    __device__ int64_t word(int y, int z, int w) const { return ((int64_t)z * ny + y) * wx + w; }
+    __device__ uint32_t voxel(int x, int y, int z) const
+    {
+        return (uint32_t)x + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
+    }
+};
+
+// First bits of the word's runs.
+__device__ __forceinline__ uint64_t run_starts(uint64_t w) { return w & ~(w << 1); }
+
+// Start of the run that holds bit b of half h (0: bits 0..31) of a word.
+__device__ __forceinline__ int run_start(uint64_t starts, int h, int b)
+{
+    const uint32_t lo = (uint32_t)starts, hi = (uint32_t)(starts >> 32);
+    const uint32_t upto = 0xFFFFFFFFu >> (31 - b);
+    const uint32_t m = (h ? hi : lo) & upto;
+    return m ? 32 * h + 31 - __clz((int)m) : 31 - __clz((int)lo);
+}
+
+// Start bit of the run in a slot.
+__device__ __forceinline__ int slot_start(uint64_t starts, int slot)
+{
+    return 2 * slot + (int)((starts >> (2 * slot + 1)) & 1);
+}
+
+// Parent reads during the merge and flatten passes go through L1
 // (ld.global.ca): a read may return a stale parent written earlier in the
 // same pass by another SM, which is harmless.  Every value ever stored is a
 // pointer to a smaller index of the same component, so a walk that follows
@@ -75,8 +129,7 @@ __device__ __forceinline__ uint32_t find_root(const uint32_t *par, uint32_t a)
 // have the same parent, which for two voxels already in one component
 // usually happens well below the root.  Invariants: a parent never exceeds
 // its node (so a root is its tree's smallest index) and every stored parent
-// is a run start (a voxel inside a run is never anyone's parent), which the
-// starts and relabel passes rely on.  A link or splice that loses a race
+// is a local root, which the flatten and relabel passes rely on.  A link or splice that loses a race
 // only fails its compare-and-swap; a failed link hands back the node's
 // current parent, so a stale read cannot make the loop spin, and every
 // step moves a node to a strictly smaller index.
@@ -106,82 +159,221 @@ __device__ void unite(uint32_t *par, uint32_t x, uint32_t y)
     }
 }
 
-// Pass 1: one warp per row.
-__global__ void ccl_rows(const uint8_t *__restrict__ m, uint32_t *__restrict__ par, int nx, int64_t rows,
-                         uint8_t bg)
+// Root of a run of the brick; every second node on the way is pointed at its
+// grandparent (a plain store: it may undo a concurrent shortening, never a
+// link, since only roots are linked).
+__device__ __forceinline__ uint32_t find_local(volatile uint32_t *par, uint32_t u)
 {
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (row >= rows) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t base = (uint32_t)(row * nx);
-    uint32_t carry_start = 0;
-    uint32_t carry_fg = 0;
-    for (int x0 = 0; x0 < nx; x0 += 32) {
-        const int x = x0 + lane;
-        const bool fg = x < nx && m[(int64_t)base + x] != bg;
-        const uint32_t bfg = __ballot_sync(0xFFFFFFFFu, fg);
-        const uint32_t prev = (bfg << 1) | carry_fg;  // bit l: voxel x0+l-1 is foreground
-        const uint32_t bstart = bfg & ~prev;          // bit l: an x-run starts at x0+l
-        const uint32_t upto = lane == 31 ? 0xFFFFFFFFu : ((2u << lane) - 1u);
-        const uint32_t below = bstart & upto;
-        const uint32_t start = below ? (uint32_t)(x0 + 31 - __clz(below)) : carry_start;
-        if (x < nx) par[base + (uint32_t)x] = fg ? base + start : kNone;
-        carry_fg = bfg >> 31;
-        if (carry_fg) carry_start = bstart ? (uint32_t)(x0 + 31 - __clz(bstart)) : carry_start;
+    uint32_t p = par[u >> 1];
+    while (p != u) {
+        const uint32_t g = par[p >> 1];
+        if (g != p) par[u >> 1] = g;
+        u = p;
+        p = g;
+    }
+    return u;
+}
+
+// Joins two runs of the brick: the larger root is hung under the smaller; a
+// root that got a parent meanwhile is followed up.
+__device__ __forceinline__ void join_local(uint32_t *par, uint32_t u, uint32_t v)
+{
+    for (;;) {
+        u = find_local(par, u);
+        v = find_local(par, v);
+        if (u == v) return;
+        if (u < v) {
+            const uint32_t t = u;
+            u = v;
+            v = t;
+        }
+        const uint32_t old = atomicCAS(par + (u >> 1), u, v);
+        if (old == u) return;
+        u = old;
     }
 }
 
-// Pass 2: joins across y and z.
-__global__ void ccl_union(const uint8_t *__restrict__ m, uint32_t *par, int nx, int ny, int nz, uint8_t bg)
+// Pass 1: one brick per block.
+__global__ void __launch_bounds__(kBrickThreads) ccl_bricks(Ccl A)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= nx || y >= ny) return;
-    const uint32_t sy = (uint32_t)nx, sz = (uint32_t)nx * (uint32_t)ny;
-    for (int z = blockIdx.z; z < nz; z += gridDim.z) {
-        const uint32_t i = (uint32_t)x + sy * (uint32_t)y + sz * (uint32_t)z;
-        // The six mask bytes are loaded together (one round trip), not one
-        // behind the other's branch.
-        const uint8_t c = m[i];
-        const uint8_t l = x > 0 ? m[i - 1] : bg;
-        const uint8_t u = y > 0 ? m[i - sy] : bg;
-        const uint8_t ul = (x > 0 && y > 0) ? m[i - 1 - sy] : bg;
-        const uint8_t b = z > 0 ? m[i - sz] : bg;
-        const uint8_t bl = (x > 0 && z > 0) ? m[i - 1 - sz] : bg;
-        if (c == bg) continue;
-        const bool left = l != bg;
-        if (u != bg && !(left && ul != bg)) unite(par, i, i - sy);
-        if (b != bg && !(left && bl != bg)) unite(par, i, i - sz);
-    }
-}
+    __shared__ uint64_t s_bits[ROWS];
+    __shared__ uint32_t s_par[ROWS * kSlots];  // parent of the run in slot `node / 2`
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t b = blockIdx.x;
+    const int w = (int)(b % A.wx);
+    const int y0 = (int)(b / A.wx % A.by) * RY, z0 = (int)(b / A.wx / A.by) * RZ;
+    const int x0 = w * 64;
 
-// Pass 3: run starts.  A root (a start whose parent is itself) counts
-// itself in its chunk and sets its bit in the root bitmap; another start
-// gets its root as parent.  The other voxels of a run keep the start.
-__global__ void ccl_starts(const uint8_t *__restrict__ m, uint32_t *par, int nx, int64_t rows, uint8_t bg,
-                           uint32_t *chunk_cnt, uint32_t *root_bits)
-{
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (row >= rows) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t base = (uint32_t)(row * nx);
-    bool carry = false;  // voxel x0 - 1 is foreground
-    for (int x0 = 0; x0 < nx; x0 += 32) {
-        const int x = x0 + lane;
-        const bool fg = x < nx && m[base + x] != bg;
-        const unsigned fgm = __ballot_sync(0xFFFFFFFFu, fg);
-        const bool prev = lane == 0 ? carry : ((fgm >> (lane - 1)) & 1u) != 0;
-        carry = (fgm >> 31) & 1u;
-        if (fg && !prev) {
-            const uint32_t i = base + (uint32_t)x;
-            const uint32_t p = ld_par(par, i);
-            if (p == i) {
-                atomicAdd(chunk_cnt + i / (uint32_t)kChunk, 1u);
-                atomicOr(root_bits + (i >> 5), 1u << (i & 31u));
+    // A warp takes consecutive rows; all its loads are in flight together.
+    constexpr int PER = ROWS / (kBrickThreads / 32), U = 8;
+    const bool in0 = x0 + lane < A.nx, in1 = x0 + 32 + lane < A.nx;
+#pragma unroll
+    for (int k0 = 0; k0 < PER; k0 += U) {
+        uint8_t m[U][2];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int r = warp * PER + k0 + u;
+            const int y = y0 + r % RY, z = z0 + r / RY;
+            const uint8_t *row = A.mask + ((int64_t)z * A.ny + y) * A.nx + x0 + lane;
+            const bool in = y < A.ny && z < A.nz;
+            m[u][0] = in && in0 ? __ldg(row) : A.bg;
+            m[u][1] = in && in1 ? __ldg(row + 32) : A.bg;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t lo = __ballot_sync(0xFFFFFFFFu, m[u][0] != A.bg);
+            const uint32_t hi = __ballot_sync(0xFFFFFFFFu, m[u][1] != A.bg);
+            if (lane == 0) s_bits[warp * PER + k0 + u] = (uint64_t)hi << 32 | lo;
+        }
+    }
+    __syncthreads();
+    if (tid < ROWS) {
+        for (uint64_t o = run_starts(s_bits[tid]); o; o &= o - 1) {
+            const uint32_t v = (uint32_t)(tid * 64 + __ffsll((long long)o) - 1);
+            s_par[v >> 1] = v;
+        }
+    }
+    __syncthreads();
+
+    // Joins of neighbouring rows, one per stretch of voxels that both have, in
+    // six steps: rows 1, 3, 5, 7 of every plane with the row before, then 2
+    // and 6, then 4, then the planes likewise.  A step joins pairs of groups
+    // that nothing else touches, so trees stay shallow and links rarely race.
+    // A thread takes a quarter of a word, so the later steps leave whole warps
+    // out: most words hold one or two stretches.  (All rows at once, a thread per
+    // row, made chains as long as the brick and retried links: 35 us for one
+    // brick; as many pieces of a row as there are threads, 14,800 instructions
+    // per brick.)
+#pragma unroll 1
+    for (int step = 0; step < 6; step++) {
+        const int lvl = step % 3;         // lowest set bit of the row (plane) number
+        const int n = ROWS >> (lvl + 1);  // rows in this step
+        if (tid < 4 * n) {
+            const int q = tid % n, piece = tid / n, h = piece >> 1;
+            int r, to;
+            if (step < 3) {
+                const int per = RY >> (lvl + 1);
+                r = q / per * RY + ((2 * (q % per) + 1) << lvl);
+                to = r - 1;
             } else {
-                const uint32_t r = find_root(par, p);
-                if (r != p) par[i] = r;
+                r = ((2 * (q / RY) + 1) << lvl) * RY + q % RY;
+                to = r - RY;
             }
+            const uint64_t a = s_bits[r], c = s_bits[to];
+            const uint64_t both = run_starts(a & c), sa = run_starts(a), sc = run_starts(c);
+            const uint32_t half = (uint32_t)(h ? both >> 32 : both) & (piece & 1 ? 0xFFFF0000u : 0x0000FFFFu);
+            for (uint32_t o = half; o; o &= o - 1) {
+                const int bit = __ffs((int)o) - 1;
+                join_local(s_par, (uint32_t)(r * 64 + run_start(sa, h, bit)),
+                           (uint32_t)(to * 64 + run_start(sc, h, bit)));
+            }
+        }
+        __syncthreads();
+    }
+
+    if (tid < ROWS) {
+        const int y = y0 + tid % RY, z = z0 + tid / RY;
+        if (y < A.ny && z < A.nz) {
+            const int64_t at = A.word(y, z, w);
+            const uint64_t bits = s_bits[tid];
+            uint32_t roots = 0;
+            for (uint64_t o = run_starts(bits); o; o &= o - 1) {
+                const int start = __ffsll((long long)o) - 1;
+                const uint32_t u = (uint32_t)(tid * 64 + start);
+                uint32_t v = u, p;
+                while ((p = s_par[v >> 1]) != v) v = p;
+                A.local[at * A.slots + (start >> 1)] = (uint16_t)v;
+                if (u == v) {
+                    roots |= 1u << (start >> 1);
+                    const uint32_t i = A.voxel(x0 + start, y, z);
+                    A.par[i] = i;
+                }
+            }
+            A.bits[at] = bits;
+            A.roots[at] = roots;
+        }
+    }
+}
+
+// Linear index of the local root of the run that starts at bit `start` of a word.
+__device__ __forceinline__ uint32_t local_root(const Ccl &A, int y, int z, int w, int start)
+{
+    const uint32_t v = A.local[A.word(y, z, w) * A.slots + (start >> 1)];
+    const int r = (int)(v >> 6);
+    return A.voxel(w * 64 + (int)(v & 63u), y / RY * RY + r % RY, z / RZ * RZ + r / RY);
+}
+
+// Pass 2: joins across brick faces.  Tasks: every word with a word to its
+// left, every half word of the rows that begin a brick in y, and in z.
+__global__ void __launch_bounds__(256) ccl_merge(Ccl A, int64_t tasks_x, int64_t tasks_y, int64_t tasks_z)
+{
+    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < tasks_x) {
+        const int w = 1 + (int)(t % (A.wx - 1));
+        t /= A.wx - 1;
+        const int y = (int)(t % A.ny), z = (int)(t / A.ny);
+        const uint64_t a = A.bits[A.word(y, z, w)], c = A.bits[A.word(y, z, w - 1)];
+        if ((a & 1) && (c >> 63))
+            unite(A.par, local_root(A, y, z, w, 0), local_root(A, y, z, w - 1, run_start(run_starts(c), 1, 31)));
+        return;
+    }
+    t -= tasks_x;
+    int w, y, z, ty, tz;
+    const int h = (int)(t & 1);
+    t >>= 1;
+    if (t < tasks_y) {
+        w = (int)(t % A.wx);
+        t /= A.wx;
+        y = RY * (1 + (int)(t % (A.by - 1)));
+        z = (int)(t / (A.by - 1));
+        ty = y - 1;
+        tz = z;
+    } else {
+        t -= tasks_y;
+        if (t >= tasks_z) return;
+        w = (int)(t % A.wx);
+        t /= A.wx;
+        y = (int)(t % A.ny);
+        z = RZ * (1 + (int)(t / A.ny));
+        ty = y;
+        tz = z - 1;
+    }
+    const uint64_t a = A.bits[A.word(y, z, w)], c = A.bits[A.word(ty, tz, w)];
+    const uint64_t sa = run_starts(a), sc = run_starts(c);
+    uint32_t u0 = 0, v0 = 0;
+    bool any = false;
+    const uint64_t both = run_starts(a & c);
+    for (uint32_t o = (uint32_t)(h ? both >> 32 : both); o; o &= o - 1) {
+        const int bit = __ffs((int)o) - 1;
+        const uint32_t u = local_root(A, y, z, w, run_start(sa, h, bit));
+        const uint32_t v = local_root(A, ty, tz, w, run_start(sc, h, bit));
+        if (any && u == u0 && v == v0) continue;  // the pair just joined
+        unite(A.par, u, v);
+        u0 = u;
+        v0 = v;
+        any = true;
+    }
+}
+
+// Pass 3: local roots.  A global root (its own parent) counts itself in its
+// chunk and sets its bit in the root bitmap; another gets its root as parent.
+__global__ void __launch_bounds__(256) ccl_flatten(Ccl A, int64_t words)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= words) return;
+    uint32_t m = A.roots[t];
+    if (!m) return;
+    const uint64_t starts = run_starts(A.bits[t]);
+    const uint32_t row = (uint32_t)(t / A.wx) * (uint32_t)A.nx + (uint32_t)(t % A.wx) * 64u;
+    for (; m; m &= m - 1) {
+        const uint32_t i = row + (uint32_t)slot_start(starts, __ffs((int)m) - 1);
+        const uint32_t p = ld_par(A.par, i);
+        if (p == i) {
+            atomicAdd(A.cnt + i / (uint32_t)kChunk, 1u);
+            atomicOr(A.root_bits + (i >> 5), 1u << (i & 31u));
+        } else {
+            const uint32_t r = find_root(A.par, p);
+            if (r != p) A.par[i] = r;
         }
     }
 }
@@ -240,55 +432,90 @@ __global__ void __launch_bounds__(1024) ccl_scan_chunks(uint32_t *cnt, uint32_t 
     if (threadIdx.x == 1023) cnt[nchunks] = s[1023];
 }
 
-// Pass 5: label of every root = 1 + its rank.  One block per chunk, one
-// bitmap word (32 voxels) per thread.
-__global__ void __launch_bounds__(kRankThreads) ccl_rank(const uint32_t *__restrict__ root_bits, uint32_t nwords,
+// Pass 5: label of every root = 1 + its rank.  One block per chunk,
+// kRankWords neighbouring bitmap words per thread.
+__global__ void __launch_bounds__(kRankThreads) ccl_rank(const uint32_t *__restrict__ root_bits,
                                                          const uint32_t *__restrict__ chunk_off, uint32_t *labels)
 {
     __shared__ uint32_t s_warp[kRankThreads / 32 + 1];
-    const uint32_t w = blockIdx.x * (uint32_t)kRankThreads + threadIdx.x;
-    uint32_t bits = w < nwords ? root_bits[w] : 0u;
+    const uint32_t w = (blockIdx.x * (uint32_t)kRankThreads + threadIdx.x) * kRankWords;
+    uint32_t bits[kRankWords], mine = 0;
+#pragma unroll
+    for (int k = 0; k < kRankWords; k++) {
+        bits[k] = root_bits[w + k];
+        mine += (uint32_t)__popc(bits[k]);
+    }
     uint32_t total;
-    uint32_t r = chunk_off[blockIdx.x] + block_exclusive_scan((uint32_t)__popc(bits), s_warp, total) + 1u;
-    while (bits) {
-        const uint32_t k = (uint32_t)(__ffs(bits) - 1);
-        labels[w * 32u + k] = r++;
-        bits &= bits - 1u;
+    uint32_t r = chunk_off[blockIdx.x] + block_exclusive_scan(mine, s_warp, total) + 1u;
+#pragma unroll
+    for (int k = 0; k < kRankWords; k++) {
+        while (bits[k]) {
+            labels[(w + k) * 32u + (uint32_t)(__ffs((int)bits[k]) - 1)] = r++;
+            bits[k] &= bits[k] - 1u;
+        }
     }
 }
 
-// Pass 6: every other voxel: 0 on the background, else the label of its
-// root, which is its parent's parent (a run start points at its root, a
-// root at itself).  Roots were labelled by pass 5 and are not written here.
-// Four voxels a thread per step, their loads issued together.  A root's
-// label is read through the non-coherent L1 path: one component can own
-// most of the volume, and its root's label, read by every one of its
-// voxels, would otherwise be one L2 line hit by every SM.  Root entries
-// were written by the rank pass and are not written here (only non-root
-// entries are), so the cached values are current.
-__global__ void ccl_relabel(const uint32_t *__restrict__ par, uint32_t n, uint32_t *labels)
+// Pass 6: labels, in place of the parents.  A local root's place holds its
+// label if it is a global root (pass 5), else its root's index.  A block
+// reads its own local roots before it writes, and other blocks read only the
+// places of global roots, where a block writes the label that is already
+// there.  Reads go through L1: one component can own most of the volume, and
+// every brick fetches its root's label.
+__global__ void __launch_bounds__(kBrickThreads) ccl_relabel(Ccl A)
 {
-    constexpr int U = 4;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
-        uint32_t p[U], r[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const uint64_t i = i0 + u * stride;
-            p[u] = i < n ? __ldg(par + i) : kNone;
+    __shared__ uint64_t s_bits[ROWS];
+    __shared__ uint32_t s_label[ROWS * kSlots];  // of the local roots, then of every run
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t b = blockIdx.x;
+    const int w = (int)(b % A.wx);
+    const int y0 = (int)(b / A.wx % A.by) * RY, z0 = (int)(b / A.wx / A.by) * RZ;
+    const int x0 = w * 64;
+    const int ry = tid % RY, rz = tid / RY;
+    const bool mine = tid < ROWS && y0 + ry < A.ny && z0 + rz < A.nz;  // a row per thread
+    int64_t at = 0;
+    uint64_t starts = 0;
+    if (mine) {
+        at = A.word(y0 + ry, z0 + rz, w);
+        const uint64_t bits = __ldg(A.bits + at);
+        s_bits[tid] = bits;
+        starts = run_starts(bits);
+        for (uint32_t m = __ldg(A.roots + at); m; m &= m - 1) {
+            const int slot = __ffs((int)m) - 1;
+            const uint32_t i = A.voxel(x0 + slot_start(starts, slot), y0 + ry, z0 + rz);
+            const bool root = (__ldg(A.root_bits + (i >> 5)) >> (i & 31u)) & 1u;
+            uint32_t v = ld_par(A.par, i);
+            if (!root) v = ld_par(A.par, v);
+            s_label[tid * kSlots + slot] = v;
         }
+    }
+    __syncthreads();
+    // A run that is no local root takes its root's label (roots' entries are
+    // not written here).
+    for (uint64_t o = starts; o; o &= o - 1) {
+        const int start = __ffsll((long long)o) - 1;
+        const uint32_t v = __ldg(A.local + at * A.slots + (start >> 1));
+        if (v != (uint32_t)(tid * 64 + start)) s_label[tid * kSlots + (start >> 1)] = s_label[v >> 1];
+    }
+    __syncthreads();
+    constexpr int PER = ROWS / (kBrickThreads / 32);
+    const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);
+    const bool in0 = x0 + lane < A.nx, in1 = x0 + 32 + lane < A.nx;
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const uint64_t i = i0 + u * stride;
-            r[u] = (p[u] != kNone && p[u] != i) ? __ldg(par + p[u]) : kNone;
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const uint64_t i = i0 + u * stride;
-            if (i >= n) break;
-            if (p[u] == kNone) labels[i] = 0u;
-            else if (r[u] != kNone) labels[i] = __ldg(labels + r[u]);
-        }
+    for (int k = 0; k < PER; k++) {
+        const int r = warp * PER + k, y = y0 + r % RY, z = z0 + r / RY;
+        if (y >= A.ny || z >= A.nz) continue;
+        const uint64_t row = s_bits[r], st = run_starts(row);
+        const uint32_t *lab = s_label + r * kSlots;
+        uint32_t *out = A.par + (A.voxel(x0, y, z) + (uint32_t)lane);
+        const uint32_t lo = (uint32_t)row, hi = (uint32_t)(row >> 32);
+        const uint32_t slo = (uint32_t)st, shi = (uint32_t)(st >> 32);
+        // slot = start / 2; a run of the high half may start in the low one
+        const int s0 = (31 - __clz((int)(slo & upto))) >> 1;
+        const uint32_t mh = shi & upto;
+        const int s1 = (mh ? 63 - __clz((int)mh) : 31 - __clz((int)slo)) >> 1;
+        if (in0) out[0] = (lo >> lane) & 1u ? lab[s0] : 0u;
+        if (in1) out[32] = (hi >> lane) & 1u ? lab[s1] : 0u;
     }
 }
 
@@ -343,41 +570,51 @@ int check_dims(int64_t nx, int64_t ny, int64_t nz)
     return FAST_OK;
 }
 
-// Scratch words of a labelling beside the parent array: the chunk counts
-// (nchunks + 1) and the root bitmap (one bit per voxel).
-size_t scratch_words(uint32_t n)
+// Geometry and scratch plan of a labelling; `base` null: sizes only.
+// Returns the scratch bytes: 8 + 2 x slots + 4 per 64-voxel word, one bit per
+// voxel and one count per chunk (1.2 bytes per voxel of a wide volume).
+size_t plan(Ccl &A, char *base, size_t &zero_off, size_t &zero_bytes)
 {
+    const size_t words = (size_t)A.wx * A.ny * A.nz;
+    const size_t n = (size_t)A.nx * A.ny * A.nz;
     const size_t nchunks = (n + kChunk - 1) / kChunk;
-    return nchunks + 1 + nchunks * (kChunk / 32);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off += (bytes + 255) / 256 * 256;
+        return p;
+    };
+    A.bits = (uint64_t *)take(words * 8);
+    A.local = (uint16_t *)take(words * A.slots * 2);
+    A.roots = (uint32_t *)take(words * 4);
+    zero_off = off;
+    A.cnt = (uint32_t *)take((nchunks + 1) * 4);
+    A.root_bits = (uint32_t *)take(nchunks * (kChunk / 32) * 4);
+    zero_bytes = off - zero_off;
+    return off;
 }
 
-// Labels of d_mask into d_labels (device, N uint32) on `st`, using d_par
-// (device, N uint32) and d_scr (device, scratch_words(N) uint32) as scratch.
-int label_device(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint8_t bg, uint32_t *d_labels,
-                 uint32_t *d_par, uint32_t *d_scr, uint32_t *num_labels, cudaStream_t st)
+// Labels of A.mask into A.par (device, N uint32) on `st`; scratch planned.
+int label_device(const Ccl &A, char *scratch, size_t zero_off, size_t zero_bytes, uint32_t *num_labels,
+                 cudaStream_t st)
 {
-    const uint32_t n = (uint32_t)(nx * ny * nz);
-    const int64_t rows = ny * nz;
-    const uint32_t nchunks = (n + kChunk - 1) / kChunk;
-    uint32_t *d_cnt = d_scr, *d_bits = d_scr + nchunks + 1;
-    CK(cudaMemsetAsync(d_scr, 0, scratch_words(n) * 4, st));
-    ccl_rows<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(d_mask, d_par, (int)nx, rows, bg);
-    const dim3 ub(32, 8, 1);
-    // At most 128 grid layers in z, each thread striding over nz/128 planes:
-    // 1024^3 labelling 18.2 ms against 19.0 with one layer per plane (24.5
-    // with 32 layers, 35.5 with 8: fewer threads, fewer joins in flight).
-    const dim3 ug((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)(nz < 128 ? nz : 128));
-    ccl_union<<<ug, ub, 0, st>>>(d_mask, d_par, (int)nx, (int)ny, (int)nz, bg);
-    ccl_starts<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(d_mask, d_par, (int)nx, rows, bg, d_cnt, d_bits);
-    ccl_scan_chunks<<<1, 1024, 0, st>>>(d_cnt, nchunks);
-    ccl_rank<<<nchunks, kRankThreads, 0, st>>>(d_bits, (n + 31) / 32, d_cnt, d_labels);
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ccl_relabel<<<(unsigned)sms * 8u, 256, 0, st>>>(d_par, n, d_labels);
+    const size_t n = (size_t)A.nx * A.ny * A.nz;
+    const uint32_t nchunks = (uint32_t)((n + kChunk - 1) / kChunk);
+    const int64_t words = (int64_t)A.wx * A.ny * A.nz;
+    const int64_t bricks = (int64_t)A.wx * A.by * A.bz;
+    CK(cudaMemsetAsync(scratch + zero_off, 0, zero_bytes, st));
+    ccl_bricks<<<(unsigned)bricks, kBrickThreads, 0, st>>>(A);
+    const int64_t tx = (int64_t)(A.wx - 1) * A.ny * A.nz, ty = (int64_t)A.wx * (A.by - 1) * A.nz,
+                  tz = (int64_t)A.wx * A.ny * (A.bz - 1);
+    const int64_t tasks = tx + 2 * (ty + tz);
+    if (tasks > 0) ccl_merge<<<(unsigned)((tasks + 255) / 256), 256, 0, st>>>(A, tx, ty, tz);
+    ccl_flatten<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(A, words);
+    ccl_scan_chunks<<<1, 1024, 0, st>>>(A.cnt, nchunks);
+    ccl_rank<<<nchunks, kRankThreads, 0, st>>>(A.root_bits, A.cnt, A.par);
+    ccl_relabel<<<(unsigned)bricks, kBrickThreads, 0, st>>>(A);
     CK(cudaGetLastError());
     uint32_t roots = 0;
-    CK(cudaMemcpyAsync(&roots, d_cnt + nchunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&roots, A.cnt + nchunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     *num_labels = roots + 1u;
     return FAST_OK;
@@ -408,20 +645,28 @@ int boundary_device(const uint32_t *d_labels, int64_t nx, int64_t ny, int64_t nz
 int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint8_t bg, uint32_t *d_labels,
                  uint32_t *num_labels, uint8_t *boundary, uint64_t boundary_cap, cudaStream_t st)
 {
-    const uint32_t n = (uint32_t)(nx * ny * nz);
     int dev = 0;
     CK(cudaGetDevice(&dev));
     ft_retain_pool_memory(dev);
-    uint32_t *d_par = nullptr, *d_cnt = nullptr;
-    CK(cudaMallocAsync((void **)&d_par, (size_t)n * 4, st));
-    cudaError_t e = cudaMallocAsync((void **)&d_cnt, scratch_words(n) * 4, st);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(d_par, st);
-        return ft_fail(FAST_NOMEM, "labelling scratch: %s", cudaGetErrorString(e));
-    }
-    int s = label_device(d_mask, nx, ny, nz, bg, d_labels, d_par, d_cnt, num_labels, st);
-    cudaFreeAsync(d_par, st);
-    cudaFreeAsync(d_cnt, st);
+    Ccl A = {};
+    A.nx = (int)nx;
+    A.ny = (int)ny;
+    A.nz = (int)nz;
+    A.wx = (int)((nx + 63) / 64);
+    A.by = (int)((ny + RY - 1) / RY);
+    A.bz = (int)((nz + RZ - 1) / RZ);
+    A.slots = nx >= 64 ? kSlots : (int)((nx + 1) / 2);
+    A.bg = bg;
+    A.mask = d_mask;
+    A.par = d_labels;
+    size_t zero_off = 0, zero_bytes = 0;
+    const size_t need = plan(A, nullptr, zero_off, zero_bytes);
+    char *scratch = nullptr;
+    cudaError_t e = cudaMallocAsync((void **)&scratch, need, st);
+    if (e != cudaSuccess) return ft_fail(FAST_NOMEM, "labelling scratch: %s", cudaGetErrorString(e));
+    plan(A, scratch, zero_off, zero_bytes);
+    int s = label_device(A, scratch, zero_off, zero_bytes, num_labels, st);
+    cudaFreeAsync(scratch, st);
     if (s == FAST_OK && boundary) {
         if (boundary_cap < (uint64_t)7 * *num_labels)
             s = ft_fail(FAST_BAD_ARG, "boundary buffer holds %llu bytes, 7 x %u needed",
