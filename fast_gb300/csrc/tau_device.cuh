@@ -563,16 +563,20 @@ __device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, d
     }
 }
 
-// Arrival of a block at the end of a kernel.  Returns true (block-uniform)
-// in the last block to arrive for this job; that block then sums all
-// partials of the job, in a fixed order.
+// Arrival of a block at the end of a kernel, after block_sum_store: one
+// release by the first warp, whose lanes wrote the block's partial sums (the
+// vectors a block wrote are for the next kernel; the finisher does not read
+// them).  Returns true (block-uniform) in the last block to arrive for this
+// job; that block then sums all partials of the job, in a fixed order.
 __device__ __forceinline__ bool arrive_last(uint32_t *counter, int64_t ntiles, int *s_flag)
 {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t prev = atomicAdd(counter, 1u);
-        *s_flag = (prev == (uint32_t)(ntiles - 1)) ? 1 : 0;
+    if (threadIdx.x < 32) {
+        __syncwarp();
+        if (threadIdx.x == 0) {
+            uint32_t prev;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+            *s_flag = (prev == (uint32_t)(ntiles - 1)) ? 1 : 0;
+        }
     }
     __syncthreads();
     return *s_flag != 0;
@@ -582,7 +586,6 @@ template <int NV, int NT = NTHREADS>
 __device__ __forceinline__ void sum_partials(const double *part, int64_t ntiles, double (&tot)[NV], double *s_red)
 {
     const int tid = threadIdx.x;
-    __threadfence();
     double v[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = 0.0;
