@@ -93,7 +93,7 @@ struct Coef<float> {
     const float2 *bnd;  // Job::bnd
     float face[2][2];
     float cell2[2];
-    float2 di[NBC][128];  // {diag, 1/diag} by (boundary count + 2, code)
+    alignas(16) float2 di[NBC][128];  // {diag, 1/diag} by (boundary count + 2, code)
 };
 
 // The six face coefficients of each stencil code (X+, X-, Y+, Y-, Z+, Z-):
@@ -115,9 +115,12 @@ __device__ __forceinline__ void load_face_table(FaceTable &t, const Job &J, int 
     }
 }
 
-// Fills the block's coefficient tables; nt = the block's threads.
-template <typename T>
-__device__ __forceinline__ void load_coef(Coef<T> &C, const Job &J, int tid, int nt = NTHREADS)
+// Fills the block's coefficient tables; NT = the block's threads.  Every
+// thread's loads are issued together: a block of a small launch lives for a
+// few planes, and loading the FP32 table entry by entry took 4400 of its
+// 23,000 cycles (48^3 MIXED CG).
+template <typename T, int NT = NTHREADS>
+__device__ __forceinline__ void load_coef(Coef<T> &C, const Job &J, int tid)
 {
     if (tid == 0) C.bnd = static_cast<decltype(C.bnd)>(J.bnd);
     if constexpr (sizeof(T) == 8) {
@@ -128,8 +131,15 @@ __device__ __forceinline__ void load_coef(Coef<T> &C, const Job &J, int tid, int
         if (tid < 4) C.face[tid >> 1][tid & 1] = J.dface[tid >> 1][tid & 1];
         if (tid < 2) C.cell2[tid] = 2.0 * J.dcell[tid];
     } else {
-        for (int k = tid; k < NBC * 128; k += nt)
-            C.di[k >> 7][k & 127] = make_float2(J.fdiag_b[k >> 7][k & 127], J.finv_b[k >> 7][k & 127]);
+        constexpr int N = NBC * 128 / 2, PER = (N + NT - 1) / NT;  // pairs of entries
+        const float4 *src = reinterpret_cast<const float4 *>(&J.fdi[0][0][0]);
+        float4 v[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (tid + k * NT < N) v[k] = __ldg(src + tid + k * NT);
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (tid + k * NT < N) reinterpret_cast<float4 *>(&C.di[0][0])[tid + k * NT] = v[k];
         if (tid < 4) C.face[tid >> 1][tid & 1] = J.fface[tid >> 1][tid & 1];
         if (tid < 2) C.cell2[tid] = (float)(2.0 * J.dcell[tid]);
     }
@@ -145,9 +155,9 @@ struct Coef<FF> {
 };
 
 template <>
-__device__ __forceinline__ void load_coef<FF>(Coef<FF> &C, const Job &J, int tid, int nt)
+__device__ __forceinline__ void load_coef<FF>(Coef<FF> &C, const Job &J, int tid)
 {
-    for (int k = tid; k < NBC * 128; k += nt) {
+    for (int k = tid; k < NBC * 128; k += NTHREADS) {
         C.dhi[k >> 7][k & 127] = J.xdiag_hi[k >> 7][k & 127];
         C.dlo[k >> 7][k & 127] = J.xdiag_lo[k >> 7][k & 127];
     }
@@ -541,10 +551,7 @@ __device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, d
                 const float c2 = __shfl_down_sync(0xffffffffu, c, o);
                 pair_add(a, c, a2, c2);
             }
-            if (lane == 0) {
-                s_red[k * 2 * NW + warp] = (double)a;
-                s_red[k * 2 * NW + NW + warp] = (double)c;
-            }
+            if (lane == 0) reinterpret_cast<float2 *>(s_red)[k * NW + warp] = make_float2(a, c);
         }
     }
     __syncthreads();
@@ -556,7 +563,10 @@ __device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, d
         } else {
             float s = 0.f, c = 0.f;
 #pragma unroll
-            for (int w = 0; w < NW; w++) pair_add(s, c, (float)s_red[tid * 2 * NW + w], (float)s_red[tid * 2 * NW + NW + w]);
+            for (int w = 0; w < NW; w++) {
+                const float2 p = reinterpret_cast<const float2 *>(s_red)[tid * NW + w];
+                pair_add(s, c, p.x, p.y);
+            }
             a = (double)s + (double)c;
         }
         out[tid] = a;
@@ -589,15 +599,55 @@ __device__ __forceinline__ void sum_partials(const double *part, int64_t ntiles,
     double v[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = 0.0;
-    for (int64_t t = tid; t < ntiles; t += NT) {
+    constexpr int U = 4;  // partials in flight per thread, added in order
+    for (int64_t t0 = tid; t0 < ntiles; t0 += U * NT) {
+        double p[U][NV];
 #pragma unroll
-        for (int k = 0; k < NV; k++) v[k] += __ldcg(part + t * NPART + k);
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                p[u][k] = t0 + u * NT < ntiles ? __ldcg(part + (t0 + u * NT) * NPART + k) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (t0 + u * NT < ntiles) {
+#pragma unroll
+                for (int k = 0; k < NV; k++) v[k] += p[u][k];
+            }
     }
     __shared__ double s_tot[NV];
     block_sum_store<NV, double, NT>(v, s_tot, s_red);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NV; k++) tot[k] = s_tot[k];
+}
+
+// The finisher's work in the last block of a job: the partial sums, then
+// Op::finish on a copy of the job's scalars in shared memory.  The copy is
+// loaded beside the partial sums and written back at once; in global memory
+// each of finish's branches waited for the fields it reads (8000 cycles for
+// MIXED CG step 2, 3500 now).  No other block of the job touches the scalars
+// then: all have arrived.
+template <class Op, int NV, int NT = NTHREADS>
+__device__ __forceinline__ void finish_job(const Launch &L, const Job &J, double *s_red)
+{
+    __shared__ Scalars s_sc;
+    constexpr int W = (int)(sizeof(Scalars) / 4);
+    static_assert(sizeof(Scalars) % 8 == 0 && W <= NT, "one word per thread");
+    const int tid = threadIdx.x;
+    uint32_t w = 0;
+    if (tid < W) w = __ldcg(reinterpret_cast<const uint32_t *>(J.sc) + tid);
+    double tot[NV];
+    sum_partials<NV, NT>(J.part, J.ntiles, tot, s_red);
+    if (tid < W) reinterpret_cast<uint32_t *>(&s_sc)[tid] = w;
+    __syncthreads();
+    if (tid == 0) {
+        for (int k = 0; k < NV && k < 4; k++) s_sc.dbg[k] = tot[k];
+        Op::finish(s_sc, tot);
+        *J.counter = 0u;
+        if (L.gate != nullptr && s_sc.replace != 0 && s_sc.state == RUNNING) *L.gate = 1u;
+    }
+    __syncthreads();
+    if (tid < W) reinterpret_cast<uint32_t *>(J.sc)[tid] = reinterpret_cast<const uint32_t *>(&s_sc)[tid];
 }
 
 // Locate the job of this block (jobs are laid out back to back by tile_base).

@@ -230,8 +230,8 @@ void fill_tables(Job &J, double d0, double d1, int face_mean)
         // face contributes 0 and a Dirichlet face -2 D_self.
         for (int bc = -2; bc <= 4; bc++) {
             const float d = df + Df[self] * (float)bc;
-            J.fdiag_b[bc + 2][code] = d;
-            J.finv_b[bc + 2][code] = 1.0f / d;
+            J.fdi[bc + 2][code][0] = d;
+            J.fdi[bc + 2][code][1] = 1.0f / d;
         }
     }
     // Float-float splits (hi = nearest float, lo = nearest float of the rest).

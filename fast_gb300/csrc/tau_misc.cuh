@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256) bnd_kernel(const Job *jobs, int j0, int j
 {
     __shared__ Coef<T> C;
     const Job &J = jobs[blockIdx.y == 0 ? j0 : (blockIdx.y == 1 ? j1 : j2)];
-    load_coef<T>(C, J, threadIdx.x, 256);
+    load_coef<T>(C, J, threadIdx.x);
     __syncthreads();
     const int e = blockIdx.x * 256 + threadIdx.x;
     const int miss = e >> 7;

@@ -81,15 +81,7 @@ __global__ void __launch_bounds__(NTHREADS) pointwise_kernel(Launch L)
     op.partials(v);
     if (!ft_in(J, local * NPART, local * NPART + NPART - 1, J.ntiles * NPART, OOB_PARTIALS)) return;
     block_sum_store<Op::NV, T>(v, J.part + local * NPART, s_red);
-    if (arrive_last(J.counter, J.ntiles, &s_flag)) {
-        double tot[Op::NV];
-        sum_partials<Op::NV>(J.part, J.ntiles, tot, s_red);
-        if (tid == 0) {
-            for (int k = 0; k < Op::NV && k < 4; k++) J.sc->dbg[k] = tot[k];
-            Op::finish(*J.sc, tot);
-            *J.counter = 0u;
-        }
-    }
+    if (arrive_last(J.counter, J.ntiles, &s_flag)) finish_job<Op, Op::NV>(L, J, s_red);
 }
 
 // A pair of neighbouring elements (even index: one vector load).

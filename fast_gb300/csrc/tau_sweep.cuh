@@ -368,7 +368,7 @@ __device__ __forceinline__ int sweep_body(const Launch &L, int64_t blk, int &qb,
         return SWEEP_IDLE;
     }
     const Job &J = L.jobs[s_job];
-    load_coef<T>(C, J, tid, NT);
+    load_coef<T, NT>(C, J, tid);
     Op::load_shared(S, J, tid);
 
     const Geo g{J.nx, J.ny, J.nz, J.dir >> 1, (J.dir & 1) ? -1 : 1, J.pitch};
@@ -615,16 +615,7 @@ __device__ __forceinline__ int sweep_body(const Launch &L, int64_t blk, int &qb,
     op.partials(v);
     if (!ft_in(J, local * NPART, local * NPART + NPART - 1, J.ntiles * NPART, OOB_PARTIALS)) return SWEEP_FAULT;
     block_sum_store<NV, RT, NT>(v, J.part + local * NPART, s_red);
-    if (arrive_last(J.counter, J.ntiles, &s_flag)) {
-        double tot[NV];
-        sum_partials<NV, NT>(J.part, J.ntiles, tot, s_red);
-        if (tid == 0) {
-            for (int k = 0; k < NV && k < 4; k++) J.sc->dbg[k] = tot[k];
-            Op::finish(*J.sc, tot);
-            *J.counter = 0u;
-            if (L.gate != nullptr && J.sc->replace != 0 && J.sc->state == RUNNING) *L.gate = 1u;
-        }
-    }
+    if (arrive_last(J.counter, J.ntiles, &s_flag)) finish_job<Op, NV, NT>(L, J, s_red);
     return SWEEP_DONE;
 }
 

@@ -129,8 +129,7 @@ struct Job {
     double dface[2][2];          // face coefficient by (self solid, neighbour solid)
     double dcell[2];             // cell diffusivity by solid bit (pore, solid)
     float fface[2][2];
-    float fdiag_b[7][128];       // FP32 diagonal by (boundary count + 2, code 7 bits)
-    float finv_b[7][128];        // 1/diag, FP32
+    alignas(16) float fdi[7][128][2];  // FP32 {diagonal, 1/diagonal} by (boundary count + 2, code 7 bits)
     double ddiag_int[128];       // interior diagonal, FP64
     double dinv_int[128];        // 1/diag, FP64
     // MIXED residual replacement in float-float (x64_ff): the FP64 values
