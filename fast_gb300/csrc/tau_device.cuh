@@ -529,9 +529,11 @@ __device__ __forceinline__ FF diag_ff(const Coef<FF> &C, uint32_t code, const Po
 
 // Sum NV per-thread values over the block (fixed tree) and store the block
 // totals, as doubles, to out[0..NV).  FP32 values are combined as
-// compensated (sum, error) pairs.  NT = the block's threads.
+// compensated (sum, error) pairs.  NT = the block's threads; those from
+// `live` on hold 0 (FP64: their warps skip the tree).
 template <int NV, typename V, int NT = NTHREADS>
-__device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, double *s_red /* [NV][2*NT/32] */)
+__device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, double *s_red /* [NV][2*NT/32] */,
+                                                int live = NT)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -540,8 +542,10 @@ __device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, d
     for (int k = 0; k < NV; k++) {
         if constexpr (sizeof(V) == 8) {
             double a = (double)v[k];
+            if (warp * 32 < live) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+            }
             if (lane == 0) s_red[k * 2 * NW + warp] = a;
         } else {
             float a = (float)v[k], c = 0.f;
@@ -615,7 +619,7 @@ __device__ __forceinline__ void sum_partials(const double *part, int64_t ntiles,
             }
     }
     __shared__ double s_tot[NV];
-    block_sum_store<NV, double, NT>(v, s_tot, s_red);
+    block_sum_store<NV, double, NT>(v, s_tot, s_red, ntiles < NT ? (int)ntiles : NT);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NV; k++) tot[k] = s_tot[k];

@@ -31,13 +31,10 @@ __global__ void __launch_bounds__(NTHREADS) pointwise_kernel(Launch L)
     __shared__ Coef<T> C;
     __shared__ double s_red[2 * Op::NV * (NTHREADS / 32)];
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        s_job = find_job(L, (int64_t)blockIdx.x);
-        s_go = L.jobs[s_job].sc->state == RUNNING ? 1 : 0;
-    }
+    if (tid == 0) s_job = find_job(L, (int64_t)blockIdx.x);
     __syncthreads();
-    if (!s_go) return;
     const Job &J = L.jobs[s_job];
+    if (tid == 0) s_go = J.sc->state == RUNNING ? 1 : 0;
     load_coef<T>(C, J, tid);
     const Geo g{J.nx, J.ny, J.nz, J.dir >> 1, (J.dir & 1) ? -1 : 1, J.pitch};
     const int64_t local = (int64_t)blockIdx.x - J.tile_base;
@@ -52,6 +49,7 @@ __global__ void __launch_bounds__(NTHREADS) pointwise_kernel(Launch L)
     Op op;
     op.init(J);
     __syncthreads();
+    if (!s_go) return;
     if (v0) {
         for (int z = z0; z < z1; z += U) {
             typename Op::Vals v[U];

@@ -293,13 +293,28 @@ struct GateRole<Op, std::void_t<decltype(Op::clears_gate)>> {
     static constexpr bool clears = Op::clears_gate;
 };
 
+// Operations that most launches find nothing to do for (Op::rare): their
+// blocks look before they prepare.
+template <class Op, class = void>
+struct Rare {
+    static constexpr bool value = false;
+};
+template <class Op>
+struct Rare<Op, std::void_t<decltype(Op::rare)>> {
+    static constexpr bool value = Op::rare;
+};
+
 // The sweep of one tile `blk` (a block index of the launch), shared by the
 // kernel entries below.  `qb` counts the planes this block has taken through
 // its stage ring so far (ring slot and mbarrier phase continue from it), and
 // `ready` tells whether the block's mbarriers are initialised; both carry
 // over when one block sweeps several tiles.  Returns SWEEP_DONE, SWEEP_IDLE
 // (the tile's right-hand side is not active; *idle_end = its last tile + 1)
-// or SWEEP_FAULT.
+// or SWEEP_FAULT.  WALK: the block goes on to other tiles.  It looks whether
+// the right-hand side is active before it prepares anything; a block of one
+// tile of an operation that is not rare prepares at the same time, so that
+// its start is two round trips to L2 (the job's pointers, then the scalars)
+// and not four.
 enum { SWEEP_DONE = 0, SWEEP_IDLE = 1, SWEEP_FAULT = 2 };
 
 // Rows per thread: an operation that names RPT = 2 sweeps its TX x TY tile
@@ -329,13 +344,14 @@ __host__ __device__ constexpr int sweep_threads()
 #define FAST_TAU_FULL_TILE 1
 #endif
 
-template <class Op, int NSTAGE>
+template <class Op, int NSTAGE, bool WALK>
 __device__ __forceinline__ int sweep_body(const Launch &L, int64_t blk, int &qb, bool &ready, int64_t *idle_end)
 {
     using T = typename Op::T;
     using SL = typename Op::SL;
     using V = typename Op::Vals;
     constexpr int NV = Op::NV;
+    constexpr bool LOOK = WALK || Rare<Op>::value;
     constexpr int SB = SL::stage_bytes();
     constexpr int RPT = RowsPerThread<Op>::n;
     constexpr int NT = sweep_threads<Op>();
@@ -356,18 +372,19 @@ __device__ __forceinline__ int sweep_body(const Launch &L, int64_t blk, int &qb,
     // The first sweep after the replacement slot re-arms the launch's gate
     // (before any block of it can arrive at the finisher, which may set it).
     if (GateRole<Op>::clears && L.gate != nullptr && blk == 0 && tid == 0) *L.gate = 0u;
-    __syncthreads();  // the previous tile of this block is done with the shared state
+    if (WALK) __syncthreads();  // the previous tile of this block is done with the shared state
     if (tid == 0) {
         s_job = find_job(L, blk);
-        s_go = Op::active(*L.jobs[s_job].sc) ? 1 : 0;
+        if (LOOK) s_go = Op::active(*L.jobs[s_job].sc) ? 1 : 0;
         s_err = 0;
     }
     __syncthreads();
-    if (!s_go) {
-        *idle_end = L.jobs[s_job].tile_base + L.jobs[s_job].ntiles;
+    const Job &J = L.jobs[s_job];
+    if (LOOK && !s_go) {
+        *idle_end = J.tile_base + J.ntiles;
         return SWEEP_IDLE;
     }
-    const Job &J = L.jobs[s_job];
+    if (!LOOK && tid == 0) s_go = Op::active(*J.sc) ? 1 : 0;
     load_coef<T, NT>(C, J, tid);
     Op::load_shared(S, J, tid);
 
@@ -401,14 +418,15 @@ __device__ __forceinline__ int sweep_body(const Launch &L, int64_t blk, int &qb,
     const uint32_t stage0 = (raw0 + 127u) & ~127u;
     unsigned char *const sbase = dsm + (stage0 - raw0);
     if (tid == 0) {
+#pragma unroll
+        for (int s = 0; s < SL::N; ++s) prefetch_tmap(op.tmap[s]);
         if (!ready)
             for (int s = 0; s < NSTAGE; ++s) mbar_init(smem_u32(&bars[s]), 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-        for (int s = 0; s < SL::N; ++s) prefetch_tmap(op.tmap[s]);
     }
     ready = true;
     __syncthreads();
+    if (!LOOK && !s_go) return SWEEP_IDLE;
     // Tile loads of plane pa+q into ring slot (qb + q) % NSTAGE (one thread:
     // thread 0 for the first NSTAGE planes, the refill thread after).
     auto issue = [&](int q) {
@@ -628,7 +646,7 @@ __global__ void __launch_bounds__(sweep_threads<Op>()) sweep_kernel(Launch L)
     int qb = 0;
     bool ready = false;
     int64_t idle_end;
-    sweep_body<Op, NSTAGE>(L, (int64_t)blockIdx.x, qb, ready, &idle_end);
+    sweep_body<Op, NSTAGE, false>(L, (int64_t)blockIdx.x, qb, ready, &idle_end);
 }
 
 template <class Op, int NSTAGE, int MB>
@@ -637,7 +655,7 @@ __global__ void __launch_bounds__(sweep_threads<Op>(), MB) sweep_kernel_mb(Launc
     int qb = 0;
     bool ready = false;
     int64_t idle_end;
-    sweep_body<Op, NSTAGE>(L, (int64_t)blockIdx.x, qb, ready, &idle_end);
+    sweep_body<Op, NSTAGE, false>(L, (int64_t)blockIdx.x, qb, ready, &idle_end);
 }
 
 // A resident grid that walks the launch's tiles (tile = blockIdx.x +
@@ -654,7 +672,7 @@ __global__ void __launch_bounds__(sweep_threads<Op>()) sweep_kernel_tiles(Launch
     bool ready = false;
     for (int64_t blk = blockIdx.x; blk < L.nblocks;) {
         int64_t idle_end = 0;
-        const int r = sweep_body<Op, NSTAGE>(L, blk, qb, ready, &idle_end);
+        const int r = sweep_body<Op, NSTAGE, true>(L, blk, qb, ready, &idle_end);
         if (r == SWEEP_FAULT) {
             // The stage ring of this block is unusable now: the right-hand
             // sides of the tiles it leaves undone cannot finish this step
@@ -1083,6 +1101,7 @@ struct OpBiRestart {
     static constexpr bool FB = sizeof(TT) == 4 && sizeof(ST) == 8;  // MIXED FP32 iterations
     using SL = Streams<sizeof(TT), 1>;
     static constexpr int NV = 1;
+    static constexpr bool rare = true;
     using Shared = NoShared;
     struct Vals { T x; uint32_t code; };
     struct Own { uint32_t code; };
