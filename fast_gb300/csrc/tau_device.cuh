@@ -527,6 +527,40 @@ __device__ __forceinline__ FF diag_ff(const Coef<FF> &C, uint32_t code, const Po
     return FF(C.dhi[p.bc + 2][code & 127], C.dlo[p.bc + 2][code & 127]);
 }
 
+// Sums of up to four values over a warp, the additions of lane 0 in
+// `a += shfl_down(a, 16), 8, 4, 2, 1`.  At each of the first levels two values
+// share one addition: half of the lanes hold what the tree still needs of the
+// one, half of the other.  FP64 additions are slow (a warp's takes 16 cycles
+// of the SM's pipe), and one value after the other took 5 NV of them in a
+// chain.  On return a[0] is the sum of value `k` for the k returned (-1: the
+// lane has none to give).
+template <int NV>
+__device__ __forceinline__ int warp_sums(double (&a)[NV], int lane)
+{
+    static_assert(NV >= 1 && NV <= 4, "one to four values");
+    auto merge = [&](double p, double q, int o) {  // lanes without bit o go on with p, with it with q
+        const bool hi = (lane & o) != 0;
+        const double other = __shfl_xor_sync(0xffffffffu, hi ? p : q, o);
+        return (hi ? q : p) + other;
+    };
+    int k = 0, o = 16;
+    if constexpr (NV >= 3) {
+        const double x = merge(a[0], a[1], 16);
+        const double y = merge(a[2], NV == 4 ? a[NV - 1] : 0.0, 16);
+        a[0] = merge(x, y, 8);
+        k = (lane & 16 ? 1 : 0) + (lane & 8 ? 2 : 0);
+        o = 4;
+    } else if constexpr (NV == 2) {
+        a[0] = merge(a[0], a[1], 16);
+        k = lane & 16 ? 1 : 0;
+        o = 8;
+    }
+#pragma unroll
+    for (int b = 16; b > 0; b >>= 1)
+        if (b <= o) a[0] += __shfl_xor_sync(0xffffffffu, a[0], b);
+    return (lane & (2 * o - 1)) == 0 && k < NV ? k : -1;
+}
+
 // Sum NV per-thread values over the block (fixed tree) and store the block
 // totals, as doubles, to out[0..NV).  FP32 values are combined as
 // compensated (sum, error) pairs.  NT = the block's threads; those from
@@ -538,16 +572,19 @@ __device__ __forceinline__ void block_sum_store(const V (&v)[NV], double *out, d
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     constexpr int NW = NT / 32;
+    if constexpr (sizeof(V) == 8) {
+        if (warp * 32 < live) {
+            double a[NV];
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
-        if constexpr (sizeof(V) == 8) {
-            double a = (double)v[k];
-            if (warp * 32 < live) {
+            for (int k = 0; k < NV; k++) a[k] = (double)v[k];
+            const int mine = warp_sums<NV>(a, lane);
+            if (mine >= 0) s_red[mine * 2 * NW + warp] = a[0];
+        } else if (lane < NV) {
+            s_red[lane * 2 * NW + warp] = 0.0;
+        }
+    } else {
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-            }
-            if (lane == 0) s_red[k * 2 * NW + warp] = a;
-        } else {
+        for (int k = 0; k < NV; k++) {
             float a = (float)v[k], c = 0.f;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
