@@ -463,7 +463,9 @@ size_t code_bytes(int64_t nx, int64_t ny, int64_t nz) { return align_up((size_t)
 // iterations at every candidate depth on a GB300), or from a table installed
 // at run time with fast_tau_set_slab_table.  A class without an entry uses
 // the full depth, halved (down to 2 planes) while the launch would give the
-// GPU fewer than kMinBlocks blocks.  FAST_TAU_ZC overrides all of it.
+// GPU fewer than kMinBlocks blocks.  A CG launch on the built-in table may
+// take another depth by a model of its waves of blocks (modelled_depth).
+// FAST_TAU_ZC overrides all of it.
 // slab_depth sizes a volume solved alone (one right-hand side, the serving
 // context's unit, so a served result equals the same request solved alone);
 // launch_slab_depth a whole launch.
@@ -471,6 +473,7 @@ size_t code_bytes(int64_t nx, int64_t ny, int64_t nz) { return align_up((size_t)
 
 namespace {
 std::atomic<int> g_slab[3][2][kSlabClasses];
+std::atomic<bool> g_slab_set[3][2];  // a table was installed at run time
 std::once_flag g_slab_once;
 
 void slab_init()
@@ -489,6 +492,77 @@ int slab_class(int64_t W)
     return c;
 }
 
+// A CG launch's time by its slab depth.  The table's classes are factors of
+// two, but what decides at a given size is how the blocks fill the GPU: a
+// launch of 1024 blocks where 912 are resident runs most of them at once and
+// then a few alone.  us per iteration of a launch of T blocks of d planes:
+//   base + full waves x (wave + (d + halo) plane[resident])
+//        + (wave + (d + halo) plane[blocks per SM of the last wave]),
+// plane[b] the time of a plane with b blocks on an SM.  The constants are
+// least-squares fits to 23 launches (28 x 24 x 20 to 450 x 390 x 420, 1 to 36
+// right-hand sides) at up to 20 depths each on a GB300; the resident blocks
+// are those of the kernels' registers.  CG alone: its iterates do not depend on
+// the summation order that the depth sets (tau differs by 1e-16 in F64, 1e-10
+// in MIXED, 1e-7 in F32), where BiCGSTAB's iteration count moves by a tenth.
+struct DepthModel {
+    int resident;
+    double base, wave, halo, plane[6];
+};
+constexpr DepthModel kDepthModel[3] = {
+    {2, 9.6, 0.9, 1.8, {2.7, 4.2}},                              // F64
+    {4, 7.9, 5.3, 0.75, {1.16, 1.44, 1.80, 2.18}},               // F32
+    {6, 11.5, 0.0, 4.1, {1.31, 1.54, 1.85, 2.06, 2.37, 2.37}},   // MIXED
+};
+constexpr int kSms = 152;
+
+double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims, int d)
+{
+    int64_t blocks = 0, deepest = 1;
+    for (const int64_t *v : dims) {
+        blocks += make_geometry(v[0], v[1], v[2], d).ntiles;
+        deepest = std::max(deepest, std::min<int64_t>(d, v[2]));
+    }
+    const int64_t cap = (int64_t)kSms * M.resident, full = blocks / cap, rem = blocks % cap;
+    double us = M.base + (double)full * (M.wave + ((double)deepest + M.halo) * M.plane[M.resident - 1]);
+    if (rem) us += M.wave + ((double)deepest + M.halo) * M.plane[(rem + kSms - 1) / kSms - 1];
+    return us;
+}
+
+// The table's depth, or the even split of the tallest volume that the model
+// puts at least 5 % below it.  Against the table on the 23 launches: F64 12 %
+// faster on average (1.29x for 12 volumes of 64^3, 0.998x the worst), MIXED
+// 4.6 % (1.27x for 256^3, none slower), F32 5 % (1.26x for 160^3, 0.994x).
+// Without the margin the means are a little higher and the worst 0.91x: near
+// equal predictions are not worth following.
+//
+// One right-hand side of a MIXED solve is what the serving context runs
+// beside others, at the depth it has alone: there it takes no less than three
+// quarters of the table's depth, since shallow slabs that fill an idle GPU
+// only read more halo planes on a busy one.  (No MIXED launch takes a single
+// plane, so that the directions of a volume of a few blocks keep the depth,
+// and with it the last bits, that each has alone.)
+int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int table)
+{
+    const DepthModel &M = kDepthModel[prec];
+    int64_t nz = 1;
+    for (const int64_t *v : dims) nz = std::max(nz, v[2]);
+    const int64_t least = prec != FAST_PREC_MIXED ? 1 : (dims.size() == 1 ? std::max(2, table * 3 / 4) : 2);
+    double best = 0.95 * modelled_us(M, dims, table);
+    int depth = table;
+    for (int64_t d = std::min<int64_t>(nz, 1024); d >= least;) {
+        const int64_t n = (nz + d - 1) / d;
+        d = (nz + n - 1) / n;  // even slabs
+        if (d < least) break;
+        const double us = modelled_us(M, dims, (int)d);
+        if (us < best) {
+            best = us;
+            depth = (int)d;
+        }
+        d = std::min<int64_t>(d - 1, d * 31 / 32);
+    }
+    return depth;
+}
+
 // The depth of a launch of right-hand sides with dimensions dims.
 int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims)
 {
@@ -502,7 +576,10 @@ int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims)
     if (prec >= 0 && prec < 3 && solver >= 0 && solver < 2) {
         slab_init();
         const int t = g_slab[prec][solver][slab_class(W)].load(std::memory_order_relaxed);
-        if (t > 0) return t;
+        if (t > 0)
+            return solver == FAST_SOLVER_CG && !g_slab_set[prec][solver].load(std::memory_order_relaxed)
+                       ? modelled_depth(prec, dims, t)
+                       : t;
     }
     int zc = kSlabDepth;
     for (; zc > 2; zc /= 2) {
@@ -1008,6 +1085,7 @@ FAST_API int fast_tau_set_slab_table(int32_t precision, int32_t solver, const in
     for (int c = 0; c < nclass; c++)
         if (depth_by_class[c] < 0 || depth_by_class[c] > 1024) return fail(FAST_BAD_ARG, "depth out of range");
     slab_init();
+    g_slab_set[precision][solver].store(depth_by_class != nullptr);
     for (int c = 0; c < kSlabClasses; c++)
         g_slab[precision][solver][c].store(!depth_by_class ? kSlabTable[precision][solver][c]
                                                            : (c < nclass ? depth_by_class[c] : 0));

@@ -243,7 +243,9 @@ FAST_API int fast_tau_last_stats(fast_tau_stats *out);
  * fast_tau_set_slab_table installs the depths of one (precision, solver) for
  * classes 0..nclass-1 (0 = no entry: the full depth, halved while the launch
  * has fewer than 608 blocks); depth_by_class NULL restores the built-in
- * table, which fast_gb300/autotune.py writes from GB300 timings. */
+ * table, which fast_gb300/autotune.py writes from GB300 timings.  With the
+ * built-in table a CG launch may take another depth than its class's, by a
+ * model of how its blocks fill the GPU; an installed table is followed. */
 FAST_API int fast_tau_slab_depth(int64_t nx, int64_t ny, int64_t nz, int32_t nrhs, int32_t precision,
                                  int32_t solver, int32_t *depth, int32_t *size_class /* nullable */);
 FAST_API int fast_tau_set_slab_table(int32_t precision, int32_t solver, const int32_t *depth_by_class,
