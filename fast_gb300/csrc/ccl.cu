@@ -74,6 +74,7 @@ struct Ccl {
     uint32_t *roots;   // [z][y][word]: slots that are local roots
     uint32_t *par;     // the label array: parents at the local roots' places
     uint32_t *cnt, *root_bits;
+    int64_t zero_words;  // cnt and root_bits, from cnt on: zeroed by pass 1
 
     __device__ int64_t word(int y, int z, int w) const { return ((int64_t)z * ny + y) * wx + w; }
     __device__ uint32_t voxel(int x, int y, int z) const
@@ -204,6 +205,8 @@ __global__ void __launch_bounds__(kBrickThreads) ccl_bricks(Ccl A)
     const int y0 = (int)(b / A.wx % A.by) * RY, z0 = (int)(b / A.wx / A.by) * RZ;
     const int x0 = w * 64;
 
+    for (int64_t k = b * kBrickThreads + tid; k < A.zero_words; k += (int64_t)gridDim.x * kBrickThreads) A.cnt[k] = 0u;
+
     // A warp takes consecutive rows; all its loads are in flight together.
     constexpr int PER = ROWS / (kBrickThreads / 32), U = 8;
     const bool in0 = x0 + lane < A.nx, in1 = x0 + 32 + lane < A.nx;
@@ -304,7 +307,7 @@ __device__ __forceinline__ uint32_t local_root(const Ccl &A, int y, int z, int w
 }
 
 // Pass 2: joins across brick faces.  Tasks: every word with a word to its
-// left, every half word of the rows that begin a brick in y, and in z.
+// left, every quarter word of the rows that begin a brick in y, and in z.
 __global__ void __launch_bounds__(256) ccl_merge(Ccl A, int64_t tasks_x, int64_t tasks_y, int64_t tasks_z)
 {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -319,8 +322,8 @@ __global__ void __launch_bounds__(256) ccl_merge(Ccl A, int64_t tasks_x, int64_t
     }
     t -= tasks_x;
     int w, y, z, ty, tz;
-    const int h = (int)(t & 1);
-    t >>= 1;
+    const int piece = (int)(t & 3), h = piece >> 1;
+    t >>= 2;
     if (t < tasks_y) {
         w = (int)(t % A.wx);
         t /= A.wx;
@@ -343,7 +346,8 @@ __global__ void __launch_bounds__(256) ccl_merge(Ccl A, int64_t tasks_x, int64_t
     uint32_t u0 = 0, v0 = 0;
     bool any = false;
     const uint64_t both = run_starts(a & c);
-    for (uint32_t o = (uint32_t)(h ? both >> 32 : both); o; o &= o - 1) {
+    const uint32_t mine = (uint32_t)(h ? both >> 32 : both) & (piece & 1 ? 0xFFFF0000u : 0x0000FFFFu);
+    for (uint32_t o = mine; o; o &= o - 1) {
         const int bit = __ffs((int)o) - 1;
         const uint32_t u = local_root(A, y, z, w, run_start(sa, h, bit));
         const uint32_t v = local_root(A, ty, tz, w, run_start(sc, h, bit));
@@ -573,7 +577,7 @@ int check_dims(int64_t nx, int64_t ny, int64_t nz)
 // Geometry and scratch plan of a labelling; `base` null: sizes only.
 // Returns the scratch bytes: 8 + 2 x slots + 4 per 64-voxel word, one bit per
 // voxel and one count per chunk (1.2 bytes per voxel of a wide volume).
-size_t plan(Ccl &A, char *base, size_t &zero_off, size_t &zero_bytes)
+size_t plan(Ccl &A, char *base)
 {
     const size_t words = (size_t)A.wx * A.ny * A.nz;
     const size_t n = (size_t)A.nx * A.ny * A.nz;
@@ -587,26 +591,24 @@ size_t plan(Ccl &A, char *base, size_t &zero_off, size_t &zero_bytes)
     A.bits = (uint64_t *)take(words * 8);
     A.local = (uint16_t *)take(words * A.slots * 2);
     A.roots = (uint32_t *)take(words * 4);
-    zero_off = off;
+    const size_t zero_off = off;
     A.cnt = (uint32_t *)take((nchunks + 1) * 4);
     A.root_bits = (uint32_t *)take(nchunks * (kChunk / 32) * 4);
-    zero_bytes = off - zero_off;
+    A.zero_words = (int64_t)((off - zero_off) / 4);
     return off;
 }
 
 // Labels of A.mask into A.par (device, N uint32) on `st`; scratch planned.
-int label_device(const Ccl &A, char *scratch, size_t zero_off, size_t zero_bytes, uint32_t *num_labels,
-                 cudaStream_t st)
+int label_device(const Ccl &A, uint32_t *num_labels, cudaStream_t st)
 {
     const size_t n = (size_t)A.nx * A.ny * A.nz;
     const uint32_t nchunks = (uint32_t)((n + kChunk - 1) / kChunk);
     const int64_t words = (int64_t)A.wx * A.ny * A.nz;
     const int64_t bricks = (int64_t)A.wx * A.by * A.bz;
-    CK(cudaMemsetAsync(scratch + zero_off, 0, zero_bytes, st));
     ccl_bricks<<<(unsigned)bricks, kBrickThreads, 0, st>>>(A);
     const int64_t tx = (int64_t)(A.wx - 1) * A.ny * A.nz, ty = (int64_t)A.wx * (A.by - 1) * A.nz,
                   tz = (int64_t)A.wx * A.ny * (A.bz - 1);
-    const int64_t tasks = tx + 2 * (ty + tz);
+    const int64_t tasks = tx + 4 * (ty + tz);
     if (tasks > 0) ccl_merge<<<(unsigned)((tasks + 255) / 256), 256, 0, st>>>(A, tx, ty, tz);
     ccl_flatten<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(A, words);
     ccl_scan_chunks<<<1, 1024, 0, st>>>(A.cnt, nchunks);
@@ -659,13 +661,12 @@ int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint
     A.bg = bg;
     A.mask = d_mask;
     A.par = d_labels;
-    size_t zero_off = 0, zero_bytes = 0;
-    const size_t need = plan(A, nullptr, zero_off, zero_bytes);
+    const size_t need = plan(A, nullptr);
     char *scratch = nullptr;
     cudaError_t e = cudaMallocAsync((void **)&scratch, need, st);
     if (e != cudaSuccess) return ft_fail(FAST_NOMEM, "labelling scratch: %s", cudaGetErrorString(e));
-    plan(A, scratch, zero_off, zero_bytes);
-    int s = label_device(A, scratch, zero_off, zero_bytes, num_labels, st);
+    plan(A, scratch);
+    int s = label_device(A, num_labels, st);
     cudaFreeAsync(scratch, st);
     if (s == FAST_OK && boundary) {
         if (boundary_cap < (uint64_t)7 * *num_labels)
