@@ -57,6 +57,13 @@ cudaError_t configure_misc()
     return cudaSuccess;
 }
 
+void launch_count_zero(const uint8_t *mask, uint64_t n, unsigned long long *total, cudaStream_t st)
+{
+    const uint64_t want = (n / 16 + 255) / 256, most = 152 * 8;  // one wave of full blocks
+    const unsigned grid = (unsigned)(want < 1 ? 1 : (want < most ? want : most));
+    count_zero_kernel<<<grid, 256, 0, st>>>(mask, n, total);
+}
+
 void launch_init64(const Launch &L, cudaStream_t st) { init64_kernel<<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); }
 
 void launch_bnd(bool f32, const Job *jobs, const int (&job)[3], int count, cudaStream_t st)

@@ -1240,38 +1240,25 @@ FAST_API int fast_porosity(const uint8_t *mask, int64_t nx, int64_t ny, int64_t 
     Engine *E = nullptr;
     int st = get_engine(&E);
     if (st != FAST_OK) return st;
-    const Geometry G = make_geometry(nx, ny, nz);
-    const size_t N = (size_t)G.N;
-    const int64_t P = row_pitch(nx);
-    const size_t NP = (size_t)(P * ny * nz);
+    const size_t N = (size_t)(nx * ny * nz);
     cudaStream_t s = E->stream;
     Arena A;
-    const size_t need = align_up(N, 256) + align_up(NP, 256) + align_up((size_t)G.ntiles * NPART * 8, 256) +
-                        align_up(sizeof(Scalars), 256) + align_up(sizeof(uint32_t), 256) + align_up(sizeof(Job), 256);
-    CU(cudaMallocAsync((void **)&A.base, need, s));
+    CU(cudaMallocAsync((void **)&A.base, align_up(N, 256) + 256, s));
     uint8_t *d_mask = (uint8_t *)A.take(N);
-    uint8_t *d_code = (uint8_t *)A.take(NP);
-    double *d_part = (double *)A.take((size_t)G.ntiles * NPART * 8);
-    Scalars *d_sc = (Scalars *)A.take(sizeof(Scalars));
-    uint32_t *d_cnt = (uint32_t *)A.take(sizeof(uint32_t));
-    Job *d_job = (Job *)A.take(sizeof(Job));
-    Job &J = E->h_jobs[0];
-    memset(&J, 0, sizeof(Job));
-    J.nx = (int32_t)nx; J.ny = (int32_t)ny; J.nz = (int32_t)nz;
-    J.pitch = (int32_t)P;
-    J.tiles_x = G.tx; J.tiles_y = G.ty; J.tiles_z = G.tz; J.zc = G.zc;
-    J.ntiles = G.ntiles;
-    J.code = d_code; J.mask = d_mask; J.part = d_part; J.sc = d_sc; J.counter = d_cnt;
-    CU(cudaMemcpyAsync(d_mask, mask, N, cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(d_job, &J, sizeof(Job), cudaMemcpyHostToDevice, s));
-    CU(cudaMemsetAsync(d_sc, 0, sizeof(Scalars), s));
-    CU(cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t), s));
-    Launch L{d_job, 1, 0, G.ntiles, nullptr};
-    launch_code(L, s);
-    CU(cudaMemcpyAsync(E->h_sc, d_sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
+    unsigned long long *d_total = (unsigned long long *)A.take(sizeof(unsigned long long));
+    unsigned long long *h_total = (unsigned long long *)E->h_sc;
+    cudaError_t e = cudaMemcpyAsync(d_mask, mask, N, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_total, 0, sizeof(*d_total), s);
+    if (e == cudaSuccess) {
+        launch_count_zero(d_mask, N, d_total, s);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_total, d_total, sizeof(*d_total), cudaMemcpyDeviceToHost, s);
     cudaFreeAsync(A.base, s);
-    CU(cudaStreamSynchronize(s));
-    const uint64_t pores = E->h_sc[0].pores;
+    const cudaError_t e2 = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = e2;
+    if (e != cudaSuccess) return fail(FAST_CUDA_ERROR, "pore count: %s", cudaGetErrorString(e));
+    const uint64_t pores = *h_total;
     if (pore_count) *pore_count = pores;
     if (porosity) *porosity = (double)pores / (double)N;
     return FAST_OK;

@@ -22,6 +22,8 @@ void launch_mixed_inner(Step s, const Launch &L, cudaStream_t st);
 // asked for one): FP64 iterate, or float-float with `ff`.
 void launch_replace(bool bicg, bool ff, const Launch &L, cudaStream_t st);
 void launch_init64(const Launch &L, cudaStream_t st);
+// Adds the zero bytes of mask[0..n) (16-byte aligned) to *total.
+void launch_count_zero(const uint8_t *mask, uint64_t n, unsigned long long *total, cudaStream_t st);
 void launch_code(const Launch &L, cudaStream_t st);
 // Fills the domain-face tables (Job::bnd) of the first `count` of jobs[job[0..2]]
 // (device table): one job per primary axis.
