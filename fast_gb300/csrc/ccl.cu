@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ccl_faces.h"
 #include "fasttau.h"
 #include "tau_errors.h"
 
@@ -523,29 +524,54 @@ __global__ void __launch_bounds__(kBrickThreads) ccl_relabel(Ccl A)
     }
 }
 
-// Pass 7: the six face bitmaps.  Face d (Dir order) of the volume, flattened
-// over the two secondary axes; faces are concatenated in d order.
-__global__ void ccl_faces(const uint32_t *labels, int nx, int ny, int nz, uint32_t num_labels, uint8_t *bnd)
+// A voxel of the six faces, its face (Dir order) and linear index.  Face d is
+// flattened over the two secondary axes; faces are concatenated in d order.
+__device__ __forceinline__ uint32_t face_voxel(int64_t t, int nx, int ny, int nz, int &d)
 {
     const int64_t fxy = (int64_t)nx * ny, fxz = (int64_t)nx * nz, fyz = (int64_t)ny * nz;
     const int64_t sizes[3] = {fyz, fxz, fxy};  // face area by primary axis
-    const int64_t total = 2 * (fyz + fxz + fxy);
+    d = 0;
+    while (t >= sizes[d >> 1]) {
+        t -= sizes[d >> 1];
+        d++;
+    }
+    const bool pos = (d & 1) == 0;  // X_POS, Y_POS, Z_POS: the last plane
+    int x, y, z;
+    if (d < 2) { x = pos ? nx - 1 : 0; y = (int)(t % ny); z = (int)(t / ny); }
+    else if (d < 4) { y = pos ? ny - 1 : 0; x = (int)(t % nx); z = (int)(t / nx); }
+    else { z = pos ? nz - 1 : 0; x = (int)(t % nx); y = (int)(t / nx); }
+    return (uint32_t)x + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
+}
+
+// Pass 7: the six face bitmaps.
+__global__ void ccl_faces(const uint32_t *labels, int nx, int ny, int nz, uint32_t num_labels, uint8_t *bnd)
+{
+    const int64_t total = 2 * ((int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny);
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (int64_t)gridDim.x * blockDim.x) {
-        int d = 0;
-        int64_t u = t;
-        while (u >= sizes[d >> 1]) {
-            u -= sizes[d >> 1];
-            d++;
-        }
-        const int k = d >> 1;
-        const bool pos = (d & 1) == 0;  // X_POS, Y_POS, Z_POS: the last plane
-        int x, y, z;
-        if (k == 0) { x = pos ? nx - 1 : 0; y = (int)(u % ny); z = (int)(u / ny); }
-        else if (k == 1) { y = pos ? ny - 1 : 0; x = (int)(u % nx); z = (int)(u / nx); }
-        else { z = pos ? nz - 1 : 0; x = (int)(u % nx); y = (int)(u / nx); }
-        const uint32_t l = labels[(uint32_t)x + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z)];
+        int d;
+        const uint32_t l = labels[face_voxel(t, nx, ny, nz, d)];
         if (l > 0) bnd[(size_t)d * num_labels + l] = 1;
+    }
+}
+
+// The faces each label touches as one byte per label, bit d = face d (label
+// 0 touches none): what the area pass reads, made where it is read instead of
+// through the face bitmaps and the host.
+__global__ void ccl_face_bits(const uint32_t *__restrict__ labels, int nx, int ny, int nz, uint32_t *bits)
+{
+    const int64_t total = 2 * ((int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < total; t0 += stride) {
+        int d = 0;
+        const uint32_t l = t0 + lane < total ? labels[face_voxel(t0 + lane, nx, ny, nz, d)] : 0u;
+        // One lane per label and face: one component can own most of a face.
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, (unsigned long long)l << 3 | (unsigned)d);
+        if (l == 0 || lane != __ffs((int)same) - 1) continue;
+        const uint32_t bit = 1u << (8 * (l & 3u) + d);
+        // a stale read only repeats the atomic
+        if (!(*(volatile uint32_t *)(bits + (l >> 2)) & bit)) atomicOr(bits + (l >> 2), bit);
     }
 }
 
@@ -682,6 +708,13 @@ int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint
 }  // namespace ft
 
 using namespace ft;
+
+cudaError_t ft_label_faces(const uint32_t *d_labels, int64_t nx, int64_t ny, int64_t nz, uint32_t *d_bits,
+                           cudaStream_t st)
+{
+    ccl_face_bits<<<1024, 256, 0, st>>>(d_labels, (int)nx, (int)ny, (int)nz, d_bits);
+    return cudaGetLastError();
+}
 
 extern "C" {
 
