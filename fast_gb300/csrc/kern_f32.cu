@@ -1,7 +1,7 @@
 // FP32 solver kernels: the reference's `-p float` (float scalars) and the
 // inner iterations of the MIXED solve (double scalars).
 #include "tau_launch.h"
-#include "tau_pointwise.cuh"
+#include "tau_resident.cuh"
 
 namespace ft {
 
@@ -162,10 +162,19 @@ cudaError_t configure_f32()
     cudaError_t f = cudaFuncSetAttribute(sweep_kernel_mb<OpCGF, kStagesCGF, kBlocksCGF>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          sweep_dyn_smem<OpCGF, kStagesCGF>());
+    const cudaError_t g = configure_resident<float>();
     if (a != cudaSuccess) return a;
+    if (g != cudaSuccess) return g;
     if (b != cudaSuccess) return b;
     if (f != cudaSuccess) return f;
     return c != cudaSuccess ? c : d;
+}
+
+int resident_per_sm(bool f32, int zc) { return f32 ? resident_fit<float>(zc) : resident_fit<double>(zc); }
+
+cudaError_t launch_resident_f32(const Launch &L, int zc, int iters, cudaStream_t st)
+{
+    return launch_resident<float>(L, zc, iters, st);
 }
 
 void launch_pure_f32(Step s, const Launch &L, cudaStream_t st) { dispatch<float>(s, L, st); }

@@ -1,6 +1,6 @@
 // Pure FP64 solver kernels (the reference's `-p double`).
 #include "tau_launch.h"
-#include "tau_pointwise.cuh"
+#include "tau_resident.cuh"
 
 namespace ft {
 
@@ -46,6 +46,11 @@ void launch_pure_f64(Step s, const Launch &L, cudaStream_t st)
     }
 }
 
+cudaError_t launch_resident_f64(const Launch &L, int zc, int iters, cudaStream_t st)
+{
+    return launch_resident<double>(L, zc, iters, st);
+}
+
 cudaError_t configure_f64()
 {
     using T = double;
@@ -57,6 +62,7 @@ cudaError_t configure_f64()
     if ((r = cfg<OpBiRestart<T, T>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpBi1<T, T>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpBi2<T, T>>()) != cudaSuccess) e = r;
+    if ((r = configure_resident<T>()) != cudaSuccess) e = r;
     return e;
 }
 

@@ -408,6 +408,51 @@ int iterate(Engine &E, const Launch &L, int njobs, Scalars *d_sc, const std::vec
     return status;
 }
 
+// CG by resident launches (tau_resident.cuh) until every job has left RUNNING,
+// polled one launch behind like iterate.  A launch ends early once its jobs
+// are done, so a long one costs nothing at the end of a solve.  launched =
+// false: the first launch was refused and nothing ran.
+int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, uint32_t *d_cnt, bool f32, int zc,
+                     uint64_t max_iter, bool &launched)
+{
+    constexpr int kIters = 128;
+    cudaStream_t st = E.stream;
+    cudaError_t cerr = cudaSuccess;
+    cudaEvent_t ev[2];
+    cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
+    const uint64_t max_launches = max_iter / kIters + 4;
+    int status = FAST_OK;
+    for (uint64_t k = 0; k < max_launches; k++) {
+        cerr = cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * njobs, st);
+        if (cerr == cudaSuccess) cerr = (f32 ? launch_resident_f32 : launch_resident_f64)(L, zc, kIters, st);
+        if (cerr != cudaSuccess && k == 0) {
+            cudaGetLastError();
+            launched = false;
+            break;
+        }
+        if (cerr != cudaSuccess) { status = fail(FAST_CUDA_ERROR, "resident launch: %s", cudaGetErrorString(cerr)); break; }
+        t_prof.st.launches += 1;
+        t_prof.st.kernel_launches[FAST_K_CG1] += 1;
+        cudaMemcpyAsync(E.h_sc + (k & 1) * Engine::kMaxJobs, d_sc, sizeof(Scalars) * njobs, cudaMemcpyDeviceToHost, st);
+        cudaEventRecord(ev[k & 1], st);
+        if (k == 0) continue;
+        cerr = cudaEventSynchronize(ev[(k - 1) & 1]);
+        if (cerr != cudaSuccess) { status = fail(FAST_CUDA_ERROR, "solver step: %s", cudaGetErrorString(cerr)); break; }
+        const Scalars *prev = E.h_sc + ((k - 1) & 1) * Engine::kMaxJobs;
+        bool running = false;
+        for (int j = 0; j < njobs; j++) running |= (prev[j].state == RUNNING);
+        if (!running) break;
+    }
+    // the next kernels count their blocks from zero again
+    if (status == FAST_OK) cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * njobs, st);
+    cerr = cudaStreamSynchronize(st);
+    if (cerr != cudaSuccess && status == FAST_OK) status = fail(FAST_CUDA_ERROR, "solver: %s", cudaGetErrorString(cerr));
+    cudaEventDestroy(ev[0]);
+    cudaEventDestroy(ev[1]);
+    return status;
+}
+
 void dispatch_f64(Step s, const Launch &L, cudaStream_t st) { launch_pure_f64(s, L, st); }
 void dispatch_f32(Step s, const Launch &L, cudaStream_t st) { launch_pure_f32(s, L, st); }
 std::vector<Step> mixed_steps(int solver, bool ff)
@@ -468,7 +513,7 @@ size_t code_bytes(int64_t nx, int64_t ny, int64_t nz) { return align_up((size_t)
 // FAST_TAU_ZC overrides all of it.
 // slab_depth sizes a volume solved alone (one right-hand side, the serving
 // context's unit, so a served result equals the same request solved alone);
-// launch_slab_depth a whole launch.
+// tuned_depth a whole launch.
 #include "slab_table.inc"
 
 namespace {
@@ -563,9 +608,53 @@ int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int table
     return depth;
 }
 
-// The depth of a launch of right-hand sides with dimensions dims.
-int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims)
+// CG in one kernel (tau_resident.cuh): the depth for right-hand sides with
+// dimensions dims, 0 where their blocks do not all fit on the GPU or the model
+// puts the sweeps within 5 %.  us per iteration with b blocks on the fullest
+// SM: base[b] + d plane[b], fits to 18 launches (28 x 24 x 20 to 100^3, 1 to 12
+// right-hand sides) at all their depths.  Steps -> best resident depth: F64 CG
+// 20.3 -> 13.9 us at 40^3, 25.3 -> 18.2 at 64^3, 42.4 -> 35.3 at 80^3, 30.2 ->
+// 22.3 for three times 48^3; F32 12.2 -> 9.0 at 28 x 24 x 20, 15.8 -> 12.1 at
+// 64^3, 24.1 -> 22.6 at 100^3, 29.3 -> 23.6 for 12 times 48^3.
+struct ResidentModel {
+    double base[2], plane[2];
+};
+constexpr ResidentModel kResidentModel[2] = {
+    {{9.6, 11.5}, {2.13, 4.1}},  // F64
+    {{8.4, 10.4}, {0.91, 1.15}},  // F32
+};
+
+int resident_depth(int prec, const std::vector<const int64_t *> &dims, int table)
 {
+    if (prec == FAST_PREC_MIXED) return 0;
+    const bool f32 = prec == FAST_PREC_F32;
+    const ResidentModel &M = kResidentModel[f32];
+    int64_t nz = 1;
+    for (const int64_t *v : dims) nz = std::max(nz, v[2]);
+    int64_t depth = 0;
+    double best = 0.95 * modelled_us(kDepthModel[prec], dims, modelled_depth(prec, dims, table));
+    for (int64_t d = std::min<int64_t>(nz, kResidentDepth); d >= 1; d--) {
+        const int64_t n = (nz + d - 1) / d;
+        d = (nz + n - 1) / n;  // even slabs
+        int64_t blocks = 0;
+        for (const int64_t *v : dims) blocks += make_geometry(v[0], v[1], v[2], (int)d).ntiles;
+        if (blocks > (int64_t)kSms * 2) break;
+        const int b = blocks > kSms;
+        if (resident_per_sm(f32, (int)d) < b + 1) continue;
+        const double us = M.base[b] + (double)d * M.plane[b];
+        if (us < best) {
+            best = us;
+            depth = d;
+        }
+    }
+    return (int)depth;
+}
+
+// The depth of a launch of right-hand sides with dimensions dims; resident =
+// it is that of a solve in one kernel.
+int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims, bool *resident = nullptr)
+{
+    if (resident) *resident = false;
     const int env = env_int("FAST_TAU_ZC", 0);
     if (env > 0) return env;
     int64_t W = 0;
@@ -576,10 +665,12 @@ int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims)
     if (prec >= 0 && prec < 3 && solver >= 0 && solver < 2) {
         slab_init();
         const int t = g_slab[prec][solver][slab_class(W)].load(std::memory_order_relaxed);
-        if (t > 0)
-            return solver == FAST_SOLVER_CG && !g_slab_set[prec][solver].load(std::memory_order_relaxed)
-                       ? modelled_depth(prec, dims, t)
-                       : t;
+        if (t > 0) {
+            if (solver != FAST_SOLVER_CG || g_slab_set[prec][solver].load(std::memory_order_relaxed)) return t;
+            const int r = resident_depth(prec, dims, t);
+            if (resident) *resident = r > 0;
+            return r > 0 ? r : modelled_depth(prec, dims, t);
+        }
     }
     int zc = kSlabDepth;
     for (; zc > 2; zc /= 2) {
@@ -597,17 +688,19 @@ int slab_depth(int64_t nx, int64_t ny, int64_t nz, int prec, int solver)
     return tuned_depth(prec, solver, {d});
 }
 
-int launch_slab_depth(const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs, int prec, int solver)
+// The dimensions of every right-hand side (pointers into flat).
+std::vector<const int64_t *> job_dims(const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs,
+                                      std::vector<int64_t> &flat)
 {
     std::vector<const int64_t *> dims;
-    std::vector<int64_t> flat(3 * vols.size());
+    flat.resize(3 * vols.size());
     for (size_t v = 0; v < vols.size(); v++) {
         flat[3 * v] = vols[v].nx;
         flat[3 * v + 1] = vols[v].ny;
         flat[3 * v + 2] = vols[v].nz;
     }
     for (const JobSpec &j : jobs) dims.push_back(&flat[3 * j.vol]);
-    return tuned_depth(prec, solver, dims);
+    return dims;
 }
 
 // The one-sweep MIXED CG (OpCGF) is opt-in (FAST_TAU_CG_FUSED=1): its
@@ -774,7 +867,13 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     const size_t vec_t = (prec == FAST_PREC_F64) ? 8 : 4;
 
     // --- memory plan (the reference's fit check, VolumeMeasures.cpp:104-125)
-    const int zc = launch_slab_depth(vols, jobs, prec, solver);
+    std::vector<int64_t> flat;
+    const std::vector<const int64_t *> dims = job_dims(vols, jobs, flat);
+    // Small CG solves run in one kernel (profiles and traces look at single
+    // steps).
+    bool resident = false;
+    const int zc = tuned_depth(prec, solver, dims, &resident);
+    resident = resident && !t_prof.on && env_int("FAST_TAU_TRACE", 0) < 2;
     size_t need = solve_bytes(vols, jobs, prec, solver, zc, false);
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
@@ -805,7 +904,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     // fits beside everything else; a volume that fills the GPU evaluates the
     // product twice instead (the same results).
     Arena A;
-    bool store_q = !mixed && solver == FAST_SOLVER_CG;
+    bool store_q = !mixed && solver == FAST_SOLVER_CG && !resident;
     if (store_q) {
         const size_t more = solve_bytes(vols, jobs, prec, solver, zc, true);
         store_q = more <= avail && cudaMallocAsync((void **)&A.base, more, st) == cudaSuccess;
@@ -888,7 +987,9 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
         std::vector<Step> steps;
         if (solver == FAST_SOLVER_CG) steps = {Step::CG1, store_q ? Step::CG2_Q : Step::CG2};
         else steps = {Step::BI_RESTART, Step::BI1, Step::BI2, Step::BI3};
-        status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
+        // (A context whose SMs are limited can refuse the cooperative launch.)
+        if (resident) status = iterate_resident(E, L, nj, d_sc, d_cnt, prec == FAST_PREC_F32, zc, P.max_iter, resident);
+        if (!resident) status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
     } else {
         // FP32 iterations with in-graph FP64 residual replacement: the
         // replacement slot leads every iteration and is a no-op launch unless
