@@ -412,7 +412,7 @@ int iterate(Engine &E, const Launch &L, int njobs, Scalars *d_sc, const std::vec
 // polled one launch behind like iterate.  A launch ends early once its jobs
 // are done, so a long one costs nothing at the end of a solve.  launched =
 // false: the first launch was refused and nothing ran.
-int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, uint32_t *d_cnt, bool f32, int zc,
+int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, bool f32, int zc,
                      uint64_t max_iter, bool &launched)
 {
     constexpr int kIters = 128;
@@ -424,8 +424,7 @@ int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, uint3
     const uint64_t max_launches = max_iter / kIters + 4;
     int status = FAST_OK;
     for (uint64_t k = 0; k < max_launches; k++) {
-        cerr = cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * njobs, st);
-        if (cerr == cudaSuccess) cerr = (f32 ? launch_resident_f32 : launch_resident_f64)(L, zc, kIters, st);
+        cerr = (f32 ? launch_resident_f32 : launch_resident_f64)(L, zc, kIters, st);
         if (cerr != cudaSuccess && k == 0) {
             cudaGetLastError();
             launched = false;
@@ -444,8 +443,6 @@ int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, uint3
         for (int j = 0; j < njobs; j++) running |= (prev[j].state == RUNNING);
         if (!running) break;
     }
-    // the next kernels count their blocks from zero again
-    if (status == FAST_OK) cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * njobs, st);
     cerr = cudaStreamSynchronize(st);
     if (cerr != cudaSuccess && status == FAST_OK) status = fail(FAST_CUDA_ERROR, "solver: %s", cudaGetErrorString(cerr));
     cudaEventDestroy(ev[0]);
@@ -613,9 +610,9 @@ int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int table
 // puts the sweeps within 5 %.  us per iteration with b blocks on the fullest
 // SM: base[b] + d plane[b], fits to 18 launches (28 x 24 x 20 to 100^3, 1 to 12
 // right-hand sides) at all their depths.  Steps -> best resident depth: F64 CG
-// 20.3 -> 13.9 us at 40^3, 25.3 -> 18.2 at 64^3, 42.4 -> 35.3 at 80^3, 30.2 ->
-// 22.3 for three times 48^3; F32 12.2 -> 9.0 at 28 x 24 x 20, 15.8 -> 12.1 at
-// 64^3, 24.1 -> 22.6 at 100^3, 29.3 -> 23.6 for 12 times 48^3.
+// 20.3 -> 13.6 us at 40^3, 25.3 -> 18.0 at 64^3, 42.4 -> 34.9 at 80^3, 30.2 ->
+// 22 for three times 48^3; F32 12.2 -> 8.3 at 28 x 24 x 20, 15.8 -> 11.2 at
+// 64^3, 24.1 -> 22 at 100^3, 22.2 -> 14.2 for 12 times 32^3.
 struct ResidentModel {
     double base[2], plane[2];
 };
@@ -638,7 +635,7 @@ int resident_depth(int prec, const std::vector<const int64_t *> &dims, int table
         d = (nz + n - 1) / n;  // even slabs
         int64_t blocks = 0;
         for (const int64_t *v : dims) blocks += make_geometry(v[0], v[1], v[2], (int)d).ntiles;
-        if (blocks > (int64_t)kSms * 2) break;
+        if (blocks > kResidentBlocks) break;
         const int b = blocks > kSms;
         if (resident_per_sm(f32, (int)d) < b + 1) continue;
         const double us = M.base[b] + (double)d * M.plane[b];
@@ -875,6 +872,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     const int zc = tuned_depth(prec, solver, dims, &resident);
     resident = resident && !t_prof.on && env_int("FAST_TAU_TRACE", 0) < 2;
     size_t need = solve_bytes(vols, jobs, prec, solver, zc, false);
+    if (resident) need += align_up(kResidentBlocks * kResidentSlotBytes, 256);
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
 #if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
@@ -919,6 +917,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     uint32_t *d_gate = (uint32_t *)A.take(sizeof(uint32_t));  // MIXED replacement gate
     void *d_bnd[3];
     for (void *&b : d_bnd) b = A.take(bnd_bytes(prec));
+    char *d_slots = resident ? (char *)A.take(kResidentBlocks * kResidentSlotBytes) : nullptr;
     int axis_job[3] = {0, 0, 0}, naxes = 0;  // a job of each primary axis in use
     bool axis_seen[3] = {false, false, false};
     std::vector<uint8_t *> d_code(nv);
@@ -948,6 +947,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
             axis_job[naxes++] = j;
         }
         if (store_q) hj[j].q = A.take(q_bytes(V.nx, V.ny, V.nz, prec));
+        if (resident) hj[j].slots = d_slots + tile_base * kResidentSlotBytes;
         hj[j].tile_base = tile_base;
         tile_base += hj[j].ntiles;
     }
@@ -968,6 +968,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     CU(cudaMemcpyAsync(d_jobs, hj, sizeof(Job) * (nj + nv), cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync(d_sc, hs, sizeof(Scalars) * nj, cudaMemcpyHostToDevice, st));
     CU(cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * nj, st));
+    if (resident) CU(cudaMemsetAsync(d_slots, 0, kResidentBlocks * kResidentSlotBytes, st));
     // every MIXED right-hand side starts with a pending replacement (x = x0):
     // the gate word reads 1
     CU(cudaMemsetAsync(d_gate, 0, sizeof(uint32_t), st));
@@ -988,7 +989,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
         if (solver == FAST_SOLVER_CG) steps = {Step::CG1, store_q ? Step::CG2_Q : Step::CG2};
         else steps = {Step::BI_RESTART, Step::BI1, Step::BI2, Step::BI3};
         // (A context whose SMs are limited can refuse the cooperative launch.)
-        if (resident) status = iterate_resident(E, L, nj, d_sc, d_cnt, prec == FAST_PREC_F32, zc, P.max_iter, resident);
+        if (resident) status = iterate_resident(E, L, nj, d_sc, prec == FAST_PREC_F32, zc, P.max_iter, resident);
         if (!resident) status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
     } else {
         // FP32 iterations with in-graph FP64 residual replacement: the

@@ -16,11 +16,12 @@ enum class Step {
 void launch_pure_f64(Step s, const Launch &L, cudaStream_t st);
 void launch_pure_f32(Step s, const Launch &L, cudaStream_t st);
 // CG of volumes whose blocks of zc planes all fit on the GPU at once: `iters`
-// iterations in one cooperative launch (tau_resident.cuh).  The jobs' counters
-// are zero at its start and are not reset.
+// iterations in one cooperative launch (tau_resident.cuh).
 // A right-hand side's planes per block at most, and the blocks of zc planes
 // that an SM holds (at most two, by their registers).
 constexpr int kResidentDepth = 24;
+constexpr int kResidentBlocks = 2 * 152;
+constexpr size_t kResidentSlotBytes = 48;  // of a block, in Job::slots, zero before the first launch
 int resident_per_sm(bool f32, int zc);
 cudaError_t launch_resident_f64(const Launch &L, int zc, int iters, cudaStream_t st);
 cudaError_t launch_resident_f32(const Launch &L, int zc, int iters, cudaStream_t st);

@@ -1,27 +1,28 @@
 // CG of small F64 and F32 volumes in one kernel: every tile of the launch is a
 // block of a cooperative launch that keeps its part of p, r and q in shared
-// memory and iterates, with a barrier over a right-hand side's blocks where
-// the sweeps have a kernel boundary.
+// memory and iterates; a right-hand side's blocks wait for one another's
+// partial sums where the sweeps have a kernel boundary.
 //
 // What bounds small volumes is not their voxels: of the 8 us of a sweep of a
 // 28 x 24 x 20 volume, two are the tile's planes, the rest the launch, the
 // block's start (its job, tables, scalars, tensor maps) and the finisher's
 // chain (count the block in, fetch the partial sums, update the scalars).
 // Here the start is paid once per launch, every block sums all partial sums
-// and updates its own copy of the scalars, and between two barriers a block
+// and updates its own copy of the scalars, and between two exchanges a block
 // reads from global memory only the residual around its tile.  In F64 the
 // pointwise updates and the stencil then run at the FP64 pipe's rate.
 //
-// Arithmetic, tiles and summation order are those of OpCG1 and PwCG2.  Every
+// Arithmetic, tiles and summation order are those of OpCG1 and PwCG2: a solve
+// has the same bits either way (the serving context runs the sweeps).  Every
 // spin is bounded (2 s); a block that gives up marks its right-hand side FAULT
 // and leaves.
 //
 // us per iteration of the two sweeps (replayed from a graph) -> here: F64 20.3
-// -> 13.9 at 40^3, 25.3 -> 18.2 at 64^3, 30.2 -> 22.3 for three times 48^3; F32
-// 16.8 -> 10.4 at 48^3, 22.2 -> 15.7 for twelve times 32^3.  At 64^3 (128 blocks
-// of four planes) 8.4 of the 18.2 are the FP64 pipe's (2.1 us a plane), the
-// rest the two barriers with their sums and the residual around the tile.
-// Two blocks on an SM hold six planes each in F64 and thirteen in F32, one
+// -> 13.6 at 40^3, 25.3 -> 18.0 at 64^3, 42.4 -> 34.9 at 80^3; F32 15.8 -> 11.2 at
+// 64^3, 22.2 -> 14.2 for twelve times 32^3.  At 64^3 (128 blocks of four
+// planes) 8.4 of the 18.0 are the FP64 pipe's (2.1 us a plane), the rest
+// the two exchanges and the residual around the tile.
+// Two blocks on an SM hold six planes each in F64 and twelve in F32, one
 // alone about twice that: larger volumes stay with the sweeps.
 #pragma once
 #include <cstddef>
@@ -40,27 +41,79 @@ __host__ __device__ constexpr size_t resident_smem(int zc)
     return (size_t)(zc + 2) * HY * PW * sizeof(T) + 2 * (size_t)zc * TX * TY * sizeof(T) + (size_t)(zc + 2) * HY * kBoxW + 16;
 }
 
-// Arrives at the right-hand side's barrier and waits for its `target`th
-// arrival.  The counter starts at zero in every launch and is not reset.
-__device__ __forceinline__ bool job_barrier(uint32_t *counter, uint32_t target, int *s_ok)
+// A tile's partial sums of a step, each with the iteration it belongs to: 16
+// bytes read and written as one, so the sums need no barrier beside them (with
+// a counter to wait on and the sums read after it: 13.9 against 13.6 us per
+// iteration at 40^3 in F64, 11.8 against 11.2 at 64^3 and 15.0 against 14.2 for
+// twelve times 32^3 in F32).  A block has read all of an iteration's step 1 when it writes its step 2, and
+// the reverse, so a slot is never overwritten unread.
+constexpr int kSlots = 3;  // p.q; |r|^2, r.z
+static_assert(kSlots * sizeof(ulonglong2) == kResidentSlotBytes);
+
+__device__ __forceinline__ void slot_write(ulonglong2 *s, double v, uint64_t epoch)
 {
-    __syncthreads();  // the block's writes precede its arrival
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-        const uint64_t t0 = global_timer_ns();
-        uint32_t seen;
-        *s_ok = 1;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-            if (seen >= target) break;
-            if (global_timer_ns() - t0 > kWaitLimitNs) {
-                *s_ok = 0;
-                break;
-            }
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.release.gpu.global.b128 [%0], t; }" ::"l"(s),
+                 "l"(__double_as_longlong(v)), "l"(epoch)
+                 : "memory");
+}
+
+// The value of a slot once it has the epoch; false after kWaitLimitNs.
+__device__ __forceinline__ bool slot_read(const ulonglong2 *s, uint64_t epoch, double &v)
+{
+    uint64_t t0 = 0;
+    for (int n = 0;; n++) {
+        uint64_t bits, e;
+        asm volatile("{ .reg .b128 t; ld.acquire.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                     : "=l"(bits), "=l"(e)
+                     : "l"(s)
+                     : "memory");
+        v = __longlong_as_double((long long)bits);
+        if (e == epoch) return true;
+        if ((n & 63) == 63) {
+            const uint64_t now = global_timer_ns();
+            if (!t0) t0 = now;
+            else if (now - t0 > kWaitLimitNs) return false;
         }
     }
+}
+
+// Publishes the block's partial sums v of `epoch` and waits for those of all
+// of the right-hand side's blocks: their totals, in sum_partials' order.  What
+// the blocks wrote before is visible then.
+template <int NV, typename V>
+__device__ __forceinline__ bool exchange(const V (&v)[NV], ulonglong2 *slots, int64_t local, int64_t ntiles,
+                                         uint64_t epoch, double (&tot)[NV], double *s_red, double *s_val, int *s_ok)
+{
+    __shared__ double s_tot[NV];
+    const int tid = threadIdx.x;
+    block_sum_store<NV, V>(v, s_tot, s_red);
+    if (tid < NV) slot_write(slots + local * kSlots + tid, s_tot[tid], epoch);
+    for (int e = tid; e < NV * (int)ntiles; e += NTHREADS)  // a slot per thread: no two waits in a row
+        if (!slot_read(slots + (e / NV) * kSlots + e % NV, epoch, s_val[e])) *s_ok = 0;
     __syncthreads();
+    double a[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) a[k] = 0.0;
+    for (int t = tid; t < (int)ntiles; t += NTHREADS) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) a[k] += s_val[t * NV + k];
+    }
+    block_sum_store<NV, double>(a, s_tot, s_red, ntiles < NTHREADS ? (int)ntiles : NTHREADS);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; k++) tot[k] = s_tot[k];
     return *s_ok != 0;
+}
+
+// p = p beta + r / diag with the roundings that the compiler gives OpCG1 (a
+// served solve runs the sweeps and equals the same solve alone).  Keeping
+// r / diag from step 2 would save an operation, 4 % here, but the rounding it
+// needs costs the FP64 sweep 2 % at 100^3.
+template <typename T>
+__device__ __forceinline__ T cg_direction(T p, T beta, T r, T inv)
+{
+    if constexpr (sizeof(T) == 8) return __fma_rn(r, inv, __dmul_rn(p, beta));
+    else return __fmaf_rn(r, inv, __fmul_rn(p, beta));
 }
 
 template <typename T>
@@ -70,9 +123,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
     __shared__ int s_job, s_ok;
     __shared__ Coef<T> C;
     __shared__ Scalars s_sc;
-    __shared__ double s_red[2 * 2 * (NTHREADS / 32)];
+    __shared__ double s_red[2 * 2 * (NTHREADS / 32)], s_val[2 * kResidentBlocks];
     const int tid = threadIdx.x;
-    if (tid == 0) s_job = find_job(L, (int64_t)blockIdx.x);
+    if (tid == 0) {
+        s_job = find_job(L, (int64_t)blockIdx.x);
+        s_ok = 1;
+    }
     __syncthreads();
     const Job &J = L.jobs[s_job];
     constexpr int W = (int)(sizeof(Scalars) / 4);
@@ -132,16 +188,18 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
         own_pair(R, k) = r;
     }
     __syncthreads();
+    auto inv_at = [&](int k, int c) {  // own point, 1/diagonal
+        return inv_of<T, false>(C, g, K[k + 1][ly + 1][2 * lp + 1 + c], Pos{gx + c, gy, z0 + k, 0});
+    };
 
     // p = p beta + r / diag at a point of the box (as OpCG1).
     auto direction = [&](int k, int row, int col, int x, int y, T r, T beta) {
         const T inv = inv_of<T, false>(C, g, K[k][row][col], Pos{x, y, z0 - 1 + k, 0});
         T &p = P[k][row][col + 1];
-        const T zi = r * inv;
-        p = p * beta + zi;
+        p = cg_direction<T>(p, beta, r, inv);
     };
 
-    uint32_t arrivals = 0;
+    ulonglong2 *slots = (ulonglong2 *)J.slots;
     bool ok = true;
     for (int it = 0; it < iters; it++) {
         const T beta = (T)s_sc.beta;
@@ -193,8 +251,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
         if (tid < zn * 2 * TY) rx = col_load(tid);
         for (int k = 0; k < zn; k++) {
             const Pair<T> r = own_pair(R, k);
-            if (v0) direction(k + 1, ly + 1, 2 * lp + 1, gx, gy, r.a, beta);
-            if (v1) direction(k + 1, ly + 1, 2 * lp + 2, gx + 1, gy, r.b, beta);
+            Pair<T> &p = *reinterpret_cast<Pair<T> *>(&P[k + 1][ly + 1][2 * lp + 2]);
+            if (v0) p.a = cg_direction<T>(p.a, beta, r.a, inv_at(k, 0));
+            if (v1) p.b = cg_direction<T>(p.b, beta, r.b, inv_at(k, 1));
         }
 #pragma unroll
         for (int s = 0; s < 2; s++) {
@@ -239,14 +298,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
             own_pair(Q, k) = q;
         }
         T va[1] = {pap.hi()};
-        block_sum_store<1, T>(va, J.part + local * NPART, s_red);
-        arrivals += (uint32_t)J.ntiles;
-        if (!(ok = job_barrier(J.counter, arrivals, &s_ok))) break;
-        {
-            double tot[1];
-            sum_partials<1>(J.part, J.ntiles, tot, s_red);
-            if (tid == 0) OpCG1<T, T>::finish(s_sc, tot);
-        }
+        const uint64_t epoch = s_sc.iter + 1;
+        double t1[1];
+        if (!(ok = exchange<1, T>(va, slots, local, J.ntiles, epoch, t1, s_red, s_val, &s_ok))) break;
+        if (tid == 0) OpCG1<T, T>::finish(s_sc, t1);
         __syncthreads();
         // Step 2.
         const T alpha = (T)s_sc.alpha;
@@ -261,26 +316,21 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
             x.a = x.a + alpha * p.a;
             r.a = r.a + (-alpha) * q.a;
             rr.add_prod(r.a, r.a);
-            rzd.add_prod(r.a, r.a * inv_of<T, false>(C, g, K[k + 1][ly + 1][2 * lp + 1], Pos{gx, gy, z0 + k, 0}));
+            rzd.add_prod(r.a, r.a * inv_at(k, 0));
             if (v1) {
                 x.b = x.b + alpha * p.b;
                 r.b = r.b + (-alpha) * q.b;
                 rr.add_prod(r.b, r.b);
-                rzd.add_prod(r.b, r.b * inv_of<T, false>(C, g, K[k + 1][ly + 1][2 * lp + 2], Pos{gx + 1, gy, z0 + k, 0}));
+                rzd.add_prod(r.b, r.b * inv_at(k, 1));
             }
             own_pair(R, k) = r;
             store2<T>(x_out, i, x.a, x.b, true, v1);
             store2<T>(r_out, i, r.a, r.b, true, v1);
         }
         T vb[2] = {rr.hi(), rzd.hi()};
-        block_sum_store<2, T>(vb, J.part + local * NPART + 1, s_red);
-        arrivals += (uint32_t)J.ntiles;
-        if (!(ok = job_barrier(J.counter, arrivals, &s_ok))) break;
-        {
-            double tot[2];
-            sum_partials<2>(J.part + 1, J.ntiles, tot, s_red);
-            if (tid == 0) OpCG2<T, T>::finish(s_sc, tot);
-        }
+        double t2[2];
+        if (!(ok = exchange<2, T>(vb, slots + 1, local, J.ntiles, epoch, t2, s_red, s_val, &s_ok))) break;
+        if (tid == 0) OpCG2<T, T>::finish(s_sc, t2);
         __syncthreads();
         if (s_sc.state != RUNNING) break;
     }
@@ -305,12 +355,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
 }
 
 // Blocks of zc planes that an SM holds: two by their registers, and by their
-// shared memory (static arrays 2.6 KB in F64, 7.7 KB in F32; 1 KB a block and
+// shared memory (static arrays 7.5 KB in F64, 12.6 KB in F32; 1 KB a block and
 // 1 KB an SM are the system's).
 template <typename T>
 constexpr int resident_fit(int zc)
 {
-    const size_t block = resident_smem<T>(zc) + (sizeof(T) == 8 ? 4096 : 8192) + 1024, sm = 227 * 1024 + 1024;
+    const size_t block = resident_smem<T>(zc) + (sizeof(T) == 8 ? 8192 : 13312) + 1024, sm = 227 * 1024 + 1024;
     return zc > kResidentDepth ? 0 : block * 2 <= sm ? 2 : block <= sm ? 1 : 0;
 }
 

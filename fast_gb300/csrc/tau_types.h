@@ -116,6 +116,7 @@ struct Job {
     void *r0;                    // BiCGSTAB shadow residual (T)
     void *p[2];                  // search direction ping-pong (T)
     void *v[2];                  // BiCGSTAB v ping-pong (T)
+    void *slots;                 // resident CG: the blocks' partial sums with their iteration
     void *q;                     // F64 / F32 CG: q = A p, kept from step 1 to the pointwise step 2 (null: no room,
                                  // step 2 evaluates it again)
     void *t;                     // MIXED BiCGSTAB: t = A s, kept from step 2 to step 1 (FP32)
