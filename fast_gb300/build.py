@@ -20,7 +20,8 @@ OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libfasttau.so")
 CLI = os.path.join(OUT, "fast")  # the `fast tau` command-line drop-in
 
-CUDA_SOURCES = ["kern_f64.cu", "kern_f32.cu", "kern_misc.cu", "tau_host.cu", "noalloc.cu", "ccl.cu", "serve.cu",
+CUDA_SOURCES = ["kern_f64.cu", "kern_f32.cu", "kern_misc.cu", "kern_f64_narrow.cu", "kern_f32_narrow.cu",
+                "kern_misc_narrow.cu", "tau_host.cu", "noalloc.cu", "ccl.cu", "serve.cu",
                 "volume_ops.cu", "alpha.cu"]
 CXX_SOURCES = ["gen.cpp", "tiff_folder.cpp"]
 CLI_SOURCE = "fast_cli.cpp"

@@ -118,7 +118,6 @@ static void dispatch(Step s, const Launch &L, cudaStream_t st)
     using T = float;
     switch (s) {
     case Step::INIT_CG: go<OpInit<T, ST, false>>(L, st); break;
-    case Step::INIT_BI: go<OpInit<T, ST, true>>(L, st); break;
     case Step::CG1: go<OpCG1<T, ST>>(L, st); break;
     case Step::CG2: go<OpCG2<T, ST>>(L, st); break;
     default: break;  // replacement steps are MIXED-only (kern_misc.cu)
@@ -126,10 +125,13 @@ static void dispatch(Step s, const Launch &L, cudaStream_t st)
     if constexpr (std::is_same<ST, float>::value) {  // MIXED BiCGSTAB has its own two sweeps
         switch (s) {
         case Step::CG2_Q: pointwise_kernel<PwCG2<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
+#if FAST_TAU_TX == 64
+        case Step::INIT_BI: go<OpInit<T, ST, true>>(L, st); break;
         case Step::BI_RESTART: go<OpBiRestart<T, ST>>(L, st); break;
         case Step::BI1: go<OpBi1<T, ST>>(L, st); break;
         case Step::BI2: go<OpBi2<T, ST>>(L, st); break;
         case Step::BI3: pointwise_kernel<PwBi3<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
+#endif
         default: break;
         }
     }
@@ -141,45 +143,57 @@ static cudaError_t configure()
     using T = float;
     cudaError_t e = cudaSuccess, r;
     if ((r = cfg<OpInit<T, ST, false>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpInit<T, ST, true>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpCG1<T, ST>>()) != cudaSuccess) e = r;
     if ((r = cfg<OpCG2<T, ST>>()) != cudaSuccess) e = r;
     if constexpr (std::is_same<ST, float>::value) {
+#if FAST_TAU_TX == 64
+        if ((r = cfg<OpInit<T, ST, true>>()) != cudaSuccess) e = r;
         if ((r = cfg<OpBiRestart<T, ST>>()) != cudaSuccess) e = r;
         if ((r = cfg<OpBi1<T, ST>>()) != cudaSuccess) e = r;
         if ((r = cfg<OpBi2<T, ST>>()) != cudaSuccess) e = r;
+#endif
     }
     return e;
 }
 
-cudaError_t configure_f32()
+template <>
+cudaError_t Kernels<TX>::configure_f32()
 {
-    cudaError_t a = configure<float>(), b = configure<double>();
-    cudaError_t c = cudaFuncSetAttribute(sweep_kernel_mb<OpBiK1, kStagesK1, kBlocksK1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         sweep_dyn_smem<OpBiK1, kStagesK1>());
-    cudaError_t d = cfg<OpBiK2>();
-    cudaError_t f = cudaFuncSetAttribute(sweep_kernel_mb<OpCGF, kStagesCGF, kBlocksCGF>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         sweep_dyn_smem<OpCGF, kStagesCGF>());
-    const cudaError_t g = configure_resident<float>();
-    if (a != cudaSuccess) return a;
-    if (g != cudaSuccess) return g;
-    if (b != cudaSuccess) return b;
-    if (f != cudaSuccess) return f;
-    return c != cudaSuccess ? c : d;
+    cudaError_t e[6] = {configure<float>(), configure<double>(), configure_resident<float>()};
+#if FAST_TAU_TX == 64
+    e[3] = cudaFuncSetAttribute(sweep_kernel_mb<OpBiK1, kStagesK1, kBlocksK1>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_dyn_smem<OpBiK1, kStagesK1>());
+    e[4] = cfg<OpBiK2>();
+    e[5] = cudaFuncSetAttribute(sweep_kernel_mb<OpCGF, kStagesCGF, kBlocksCGF>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_dyn_smem<OpCGF, kStagesCGF>());
+#endif
+    for (cudaError_t x : e)
+        if (x != cudaSuccess) return x;
+    return cudaSuccess;
 }
 
-int resident_per_sm(bool f32, int zc) { return f32 ? resident_fit<float>(zc) : resident_fit<double>(zc); }
+template <>
+int Kernels<TX>::resident_per_sm(bool f32, int zc)
+{
+    return f32 ? resident_fit<float>(zc) : resident_fit<double>(zc);
+}
 
-cudaError_t launch_resident_f32(const Launch &L, int zc, int iters, cudaStream_t st)
+template <>
+cudaError_t Kernels<TX>::resident_f32(const Launch &L, int zc, int iters, cudaStream_t st)
 {
     return launch_resident<float>(L, zc, iters, st);
 }
 
-void launch_pure_f32(Step s, const Launch &L, cudaStream_t st) { dispatch<float>(s, L, st); }
-void launch_mixed_inner(Step s, const Launch &L, cudaStream_t st)
+template <>
+void Kernels<TX>::pure_f32(Step s, const Launch &L, cudaStream_t st)
 {
+    dispatch<float>(s, L, st);
+}
+
+template <>
+void Kernels<TX>::mixed_inner(Step s, const Launch &L, cudaStream_t st)
+{
+#if FAST_TAU_TX == 64
     if (s == Step::BI_K1)
         sweep_kernel_mb<OpBiK1, kStagesK1, kBlocksK1>
             <<<(unsigned)L.nblocks, sweep_threads<OpBiK1>(), sweep_dyn_smem<OpBiK1, kStagesK1>(), st>>>(L);
@@ -187,7 +201,9 @@ void launch_mixed_inner(Step s, const Launch &L, cudaStream_t st)
     else if (s == Step::CG_F)
         sweep_kernel_mb<OpCGF, kStagesCGF, kBlocksCGF>
             <<<(unsigned)L.nblocks, sweep_threads<OpCGF>(), sweep_dyn_smem<OpCGF, kStagesCGF>(), st>>>(L);
-    else dispatch<double>(s, L, st);
+    else
+#endif
+        dispatch<double>(s, L, st);
 }
 
 }  // namespace ft

@@ -1,0 +1,3 @@
+// FP32 and MIXED CG on 32 x 16 tiles.
+#define FAST_TAU_TX 32
+#include "kern_f32.cu"

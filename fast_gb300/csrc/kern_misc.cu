@@ -10,7 +10,7 @@ constexpr int kStages = 3;
 // most: its kernels walk the tiles with one resident wave of blocks
 // (sweep_kernel_tiles), sized here from the occupancy of each kernel.
 // Index: [float-float][BiCGSTAB].
-int g_resident[2][2] = {};
+static int g_resident[2][2] = {};
 
 template <class Op>
 static void launch_tiles(const Launch &L, cudaStream_t st, int64_t resident)
@@ -19,16 +19,19 @@ static void launch_tiles(const Launch &L, cudaStream_t st, int64_t resident)
     sweep_kernel_tiles<Op, kStages><<<grid, sweep_threads<Op>(), sweep_dyn_smem<Op, kStages>(), st>>>(L);
 }
 
-void launch_replace(bool bicg, bool ff, const Launch &L, cudaStream_t st)
+template <>
+void Kernels<TX>::replace(bool bicg, bool ff, const Launch &L, cudaStream_t st)
 {
     const int64_t resident = g_resident[ff][bicg];
-    if (ff) {
-        if (bicg) launch_tiles<OpReplaceBi2<FF>>(L, st, resident);
-        else launch_tiles<OpReplace<false, FF>>(L, st, resident);
-    } else {
-        if (bicg) launch_tiles<OpReplaceBi2<double>>(L, st, resident);
-        else launch_tiles<OpReplace<false, double>>(L, st, resident);
+#if FAST_TAU_TX == 64
+    if (bicg) {
+        if (ff) launch_tiles<OpReplaceBi2<FF>>(L, st, resident);
+        else launch_tiles<OpReplaceBi2<double>>(L, st, resident);
+        return;
     }
+#endif
+    if (ff) launch_tiles<OpReplace<false, FF>>(L, st, resident);
+    else launch_tiles<OpReplace<false, double>>(L, st, resident);
 }
 
 template <class Op>
@@ -46,17 +49,21 @@ static cudaError_t configure_tiles(int &resident)
     return e;
 }
 
-cudaError_t configure_misc()
+template <>
+cudaError_t Kernels<TX>::configure_replace()
 {
-    cudaError_t e[4] = {configure_tiles<OpReplaceBi2<double>>(g_resident[0][1]),
-                        configure_tiles<OpReplace<false, double>>(g_resident[0][0]),
-                        configure_tiles<OpReplaceBi2<FF>>(g_resident[1][1]),
+    cudaError_t e[4] = {configure_tiles<OpReplace<false, double>>(g_resident[0][0]),
                         configure_tiles<OpReplace<false, FF>>(g_resident[1][0])};
+#if FAST_TAU_TX == 64
+    e[2] = configure_tiles<OpReplaceBi2<double>>(g_resident[0][1]);
+    e[3] = configure_tiles<OpReplaceBi2<FF>>(g_resident[1][1]);
+#endif
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
 }
 
+#if FAST_TAU_TX == 64  // the kernels below take either tile
 void launch_count_zero(const uint8_t *mask, uint64_t n, unsigned long long *total, cudaStream_t st)
 {
     const uint64_t want = (n / 16 + 255) / 256, most = 152 * 8;  // one wave of full blocks
@@ -91,5 +98,7 @@ void launch_ff_to_double(const void *src, double *dst, int64_t n, cudaStream_t s
     if (blocks < 1) blocks = 1;
     ff_to_double_kernel<<<(unsigned)blocks, 256, 0, st>>>((const float2 *)src, dst, n);
 }
+
+#endif
 
 }  // namespace ft

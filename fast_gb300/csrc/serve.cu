@@ -78,6 +78,9 @@ struct Group {
     cudaEvent_t done = nullptr;
 };
 
+// The groups of a context: one per solver, and CG on narrow tiles.
+constexpr int kGroups = 3, kNarrowGroup = 2;
+
 struct Ctx {
     fast_ctx_config cfg;
     fast_tau_params P[2];  // by solver
@@ -89,12 +92,12 @@ struct Ctx {
     char *d_bnd = nullptr;          // domain-face tables of the three primary axes
     Scalars *h_snap[2] = {};        // pinned copies of the slot array, one per chunk in flight
     Scalars *h_init = nullptr;      // pinned staging of new solves' scalars
-    Job *h_stage = nullptr;         // pinned staging of job tables (5 regions of kMax)
+    Job *h_stage = nullptr;         // pinned staging of job tables (kStageRegions of kMax)
     Job *d_tmp[3] = {};             // device job tables for retire / code / init launches
     std::vector<int> free_slots;
     std::deque<Request> pending;
     std::vector<Active> active;
-    Group groups[2];
+    Group groups[kGroups];
     bool dirty = true;
     // Up to two chunks in flight: the GPU runs the next one while the host
     // retires and admits from the snapshot of the previous one.
@@ -127,12 +130,14 @@ int steps_of(const Ctx &C, int solver, std::vector<Step> &steps)
     return FAST_OK;
 }
 
-void dispatch(const Ctx &C, Step s, const Launch &L, cudaStream_t st)
+constexpr int kStageRegions = 2 + 2 * kGroups;
+
+int group_of(const Active &A)
 {
-    if (C.cfg.precision == FAST_PREC_MIXED) dispatch_mixed(s, L, st);
-    else if (C.cfg.precision == FAST_PREC_F64) launch_pure_f64(s, L, st);
-    else launch_pure_f32(s, L, st);
+    return A.req.solver == FAST_SOLVER_CG && A.job.tile_w == kNarrowTX ? kNarrowGroup : A.req.solver;
 }
+int group_solver(int g) { return g == kNarrowGroup ? FAST_SOLVER_CG : g; }
+int group_width(int g) { return g == kNarrowGroup ? kNarrowTX : TX; }
 
 // Copies `n` descriptors to a device job table with consecutive tile numbering.
 int upload_jobs(Ctx &C, Job *stage, const std::vector<const Job *> &src, Job *d_dst, int64_t &nblocks)
@@ -278,16 +283,17 @@ int admit(Ctx &C)
     if (C.cfg.precision == FAST_PREC_MIXED) {
         launch_init64(Launch{C.d_tmp[1], (int32_t)jobs.size(), 0, nb, nullptr}, C.st);
     } else {
-        for (int g = 0; g < 2; g++) {
+        for (int g = 0; g < kGroups; g++) {
             std::vector<const Job *> gj;
             for (int a : fresh)
-                if (C.active[a].req.solver == g) gj.push_back(&C.active[a].job);
+                if (group_of(C.active[a]) == g) gj.push_back(&C.active[a].job);
             if (gj.empty()) continue;
             int64_t gb = 0;
-            s = upload_jobs(C, C.h_stage + (2 + g) * C.kMax, gj, C.d_tmp[2 - g], gb);
+            s = upload_jobs(C, C.h_stage + (2 + g) * C.kMax, gj, C.d_tmp[2], gb);
             if (s != FAST_OK) return s;
-            dispatch(C, g == FAST_SOLVER_CG ? Step::INIT_CG : Step::INIT_BI, Launch{C.d_tmp[2 - g], (int32_t)gj.size(), 0, gb, nullptr},
-                     C.st);
+            step_launcher(C.cfg.precision, group_width(g))(
+                group_solver(g) == FAST_SOLVER_CG ? Step::INIT_CG : Step::INIT_BI,
+                Launch{C.d_tmp[2], (int32_t)gj.size(), 0, gb, nullptr}, C.st);
         }
     }
     SV(cudaGetLastError());
@@ -298,13 +304,14 @@ int admit(Ctx &C)
 int rebuild(Ctx &C)
 {
     // The pinned staging regions of this step may still feed copies queued
-    // above; the group tables use their own regions (4 and 5 of the stage).
-    for (int g = 0; g < 2; g++) {
+    // above; the group tables use their own regions (the last kGroups of
+    // the stage).
+    for (int g = 0; g < kGroups; g++) {
         Group &G = C.groups[g];
         G.members.clear();
         std::vector<const Job *> jobs;
         for (int a = 0; a < (int)C.active.size(); a++)
-            if (C.active[a].req.solver == g) {
+            if (group_of(C.active[a]) == g) {
                 G.members.push_back(a);
                 jobs.push_back(&C.active[a].job);
             }
@@ -313,19 +320,16 @@ int rebuild(Ctx &C)
             G.exec = nullptr;
         }
         if (jobs.empty()) continue;
-        int s = upload_jobs(C, C.h_stage + (4 + g) * C.kMax, jobs, G.d_jobs, G.nblocks);
+        int s = upload_jobs(C, C.h_stage + (2 + kGroups + g) * C.kMax, jobs, G.d_jobs, G.nblocks);
         if (s != FAST_OK) return s;
         std::vector<Step> steps;
-        steps_of(C, g, steps);
+        steps_of(C, group_solver(g), steps);
         const bool mixed = C.cfg.precision == FAST_PREC_MIXED;
         // the replacement gate opens for the group's new solves (they start
         // with a pending replacement); an extra scan for the others is cheap
         if (mixed) SV(cudaMemsetAsync(G.d_gate, 1, 1, C.st));
         const Launch L{G.d_jobs, (int32_t)jobs.size(), 0, G.nblocks, mixed ? G.d_gate : nullptr};
-        s = capture_chunk(C.st, L, steps, C.cfg.chunk,
-                          C.cfg.precision == FAST_PREC_MIXED ? dispatch_mixed
-                          : C.cfg.precision == FAST_PREC_F64 ? launch_pure_f64 : launch_pure_f32,
-                          &G.exec);
+        s = capture_chunk(C.st, L, steps, C.cfg.chunk, step_launcher(C.cfg.precision, group_width(g)), &G.exec);
         if (s != FAST_OK) return s;
     }
     C.dirty = false;
@@ -339,7 +343,8 @@ int launch_chunk(Ctx &C)
     // chunks run side by side, behind everything queued on the context's stream
     // and before anything queued on it from here on.  One after the other, each
     // group's sweeps left the GPU part idle in their last wave of blocks: a
-    // burst of 24 requests of both solvers took 157 ms, side by side 138 ms.
+    // burst of 24 requests of both solvers took 157 ms, side by side 138 ms
+    // (132 with the narrow tiles' group).
     SV(cudaEventRecord(C.ev_fork, C.st));
     for (Group &G : C.groups) {
         if (!G.exec) continue;
@@ -460,28 +465,27 @@ int create(const fast_ctx_config &cfg, Ctx **out)
         cudaEventCreateWithFlags(&C->ev_copy, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&C->ev_fork, cudaEventDisableTiming) != cudaSuccess)
         return fin(ft_fail(FAST_CUDA_ERROR, "stream/event creation failed"));
+    if (cudaMallocAsync((void **)&C->d_slots, sizeof(Scalars) * K, C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_cnt, sizeof(uint32_t) * K, C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_tmp[0], sizeof(Job) * K, C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_tmp[1], sizeof(Job) * K, C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_tmp[2], sizeof(Job) * K, C->st) != cudaSuccess ||
+        cudaMallocAsync((void **)&C->d_bnd, 3 * bnd_bytes(cfg.precision), C->st) != cudaSuccess)
+        return fin(ft_fail(FAST_NOMEM, "context tables"));
     for (Group &G : C->groups)
         if (cudaStreamCreateWithFlags(&G.st, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&G.done, cudaEventDisableTiming) != cudaSuccess)
             return fin(ft_fail(FAST_CUDA_ERROR, "stream/event creation failed"));
-    if (cudaMallocAsync((void **)&C->d_slots, sizeof(Scalars) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->d_cnt, sizeof(uint32_t) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->groups[0].d_jobs, sizeof(Job) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->groups[1].d_jobs, sizeof(Job) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->d_tmp[0], sizeof(Job) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->d_tmp[1], sizeof(Job) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->d_tmp[2], sizeof(Job) * K, C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->groups[0].d_gate, sizeof(uint32_t), C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->groups[1].d_gate, sizeof(uint32_t), C->st) != cudaSuccess ||
-        cudaMallocAsync((void **)&C->d_bnd, 3 * bnd_bytes(cfg.precision), C->st) != cudaSuccess)
-        return fin(ft_fail(FAST_NOMEM, "context tables"));
+    for (Group &G : C->groups)
+        if (cudaMallocAsync((void **)&G.d_jobs, sizeof(Job) * K, C->st) != cudaSuccess ||
+            cudaMallocAsync((void **)&G.d_gate, sizeof(uint32_t), C->st) != cudaSuccess ||
+            cudaMemsetAsync(G.d_gate, 0, sizeof(uint32_t), C->st) != cudaSuccess)
+            return fin(ft_fail(FAST_NOMEM, "context tables"));
     if (cudaMemsetAsync(C->d_cnt, 0, sizeof(uint32_t) * K, C->st) != cudaSuccess ||
-        cudaMemsetAsync(C->groups[0].d_gate, 0, sizeof(uint32_t), C->st) != cudaSuccess ||
-        cudaMemsetAsync(C->groups[1].d_gate, 0, sizeof(uint32_t), C->st) != cudaSuccess ||
         cudaMallocHost(&C->h_snap[0], sizeof(Scalars) * K) != cudaSuccess ||
         cudaMallocHost(&C->h_snap[1], sizeof(Scalars) * K) != cudaSuccess ||
         cudaMallocHost(&C->h_init, sizeof(Scalars) * K) != cudaSuccess ||
-        cudaMallocHost(&C->h_stage, sizeof(Job) * 6 * K) != cudaSuccess)
+        cudaMallocHost(&C->h_stage, sizeof(Job) * kStageRegions * K) != cudaSuccess)
         return fin(ft_fail(FAST_NOMEM, "context staging"));
     // The domain-face tables depend on the context's coefficients alone.
     for (int a = 0; a < 3; a++) {

@@ -14,6 +14,7 @@
 #include "tau_types.h"
 
 namespace ft {
+inline namespace FT_TILES {
 
 // ---------------------------------------------------------------------------
 // Coefficient tables, staged in shared memory at block start.
@@ -702,4 +703,5 @@ __device__ __forceinline__ int find_job(const Launch &L, int64_t b)
     return lo;
 }
 
+}  // namespace FT_TILES
 }  // namespace ft

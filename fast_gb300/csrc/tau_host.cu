@@ -92,9 +92,11 @@ int Engine::init(int dev)
     CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CU(cudaMallocHost(&h_sc, sizeof(Scalars) * 2 * kMaxJobs));
     CU(cudaMallocHost(&h_jobs, sizeof(Job) * 2 * kMaxJobs));  // jobs + one code job per volume
-    cudaError_t ce = configure_f64();
-    if (ce == cudaSuccess) ce = configure_f32();
-    if (ce == cudaSuccess) ce = configure_misc();
+    cudaError_t ce = cudaSuccess;
+    for (auto configure : {Kernels<TX>::configure_f64, Kernels<TX>::configure_f32, Kernels<TX>::configure_replace,
+                           Kernels<kNarrowTX>::configure_f64, Kernels<kNarrowTX>::configure_f32,
+                           Kernels<kNarrowTX>::configure_replace})
+        if (ce == cudaSuccess) ce = configure();
     if (ce != cudaSuccess) return fail(FAST_CUDA_ERROR, "kernel configuration: %s", cudaGetErrorString(ce));
     ft_retain_pool_memory(dev);
     return FAST_OK;
@@ -254,13 +256,14 @@ void fill_tables(Job &J, double d0, double d1, int face_mean)
 
 void job_coefficients(Job &J, const fast_tau_params &P) { fill_tables(J, P.d0, P.d1, P.face_mean); }
 
-Geometry make_geometry(int64_t nx, int64_t ny, int64_t nz, int zc_req)
+Geometry make_geometry(int64_t nx, int64_t ny, int64_t nz, int zc_req, int width)
 {
     Geometry g;
     g.nx = nx; g.ny = ny; g.nz = nz;
     g.N = nx * ny * nz;
-    g.tx = (int)((nx + TX - 1) / TX);
-    g.ty = (int)((ny + TY - 1) / TY);
+    const int height = TX * TY / width;
+    g.tx = (int)((nx + width - 1) / width);
+    g.ty = (int)((ny + height - 1) / height);
     int zc = zc_req > 0 ? zc_req : env_int("FAST_TAU_ZC", kSlabDepth);
     if (zc < 1) zc = 1;
     if (zc > nz) zc = (int)nz;
@@ -279,7 +282,7 @@ PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 std::mutex g_encode_mu;
 
 int tensor_map(CUtensorMap *tm, const void *base, int es, int64_t nx, int64_t ny, int64_t nz, int64_t pitch,
-               bool interior = false)
+               int width, bool interior = false)
 {
     {
         std::lock_guard<std::mutex> lk(g_encode_mu);
@@ -296,10 +299,11 @@ int tensor_map(CUtensorMap *tm, const void *base, int es, int64_t nx, int64_t ny
                                  : (es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64);
     const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
     const cuuint64_t strides[2] = {(cuuint64_t)(pitch * es), (cuuint64_t)(pitch * ny * es)};
-    // Box: the TX x TY tile plus a one-voxel halo, widened in x so that its
+    // Box: the tile (width x 512 / width) plus a one-voxel halo, widened in x so that its
     // start (x0 - 16/es) and width are multiples of 16 bytes; or (interior)
     // the tile alone, for streams read only at a block's own points.
-    const cuuint32_t box[3] = {(cuuint32_t)(interior ? TX : TX + 2 * (16 / es)), (cuuint32_t)(interior ? TY : HY), 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)(interior ? width : width + 2 * (16 / es)),
+                               (cuuint32_t)(TX * TY / width + (interior ? 0 : 2)), 1u};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUresult r = g_encode(tm, dt, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -310,7 +314,7 @@ int tensor_map(CUtensorMap *tm, const void *base, int es, int64_t nx, int64_t ny
 
 // Captures `chunk` iterations of `steps` on `st` into an executable graph.
 int capture_chunk(cudaStream_t st, const Launch &L, const std::vector<Step> &steps, int chunk,
-                  void (*launch)(Step, const Launch &, cudaStream_t), cudaGraphExec_t *exec)
+                  StepLauncher launch, cudaGraphExec_t *exec)
 {
     cudaGraph_t graph = nullptr;
     CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -328,7 +332,7 @@ int capture_chunk(cudaStream_t st, const Launch &L, const std::vector<Step> &ste
 // RUNNING; polls the device scalars one chunk behind so the queue never
 // drains while the host waits.
 int iterate(Engine &E, const Launch &L, int njobs, Scalars *d_sc, const std::vector<Step> &steps,
-            void (*launch)(Step, const Launch &, cudaStream_t), uint64_t max_iter)
+            StepLauncher launch, uint64_t max_iter)
 {
     cudaStream_t st = E.stream;
     const int chunk = std::max(1, env_int("FAST_TAU_CHUNK", 16));
@@ -413,9 +417,12 @@ int iterate(Engine &E, const Launch &L, int njobs, Scalars *d_sc, const std::vec
 // are done, so a long one costs nothing at the end of a solve.  launched =
 // false: the first launch was refused and nothing ran.
 int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, bool f32, int zc,
-                     uint64_t max_iter, bool &launched)
+                     int width, uint64_t max_iter, bool &launched)
 {
     constexpr int kIters = 128;
+    const bool narrow = width == kNarrowTX;
+    auto launch = f32 ? (narrow ? Kernels<kNarrowTX>::resident_f32 : Kernels<TX>::resident_f32)
+                      : (narrow ? Kernels<kNarrowTX>::resident_f64 : Kernels<TX>::resident_f64);
     cudaStream_t st = E.stream;
     cudaError_t cerr = cudaSuccess;
     cudaEvent_t ev[2];
@@ -424,7 +431,7 @@ int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, bool 
     const uint64_t max_launches = max_iter / kIters + 4;
     int status = FAST_OK;
     for (uint64_t k = 0; k < max_launches; k++) {
-        cerr = (f32 ? launch_resident_f32 : launch_resident_f64)(L, zc, kIters, st);
+        cerr = launch(L, zc, kIters, st);
         if (cerr != cudaSuccess && k == 0) {
             cudaGetLastError();
             launched = false;
@@ -450,8 +457,6 @@ int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, bool 
     return status;
 }
 
-void dispatch_f64(Step s, const Launch &L, cudaStream_t st) { launch_pure_f64(s, L, st); }
-void dispatch_f32(Step s, const Launch &L, cudaStream_t st) { launch_pure_f32(s, L, st); }
 std::vector<Step> mixed_steps(int solver, bool ff)
 {
     if (solver == FAST_SOLVER_CG) {
@@ -461,15 +466,24 @@ std::vector<Step> mixed_steps(int solver, bool ff)
     return {ff ? Step::REPLACE_BI_FF : Step::REPLACE_BI, Step::BI_K1, Step::BI_K2};
 }
 
+template <int W>
 void dispatch_mixed(Step s, const Launch &L, cudaStream_t st)
 {
     switch (s) {
-    case Step::REPLACE_CG: launch_replace(false, false, L, st); break;
-    case Step::REPLACE_BI: launch_replace(true, false, L, st); break;
-    case Step::REPLACE_CG_FF: launch_replace(false, true, L, st); break;
-    case Step::REPLACE_BI_FF: launch_replace(true, true, L, st); break;
-    default: launch_mixed_inner(s, L, st);
+    case Step::REPLACE_CG: Kernels<W>::replace(false, false, L, st); break;
+    case Step::REPLACE_BI: Kernels<W>::replace(true, false, L, st); break;
+    case Step::REPLACE_CG_FF: Kernels<W>::replace(false, true, L, st); break;
+    case Step::REPLACE_BI_FF: Kernels<W>::replace(true, true, L, st); break;
+    default: Kernels<W>::mixed_inner(s, L, st);
     }
+}
+
+StepLauncher step_launcher(int prec, int width)
+{
+    const bool narrow = width == kNarrowTX;
+    if (prec == FAST_PREC_F64) return narrow ? Kernels<kNarrowTX>::pure_f64 : Kernels<TX>::pure_f64;
+    if (prec == FAST_PREC_F32) return narrow ? Kernels<kNarrowTX>::pure_f32 : Kernels<TX>::pure_f32;
+    return narrow ? dispatch_mixed<kNarrowTX> : dispatch_mixed<TX>;
 }
 
 int status_of(int state)
@@ -513,7 +527,31 @@ size_t code_bytes(int64_t nx, int64_t ny, int64_t nz) { return align_up((size_t)
 // tuned_depth a whole launch.
 #include "slab_table.inc"
 
+bool cg_fused_enabled();
+
 namespace {
+// The tile width of a launch: 32 x 16 tiles for CG where they cover the
+// volumes with at least 3 % fewer tiles than 64 x 8.  A tile costs the same
+// whether its columns lie inside the volume or not, so an axis of 65 to 96
+// voxels pays for 128 with the wide tile.  us per iteration wide -> narrow:
+// MIXED CG 45.3 -> 34.1 for 3 x 96^3 (25 % fewer tiles), 117 -> 99.5 for 3 x
+// 150^3, 219 -> 187 for 3 x 200 x 180 x 190, 534 -> 522 at 450 x 390 x 420 (4 %);
+// F64 60.2 -> 51.2 at 84 x 100 x 110.  At equal counts the wide tile is 1 to
+// 2.5 % faster (318 against 322 at 3 x 256^3, 114 against 117 at 256^3).
+// BiCGSTAB keeps the wide tile: its iteration count follows the order of its
+// sums.  So does the opt-in one-sweep CG, and a launch with FAST_TAU_ZC, where
+// batches equal single solves bit for bit.
+int launch_width(const std::vector<const int64_t *> &dims, int solver)
+{
+    if (solver != FAST_SOLVER_CG || cg_fused_enabled() || env_int("FAST_TAU_ZC", 0) > 0) return TX;
+    int64_t wide = 0, narrow = 0;
+    for (const int64_t *d : dims) {
+        wide += make_geometry(d[0], d[1], d[2], 1).ntiles;
+        narrow += make_geometry(d[0], d[1], d[2], 1, kNarrowTX).ntiles;
+    }
+    return narrow * 100 <= wide * 97 ? kNarrowTX : TX;
+}
+
 std::atomic<int> g_slab[3][2][kSlabClasses];
 std::atomic<bool> g_slab_set[3][2];  // a table was installed at run time
 std::once_flag g_slab_once;
@@ -557,11 +595,11 @@ constexpr DepthModel kDepthModel[3] = {
 };
 constexpr int kSms = 152;
 
-double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims, int d)
+double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims, int width, int d)
 {
     int64_t blocks = 0, deepest = 1;
     for (const int64_t *v : dims) {
-        blocks += make_geometry(v[0], v[1], v[2], d).ntiles;
+        blocks += make_geometry(v[0], v[1], v[2], d, width).ntiles;
         deepest = std::max(deepest, std::min<int64_t>(d, v[2]));
     }
     const int64_t cap = (int64_t)kSms * M.resident, full = blocks / cap, rem = blocks % cap;
@@ -583,19 +621,19 @@ double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims
 // only read more halo planes on a busy one.  (No MIXED launch takes a single
 // plane, so that the directions of a volume of a few blocks keep the depth,
 // and with it the last bits, that each has alone.)
-int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int table)
+int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int width, int table)
 {
     const DepthModel &M = kDepthModel[prec];
     int64_t nz = 1;
     for (const int64_t *v : dims) nz = std::max(nz, v[2]);
     const int64_t least = prec != FAST_PREC_MIXED ? 1 : (dims.size() == 1 ? std::max(2, table * 3 / 4) : 2);
-    double best = 0.95 * modelled_us(M, dims, table);
+    double best = 0.95 * modelled_us(M, dims, width, table);
     int depth = table;
     for (int64_t d = std::min<int64_t>(nz, 1024); d >= least;) {
         const int64_t n = (nz + d - 1) / d;
         d = (nz + n - 1) / n;  // even slabs
         if (d < least) break;
-        const double us = modelled_us(M, dims, (int)d);
+        const double us = modelled_us(M, dims, width, (int)d);
         if (us < best) {
             best = us;
             depth = (int)d;
@@ -621,7 +659,7 @@ constexpr ResidentModel kResidentModel[2] = {
     {{8.4, 10.4}, {0.91, 1.15}},  // F32
 };
 
-int resident_depth(int prec, const std::vector<const int64_t *> &dims, int table)
+int resident_depth(int prec, const std::vector<const int64_t *> &dims, int width, int table)
 {
     if (prec == FAST_PREC_MIXED) return 0;
     const bool f32 = prec == FAST_PREC_F32;
@@ -629,15 +667,15 @@ int resident_depth(int prec, const std::vector<const int64_t *> &dims, int table
     int64_t nz = 1;
     for (const int64_t *v : dims) nz = std::max(nz, v[2]);
     int64_t depth = 0;
-    double best = 0.95 * modelled_us(kDepthModel[prec], dims, modelled_depth(prec, dims, table));
+    double best = 0.95 * modelled_us(kDepthModel[prec], dims, width, modelled_depth(prec, dims, width, table));
     for (int64_t d = std::min<int64_t>(nz, kResidentDepth); d >= 1; d--) {
         const int64_t n = (nz + d - 1) / d;
         d = (nz + n - 1) / n;  // even slabs
         int64_t blocks = 0;
-        for (const int64_t *v : dims) blocks += make_geometry(v[0], v[1], v[2], (int)d).ntiles;
+        for (const int64_t *v : dims) blocks += make_geometry(v[0], v[1], v[2], (int)d, width).ntiles;
         if (blocks > kResidentBlocks) break;
         const int b = blocks > kSms;
-        if (resident_per_sm(f32, (int)d) < b + 1) continue;
+        if ((width == TX ? Kernels<TX>::resident_per_sm : Kernels<kNarrowTX>::resident_per_sm)(f32, (int)d) < b + 1) continue;
         const double us = M.base[b] + (double)d * M.plane[b];
         if (us < best) {
             best = us;
@@ -664,9 +702,10 @@ int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims, 
         const int t = g_slab[prec][solver][slab_class(W)].load(std::memory_order_relaxed);
         if (t > 0) {
             if (solver != FAST_SOLVER_CG || g_slab_set[prec][solver].load(std::memory_order_relaxed)) return t;
-            const int r = resident_depth(prec, dims, t);
+            const int width = launch_width(dims, solver);
+            const int r = resident_depth(prec, dims, width, t);
             if (resident) *resident = r > 0;
-            return r > 0 ? r : modelled_depth(prec, dims, t);
+            return r > 0 ? r : modelled_depth(prec, dims, width, t);
         }
     }
     int zc = kSlabDepth;
@@ -678,6 +717,12 @@ int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims, 
     return zc;
 }
 }  // namespace
+
+int tile_width(int64_t nx, int64_t ny, int64_t nz, int solver)
+{
+    const int64_t d[3] = {nx, ny, nz};
+    return launch_width({d}, solver);
+}
 
 int slab_depth(int64_t nx, int64_t ny, int64_t nz, int prec, int solver)
 {
@@ -712,7 +757,7 @@ bool cg_fused_enabled()
     return on != 0;
 }
 
-size_t job_bytes(int64_t nx, int64_t ny, int64_t nz, int prec, int solver, int zc)
+size_t job_bytes(int64_t nx, int64_t ny, int64_t nz, int prec, int solver, int zc, int width)
 {
     const bool mixed = prec == FAST_PREC_MIXED;
     const size_t vec_t = (prec == FAST_PREC_F64) ? 8 : 4;
@@ -722,7 +767,8 @@ size_t job_bytes(int64_t nx, int64_t ny, int64_t nz, int prec, int solver, int z
     const bool fused = mixed && solver == FAST_SOLVER_CG && cg_fused_enabled();
     const size_t nvec = (solver == FAST_SOLVER_CG && !fused) ? 4 : (mixed ? 9 : 8);
     const size_t NP = (size_t)(row_pitch(nx) * ny * nz);
-    const Geometry G = make_geometry(nx, ny, nz, zc > 0 ? zc : slab_depth(nx, ny, nz, prec, solver));
+    if (width <= 0) width = tile_width(nx, ny, nz, solver);
+    const Geometry G = make_geometry(nx, ny, nz, zc > 0 ? zc : slab_depth(nx, ny, nz, prec, solver), width);
     return nvec * align_up(NP * vec_t, 256) + (mixed ? 2 * align_up(NP * 8, 256) : 0) +
            align_up((size_t)G.ntiles * NPART * sizeof(double), 256);
 }
@@ -736,13 +782,13 @@ size_t q_bytes(int64_t nx, int64_t ny, int64_t nz, int prec)
 // Device bytes of a solve: one stencil-code array per volume, the state
 // vectors, partial sums and scalars of every right-hand side.
 size_t solve_bytes(const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs, int prec, int solver, int zc,
-                   bool store_q)
+                   int width, bool store_q)
 {
     size_t need = 4096;
     if (store_q)
         for (const JobSpec &j : jobs) need += q_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec);
     for (const VolSpec &v : vols) need += code_bytes(v.nx, v.ny, v.nz);
-    for (const JobSpec &j : jobs) need += job_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec, solver, zc);
+    for (const JobSpec &j : jobs) need += job_bytes(vols[j.vol].nx, vols[j.vol].ny, vols[j.vol].nz, prec, solver, zc, width);
     const size_t nj = jobs.size(), nv = vols.size();
     need += 3 * bnd_bytes(prec);  // one domain-face table per primary axis
     need += align_up(sizeof(Scalars) * nj, 256) + align_up(sizeof(uint32_t) * nj, 256) +
@@ -752,12 +798,13 @@ size_t solve_bytes(const std::vector<VolSpec> &vols, const std::vector<JobSpec> 
 
 int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, int dir,
               const uint8_t *d_code, Scalars *d_sc, uint32_t *d_counter, const void *d_bnd, Arena &A,
-              const fast_tau_params &P, int zc)
+              const fast_tau_params &P, int zc, int width)
 {
     const int prec = P.precision, solver = P.solver;
     const bool mixed = prec == FAST_PREC_MIXED;
     const size_t vec_t = (prec == FAST_PREC_F64) ? 8 : 4;
-    const Geometry G = make_geometry(nx, ny, nz, zc > 0 ? zc : slab_depth(nx, ny, nz, prec, solver));
+    if (width <= 0) width = tile_width(nx, ny, nz, solver);
+    const Geometry G = make_geometry(nx, ny, nz, zc > 0 ? zc : slab_depth(nx, ny, nz, prec, solver), width);
     const int64_t pitch = row_pitch(nx);
     const int64_t NP = pitch * ny * nz;
     const size_t vbytes = align_up((size_t)NP * vec_t, 256);
@@ -768,6 +815,7 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
     J.pitch = (int32_t)pitch;
     J.dir = dir;
     J.tiles_x = G.tx; J.tiles_y = G.ty; J.tiles_z = G.tz;
+    J.tile_w = width;
     J.zc = G.zc;
     J.ntiles = G.ntiles;
     J.code = d_code;
@@ -791,24 +839,24 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
     J.part = (double *)A.take((size_t)G.ntiles * NPART * sizeof(double));
     if (A.off > A.cap) return fail(FAST_CUDA_ERROR, "internal: device plan overflow");
     const int es = (int)vec_t;
-    int ts = tensor_map(&J.tm[TM_CODE], J.code, 1, nx, ny, nz, pitch);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_X], J.x, es, nx, ny, nz, pitch);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R], J.r[0], es, nx, ny, nz, pitch);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_P], J.p[0], es, nx, ny, nz, pitch);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_P + 1], J.p[1], es, nx, ny, nz, pitch);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_XI], J.x, es, nx, ny, nz, pitch, true);
-    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_RI], J.r[0], es, nx, ny, nz, pitch, true);
+    int ts = tensor_map(&J.tm[TM_CODE], J.code, 1, nx, ny, nz, pitch, width);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_X], J.x, es, nx, ny, nz, pitch, width);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R], J.r[0], es, nx, ny, nz, pitch, width);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_P], J.p[0], es, nx, ny, nz, pitch, width);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_P + 1], J.p[1], es, nx, ny, nz, pitch, width);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_XI], J.x, es, nx, ny, nz, pitch, width, true);
+    if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_RI], J.r[0], es, nx, ny, nz, pitch, width, true);
     if (ts == FAST_OK && (solver == FAST_SOLVER_BICGSTAB || fused)) {
-        ts = tensor_map(&J.tm[TM_R + 1], J.r[1], es, nx, ny, nz, pitch);
-        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R0], J.r0, es, nx, ny, nz, pitch);
-        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R0I], J.r0, es, nx, ny, nz, pitch, true);
-        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_V], J.v[0], es, nx, ny, nz, pitch);
-        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_V + 1], J.v[1], es, nx, ny, nz, pitch);
+        ts = tensor_map(&J.tm[TM_R + 1], J.r[1], es, nx, ny, nz, pitch, width);
+        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R0], J.r0, es, nx, ny, nz, pitch, width);
+        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_R0I], J.r0, es, nx, ny, nz, pitch, width, true);
+        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_V], J.v[0], es, nx, ny, nz, pitch, width);
+        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_V + 1], J.v[1], es, nx, ny, nz, pitch, width);
     }
     if (ts == FAST_OK && mixed) {
-        ts = tensor_map(&J.tm[TM_X64], J.x64[0], 8, nx, ny, nz, pitch);
-        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_X64 + 1], J.x64[1], 8, nx, ny, nz, pitch);
-        if (ts == FAST_OK && J.t) ts = tensor_map(&J.tm[TM_T], J.t, 4, nx, ny, nz, pitch);
+        ts = tensor_map(&J.tm[TM_X64], J.x64[0], 8, nx, ny, nz, pitch, width);
+        if (ts == FAST_OK) ts = tensor_map(&J.tm[TM_X64 + 1], J.x64[1], 8, nx, ny, nz, pitch, width);
+        if (ts == FAST_OK && J.t) ts = tensor_map(&J.tm[TM_T], J.t, 4, nx, ny, nz, pitch, width);
     }
     if (ts != FAST_OK) return ts;
     J.sc = d_sc;
@@ -869,9 +917,9 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     // Small CG solves run in one kernel (profiles and traces look at single
     // steps).
     bool resident = false;
-    const int zc = tuned_depth(prec, solver, dims, &resident);
+    const int zc = tuned_depth(prec, solver, dims, &resident), width = launch_width(dims, solver);
     resident = resident && !t_prof.on && env_int("FAST_TAU_TRACE", 0) < 2;
-    size_t need = solve_bytes(vols, jobs, prec, solver, zc, false);
+    size_t need = solve_bytes(vols, jobs, prec, solver, zc, width, false);
     if (resident) need += align_up(kResidentBlocks * kResidentSlotBytes, 256);
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
@@ -904,7 +952,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     Arena A;
     bool store_q = !mixed && solver == FAST_SOLVER_CG && !resident;
     if (store_q) {
-        const size_t more = solve_bytes(vols, jobs, prec, solver, zc, true);
+        const size_t more = solve_bytes(vols, jobs, prec, solver, zc, width, true);
         store_q = more <= avail && cudaMallocAsync((void **)&A.base, more, st) == cudaSuccess;
         if (store_q) need = more;
         else cudaGetLastError();
@@ -936,7 +984,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     for (int j = 0; j < nj; j++) {
         const VolSpec &V = vols[jobs[j].vol];
         const int bs = build_job(hj[j], hs[j], V.d_mask, V.nx, V.ny, V.nz, jobs[j].dir, d_code[jobs[j].vol], d_sc + j,
-                                 d_cnt + j, d_bnd[jobs[j].dir >> 1], A, P, zc);
+                                 d_cnt + j, d_bnd[jobs[j].dir >> 1], A, P, zc, width);
         if (bs != FAST_OK) {
             cudaFreeAsync(A.base, st);
             cudaStreamSynchronize(st);
@@ -980,16 +1028,16 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     Launch LC{d_jobs + nj, nv, 0, code_base, nullptr};
 
     int status = FAST_OK;
+    const StepLauncher fn = step_launcher(prec, width);
     launch_bnd(prec == FAST_PREC_F32, d_jobs, axis_job, naxes, st);
     launch_counted(FAST_K_CODE, st, [&] { launch_code(LC, st); });
     if (!mixed) {
-        void (*fn)(Step, const Launch &, cudaStream_t) = (prec == FAST_PREC_F64) ? dispatch_f64 : dispatch_f32;
         launch_counted(FAST_K_INIT, st, [&] { fn(solver == FAST_SOLVER_CG ? Step::INIT_CG : Step::INIT_BI, L, st); });
         std::vector<Step> steps;
         if (solver == FAST_SOLVER_CG) steps = {Step::CG1, store_q ? Step::CG2_Q : Step::CG2};
         else steps = {Step::BI_RESTART, Step::BI1, Step::BI2, Step::BI3};
         // (A context whose SMs are limited can refuse the cooperative launch.)
-        if (resident) status = iterate_resident(E, L, nj, d_sc, prec == FAST_PREC_F32, zc, P.max_iter, resident);
+        if (resident) status = iterate_resident(E, L, nj, d_sc, prec == FAST_PREC_F32, zc, width, P.max_iter, resident);
         if (!resident) status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
     } else {
         // FP32 iterations with in-graph FP64 residual replacement: the
@@ -998,7 +1046,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
         launch_counted(FAST_K_INIT64, st, [&] { launch_init64(L, st); });
         std::vector<Step> steps;
         steps = mixed_steps(solver, ff);
-        status = iterate(E, L, nj, d_sc, steps, dispatch_mixed, P.max_iter);
+        status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
     }
     if (status == FAST_OK)
         launch_counted(FAST_K_TAU, st, [&] { launch_tau(mixed ? (ff ? 2 : 3) : (prec == FAST_PREC_F32 ? 1 : 0), L, st); });

@@ -11,26 +11,35 @@ enum class Step {
     REPLACE_CG_FF, REPLACE_BI_FF  // the replacement with a float-float iterate (opt-in)
 };
 
-// Pure-precision solves: `f64` selects double, otherwise float (scalars in
-// the solve precision, as the reference's T).
-void launch_pure_f64(Step s, const Launch &L, cudaStream_t st);
-void launch_pure_f32(Step s, const Launch &L, cudaStream_t st);
-// CG of volumes whose blocks of zc planes all fit on the GPU at once: `iters`
-// iterations in one cooperative launch (tau_resident.cuh).
-// A right-hand side's planes per block at most, and the blocks of zc planes
-// that an SM holds (at most two, by their registers).
-constexpr int kResidentDepth = 24;
+// The solver kernels of a tile W columns wide (64, or 32 for CG alone).
+template <int W>
+struct Kernels {
+    // Pure-precision solves (scalars in the solve precision, as the
+    // reference's T).
+    static void pure_f64(Step s, const Launch &L, cudaStream_t st);
+    static void pure_f32(Step s, const Launch &L, cudaStream_t st);
+    // FP32 iterations of a MIXED solve (scalars in double); BI_K1/BI_K2 are
+    // the two-sweep BiCGSTAB steps, MIXED only.
+    static void mixed_inner(Step s, const Launch &L, cudaStream_t st);
+    // Residual replacement of a MIXED solve (a no-op launch unless the solve
+    // asked for one): FP64 iterate, or float-float with `ff`.
+    static void replace(bool bicg, bool ff, const Launch &L, cudaStream_t st);
+    // CG of volumes whose blocks of zc planes all fit on the GPU at once:
+    // `iters` iterations in one cooperative launch (tau_resident.cuh), and the
+    // blocks of zc planes that an SM holds (at most two, by their registers).
+    static cudaError_t resident_f64(const Launch &L, int zc, int iters, cudaStream_t st);
+    static cudaError_t resident_f32(const Launch &L, int zc, int iters, cudaStream_t st);
+    static int resident_per_sm(bool f32, int zc);
+    // Raise the dynamic shared-memory limit of every sweep kernel (once per
+    // device).
+    static cudaError_t configure_f64();
+    static cudaError_t configure_f32();
+    static cudaError_t configure_replace();
+};
+constexpr int kResidentDepth = 24;  // planes per block at most
 constexpr int kResidentBlocks = 2 * 152;
 constexpr size_t kResidentSlotBytes = 48;  // of a block, in Job::slots, zero before the first launch
-int resident_per_sm(bool f32, int zc);
-cudaError_t launch_resident_f64(const Launch &L, int zc, int iters, cudaStream_t st);
-cudaError_t launch_resident_f32(const Launch &L, int zc, int iters, cudaStream_t st);
-// FP32 iterations of a MIXED solve (scalars in double); BI_K1/BI_K2 are the
-// two-sweep BiCGSTAB steps, MIXED only.
-void launch_mixed_inner(Step s, const Launch &L, cudaStream_t st);
-// Residual replacement of a MIXED solve (a no-op launch unless the solve
-// asked for one): FP64 iterate, or float-float with `ff`.
-void launch_replace(bool bicg, bool ff, const Launch &L, cudaStream_t st);
+
 void launch_init64(const Launch &L, cudaStream_t st);
 // Adds the zero bytes of mask[0..n) (16-byte aligned) to *total.
 void launch_count_zero(const uint8_t *mask, uint64_t n, unsigned long long *total, cudaStream_t st);
@@ -43,9 +52,5 @@ void launch_bnd(bool f32, const Job *jobs, const int (&job)[3], int count, cudaS
 void launch_tau(int src, const Launch &L, cudaStream_t st);
 // n float-float pairs at src -> n doubles at dst (device).
 void launch_ff_to_double(const void *src, double *dst, int64_t n, cudaStream_t st);
-// Raise the dynamic shared-memory limit of every sweep kernel (once per device).
-cudaError_t configure_f64();
-cudaError_t configure_f32();
-cudaError_t configure_misc();
 
 }  // namespace ft

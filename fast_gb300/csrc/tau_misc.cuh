@@ -6,6 +6,7 @@
 #include "tau_sweep.cuh"
 
 namespace ft {
+inline namespace FT_TILES {
 
 // ===========================================================================
 // Arithmetic of the MIXED iterate x64, by its storage type XT (8 bytes per
@@ -399,12 +400,13 @@ __device__ __forceinline__ TileCoords tile_coords(const Job &J, int tid)
     const int tx_t = (int)(t.local % J.tiles_x);
     const int ty_t = (int)((t.local / J.tiles_x) % J.tiles_y);
     const int tz_t = (int)(t.local / ((int64_t)J.tiles_x * J.tiles_y));
-    t.x0 = tx_t * TX;
-    t.y0 = ty_t * TY;
+    const int w = J.tile_w, pairs = w / 2;  // these kernels take either tile
+    t.x0 = tx_t * w;
+    t.y0 = ty_t * (NTHREADS / pairs);
     t.z0 = tz_t * J.zc;
     t.z1 = min(t.z0 + J.zc, J.nz);
-    t.gx = t.x0 + 2 * (tid % TPR);
-    t.gy = t.y0 + tid / TPR;
+    t.gx = t.x0 + 2 * (tid % pairs);
+    t.gy = t.y0 + tid / pairs;
     t.v[0] = t.gx < J.nx && t.gy < J.ny;
     t.v[1] = t.gx + 1 < J.nx && t.gy < J.ny;
     return t;
@@ -624,4 +626,5 @@ __global__ void __launch_bounds__(NTHREADS) tau_kernel(Launch L, int use_x64)
     }
 }
 
+}  // namespace FT_TILES
 }  // namespace ft

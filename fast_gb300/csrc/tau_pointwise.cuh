@@ -22,6 +22,7 @@
 #include "tau_sweep.cuh"
 
 namespace ft {
+inline namespace FT_TILES {
 
 template <class Op, int U>
 __global__ void __launch_bounds__(NTHREADS) pointwise_kernel(Launch L)
@@ -212,4 +213,5 @@ struct PwBi3 {
     }
 };
 
+}  // namespace FT_TILES
 }  // namespace ft

@@ -31,6 +31,7 @@
 #include "tau_pointwise.cuh"
 
 namespace ft {
+inline namespace FT_TILES {
 
 constexpr int kBoxW = TX + 2;  // codes of a plane's box: columns -1 .. TX
 
@@ -389,4 +390,5 @@ cudaError_t launch_resident(const Launch &L, int zc, int iters, cudaStream_t st)
     return cudaLaunchKernelEx(&c, cg_resident_kernel<T>, L, iters);
 }
 
+}  // namespace FT_TILES
 }  // namespace ft

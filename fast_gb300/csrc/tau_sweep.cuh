@@ -26,6 +26,7 @@
 #include "tau_device.cuh"
 
 namespace ft {
+inline namespace FT_TILES {
 
 // ---------------------------------------------------------------------------
 // TMA / mbarrier primitives (inline PTX).
@@ -1733,4 +1734,5 @@ struct OpCGF {
     __device__ static void finish(Scalars &sc, const double (&t)[NV]) { cgf_finish(sc, t[0], t[1], t[2]); }
 };
 
+}  // namespace FT_TILES
 }  // namespace ft

@@ -10,10 +10,20 @@ namespace ft {
 // voxels is TPR threads; NTHREADS = 256 threads cover the TX * TY = 512
 // columns with one row each (a sweep with two rows per thread runs
 // NTHREADS / 2).
+//
+// The solver kernels are compiled for two tiles of 512 columns, 64 x 8 and 32 x
+// 16 (the kern_*_narrow.cu units set FAST_TAU_TX), in a namespace of their own
+// each; tile_width() picks one for a launch.
 #ifndef FAST_TAU_TX
 #define FAST_TAU_TX 64
 #endif
+#if FAST_TAU_TX == 64
+#define FT_TILES tiles64
+#else
+#define FT_TILES tiles32
+#endif
 constexpr int TX = FAST_TAU_TX;
+constexpr int kNarrowTX = 32;
 constexpr int LANES = 2;
 constexpr int TPR = TX / LANES;
 constexpr int TY = 256 / TPR;
@@ -106,6 +116,7 @@ struct Job {
     int32_t nx, ny, nz;
     int32_t dir;                 // 0..5
     int32_t tiles_x, tiles_y, tiles_z;
+    int32_t tile_w;              // columns of a tile in x (64 or 32)
     int32_t zc;                  // planes per block
     int64_t tile_base;           // first block index of this job in the launch
     int64_t ntiles;
