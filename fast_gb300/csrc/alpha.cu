@@ -56,6 +56,7 @@
 
 #include "ccl_faces.h"
 #include "fasttau.h"
+#include "fp_convert.h"
 #include "tau_errors.h"
 
 namespace {
@@ -274,22 +275,6 @@ __device__ __forceinline__ float triangle_area(const float3 &v0, const float3 &v
     return __fmul_rn(__fsqrt_rn(d), 0.5f);
 }
 
-// A sum of floats as an unevaluated pair (Knuth's two-sum): a thread adds a
-// few dozen areas of a brick, so the pair holds them to about 2^-47; the FP64
-// pipe is narrow enough that adding every area in double would cost more than
-// finding the triangles.
-struct PairSum {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float a, float ac = 0.f)
-    {
-        const float t = __fadd_rn(s, a);
-        const float b = __fsub_rn(t, s);
-        const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(a, b));
-        s = t;
-        c = __fadd_rn(c, __fadd_rn(e, ac));
-    }
-};
-
 // Full adder of three words: sum and carry.
 __device__ __forceinline__ uint64_t maj3(uint64_t a, uint64_t b, uint64_t c) { return (a & b) | (c & (a | b)); }
 
@@ -355,7 +340,10 @@ constexpr int QCAP = 4096;  // cells in the queue at once
 // one cell in seven of a porous volume is cut.  Queue positions come from a
 // block-wide scan and item q is done by thread q mod NT, so every sum has a
 // fixed order.  A cell's triangles are fans: a thread keeps the fan's first
-// and last vertex and makes one new vertex per triangle.
+// and last vertex and makes one new vertex per triangle.  Areas add in double
+// at every level: about two FP64 additions per cut cell beside some hundreds of
+// other instructions (512^3, seven fields, with the labelling: 1.88 ms, and
+// 1.87 with float pairs instead).
 //
 // Bound by instruction issue (384^3: 74 % of the slots busy, DRAM 6 %); most
 // of it is the cut cells' vertices and areas.  Against summing every cell's
@@ -374,7 +362,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
     __shared__ EdgeInfo s_edge[12];
     __shared__ uint16_t s_q[QCAP];  // c | row << 6
     __shared__ int s_warp[NT / 32];
-    __shared__ float2 s_red[NT / 32];
+    __shared__ double s_red[NT / 32];
     __shared__ uint32_t s_differ;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -511,7 +499,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
             at += w < warp ? t : 0;
             total += t;
         }
-        PairSum acc;
+        double acc = 0.0;
         for (int base = 0; base < total; base += QCAP) {
             while (cut && at < base + QCAP) {
                 const int c = __ffsll((long long)cut) - 1;
@@ -553,25 +541,22 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
                     }
                     const float3 v1 = v2;
                     v2 = vertex(C, s_t, s_edge, e);
-                    acc.add(triangle_area(v0, v1, v2));
+                    acc += ft::widen_f(triangle_area(v0, v1, v2));
                 }
             }
             __syncthreads();
         }
         // The brick's sum, in a fixed order.
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float s2 = __shfl_down_sync(0xffffffffu, acc.s, o), c2 = __shfl_down_sync(0xffffffffu, acc.c, o);
-            acc.add(s2, c2);
-        }
-        if (lane == 0) s_red[warp] = make_float2(acc.s, acc.c);
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if (lane == 0) s_red[warp] = acc;
         __syncthreads();
         if (tid < NF) {  // to every field of the group
             bool same = tid == f;
             if (tid > f) same = !((differ >> (bit0[tid] + f)) & 1u);
             if (same) {
                 double sum = 0.0;
-                for (int w = 0; w < NT / 32; w++) sum += (double)s_red[w].x + (double)s_red[w].y;
+                for (int w = 0; w < NT / 32; w++) sum += s_red[w];
                 A.partials[(size_t)tid * A.nblocks + blockIdx.x] = sum;
             }
         }

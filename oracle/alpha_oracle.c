@@ -138,24 +138,37 @@ static float grid_value(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz, 
 /* lerp(a, b, t) = a + t (b - a) (CUDA's helper_math form). */
 static float lerpf1(float a, float b, float t) { return a + t * (b - a); }
 
-/* Area of the isovalue surface of a 0/1 field (uint8, nonzero = 1). */
-double oracle_area_field(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz, float iso)
+/* (s, c) += v: what the sum s loses to rounding is kept in c. */
+static void add_exact(double *s, double *c, double v)
+{
+    const double t = *s + v, b = t - *s;
+    *c += (*s - (t - b)) + (v - b);
+    *s = t;
+}
+
+/* Area of the isovalue surface of a 0/1 field (uint8, nonzero = 1); low: what
+ * the sum of the areas has beyond a double, smallest: the smallest area of a
+ * triangle that is not 0. */
+double oracle_area_sum(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz, float iso, double *low, float *smallest)
 {
     int64_t k;
-    double total = 0.0;
-    double *per_z;
+    double total = 0.0, rest = 0.0;
+    double *per_z, *low_z;
+    float *min_z;
     const float vx = 1.0f / (float)nx, vy = 1.0f / (float)ny, vz = 1.0f / (float)nz;
     if (!g_ready) make_table();
     per_z = (double *)calloc((size_t)nz, sizeof(double));
+    low_z = (double *)calloc((size_t)nz, sizeof(double));
+    min_z = (float *)calloc((size_t)nz, sizeof(float));
 #pragma omp parallel for schedule(dynamic, 1)
     for (k = 0; k < nz; k++) {
         int64_t i, j;
-        double zsum = 0.0;
+        double zsum = 0.0, zlow = 0.0;
+        float zmin = INFINITY;
         for (j = 0; j < ny; j++) {
             for (i = 0; i < nx; i++) {
                 float val[8], P[8][3];
                 int c, cube = 0, t;
-                double cell = 0.0;
                 const float px = vx * (float)i, py = vy * (float)j, pz = vz * (float)k;
                 for (c = 0; c < 8; c++) {
                     val[c] = grid_value(fld, nx, ny, nz, i + CX[c], j + CY[c], k + CZ[c]);
@@ -165,7 +178,7 @@ double oracle_area_field(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz,
                     P[c][2] = CZ[c] ? pz + vz : pz;
                 }
                 for (t = 0; t < g_ntri[cube]; t++) {
-                    float V[3][3], d1[3], d2[3], cr[3];
+                    float V[3][3], d1[3], d2[3], cr[3], area;
                     int q, ax;
                     for (q = 0; q < 3; q++) {
                         const int e = g_tri[cube][3 * t + q];
@@ -184,16 +197,34 @@ double oracle_area_field(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz,
                     cr[0] = d1[1] * d2[2] - d1[2] * d2[1];
                     cr[1] = d1[2] * d2[0] - d1[0] * d2[2];
                     cr[2] = d1[0] * d2[1] - d1[1] * d2[0];
-                    cell += (double)(sqrtf(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]) * 0.5f);
+                    area = sqrtf(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]) * 0.5f;
+                    add_exact(&zsum, &zlow, (double)area);
+                    if (area > 0.0f && area < zmin) zmin = area;
                 }
-                zsum += cell;
             }
         }
         per_z[k] = zsum;
+        low_z[k] = zlow;
+        min_z[k] = zmin;
     }
-    for (k = 0; k < nz; k++) total += per_z[k];
+    *smallest = INFINITY;
+    for (k = 0; k < nz; k++) {
+        add_exact(&total, &rest, per_z[k]);
+        rest += low_z[k];
+        if (min_z[k] < *smallest) *smallest = min_z[k];
+    }
     free(per_z);
+    free(low_z);
+    free(min_z);
+    *low = rest;
     return total;
+}
+
+double oracle_area_field(const uint8_t *fld, int64_t nx, int64_t ny, int64_t nz, float iso)
+{
+    double low;
+    float smallest;
+    return oracle_area_sum(fld, nx, ny, nz, iso, &low, &smallest);
 }
 
 /* Triangle count of a corner pattern (for table checks). */

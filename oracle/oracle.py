@@ -79,6 +79,8 @@ def lib():
             L.oracle_ccl_boundary.argtypes = [P, i64, i64, i64, C.c_uint32, P]
             L.oracle_area_field.argtypes = [P, i64, i64, i64, f32]
             L.oracle_area_field.restype = f64
+            L.oracle_area_sum.argtypes = [P, i64, i64, i64, f32, C.POINTER(f64), C.POINTER(f32)]
+            L.oracle_area_sum.restype = f64
             L.oracle_mc_ntri.argtypes = [i32]
             L.oracle_mc_ntri.restype = i32
             _lib = L
@@ -240,6 +242,16 @@ def area_field(field, iso=0.5) -> float:
     f = np.ascontiguousarray(field, dtype=np.uint8)
     nx, ny, nz = _dims(f)
     return float(lib().oracle_area_field(_ptr(f), nx, ny, nz, float(iso)))
+
+
+def area_sum(mask, iso=0.5):
+    """(area, low, smallest) of a 0/255 mask: the triangles' areas added
+    exactly are area + low; smallest is the smallest that is not 0."""
+    f = np.ascontiguousarray(np.asarray(mask) != 0, dtype=np.uint8)
+    nx, ny, nz = _dims(f)
+    low, smallest = C.c_double(), C.c_float()
+    area = lib().oracle_area_sum(_ptr(f), nx, ny, nz, float(iso), C.byref(low), C.byref(smallest))
+    return float(area), low.value, smallest.value
 
 
 def reactive_area(mask, iso=0.5) -> float:
