@@ -887,6 +887,9 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
     // test builds: FAST_TAU_TEST_WITHHOLD = 1 + direction arms the withheld
     // tile load of that direction's first sweep
     S.test_withhold = env_int("FAST_TAU_TEST_WITHHOLD", 0) == dir + 1 ? 1 : 0;
+    // FAST_TAU_TEST_OOB = 1 + direction: a bounds check of that direction's
+    // one-kernel CG that fails
+    S.test_oob = env_int("FAST_TAU_TEST_OOB", 0) == dir + 1 ? 1 : 0;
 #endif
     // MIXED BiCGSTAB: no update is pending before the first replacement.
     S.alpha = 0.0;

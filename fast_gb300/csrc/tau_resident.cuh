@@ -200,6 +200,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
         p = cg_direction<T>(p, beta, r, inv);
     };
 
+#if FAST_TAU_TEST_HOOKS
+    // an index outside an empty array: the check records it, nothing is accessed
+    if (s_sc.test_oob && tid == 0 && local == J.ntiles - 1) (void)ft_in(J, 0, 0, 0, OOB_SWEEP_STORE);
+#endif
     ulonglong2 *slots = (ulonglong2 *)J.slots;
     bool ok = true;
     for (int it = 0; it < iters; it++) {
@@ -341,17 +345,18 @@ __global__ void __launch_bounds__(NTHREADS, 2) cg_resident_kernel(Launch L, int 
     }
     // For the next launch: p where its first iteration looks for it, and the
     // scalars (by one block; the others have their copies).  The state only
-    // replaces RUNNING: a block that gave up may have marked a FAULT.
+    // replaces RUNNING: a block that gave up may have marked a FAULT.  The
+    // bounds checks' record is the blocks' own (ft_in).
     T *p_out = (T *)J.p[(int)(s_sc.iter & 1)];
     for (int k = 0; k < zn && s_sc.state == RUNNING; k++) {
         const int64_t i = i_own + plane * k;
         const Pair<T> p = *reinterpret_cast<const Pair<T> *>(&P[k + 1][ly + 1][2 * lp + 2]);
         if (v0 && ft_in(J, i, i + 1, total, OOB_SWEEP_STORE)) store2<T>(p_out, i, p.a, p.b, true, v1);
     }
-    constexpr int kState = (int)(offsetof(Scalars, state) / 4);
+    constexpr int kState = (int)(offsetof(Scalars, state) / 4), kOob = (int)(offsetof(Scalars, oob) / 4);
     if (local == 0 && tid < W) {
         if (tid == kState) atomicCAS(&J.sc->state, (int32_t)RUNNING, s_sc.state);
-        else reinterpret_cast<uint32_t *>(J.sc)[tid] = reinterpret_cast<const uint32_t *>(&s_sc)[tid];
+        else if (tid != kOob) reinterpret_cast<uint32_t *>(J.sc)[tid] = reinterpret_cast<const uint32_t *>(&s_sc)[tid];
     }
 }
 

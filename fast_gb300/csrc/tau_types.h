@@ -100,7 +100,7 @@ struct Scalars {
     int32_t cg_fused;       // 1: MIXED CG runs as one sweep per iteration (OpCGF)
     int32_t oob;            // bounds-check builds: first failing access site (0 = none)
     int32_t test_withhold;  // test-hook builds: withhold one tile load of the next sweep (see tau_sweep.cuh)
-    int32_t pad_hook;
+    int32_t test_oob;       // test-hook builds: one failing bounds check in the resident kernel (tau_resident.cuh)
     // reductions for tau and porosity
     double flux_sum;    // sum over voxels of the tau flux term
     uint64_t pores;     // number of zero (pore) voxels
