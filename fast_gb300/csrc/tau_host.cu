@@ -887,9 +887,11 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
     // test builds: FAST_TAU_TEST_WITHHOLD = 1 + direction arms the withheld
     // tile load of that direction's first sweep
     S.test_withhold = env_int("FAST_TAU_TEST_WITHHOLD", 0) == dir + 1 ? 1 : 0;
-    // FAST_TAU_TEST_OOB = 1 + direction: a bounds check of that direction's
-    // one-kernel CG that fails
-    S.test_oob = env_int("FAST_TAU_TEST_OOB", 0) == dir + 1 ? 1 : 0;
+    // in that direction's one-kernel CG, FAST_TAU_TEST_OOB = 1 + direction: a
+    // bounds check that fails; FAST_TAU_TEST_SILENT: a partial sum that does
+    // not come
+    if (env_int("FAST_TAU_TEST_OOB", 0) == dir + 1) S.test_resident = 1;
+    if (env_int("FAST_TAU_TEST_SILENT", 0) == dir + 1) S.test_resident = 2;
 #endif
     // MIXED BiCGSTAB: no update is pending before the first replacement.
     S.alpha = 0.0;
@@ -1125,7 +1127,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
             fail(R.status, "right-hand side %d (direction %d): %s after %llu iterations (|r|/|b| = %.3e)", j,
                  jobs[j].dir,
                  R.status == FAST_DIVERGED  ? "solver diverged"
-                 : R.status == FAST_TIMEOUT ? "a bounded device-side wait for tile loads ran out"
+                 : R.status == FAST_TIMEOUT ? "a bounded device-side wait ran out"
                                             : "solver did not converge",
                  (unsigned long long)R.iterations, R.rel_residual);
         }

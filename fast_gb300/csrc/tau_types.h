@@ -50,7 +50,7 @@ enum SolveState : int32_t {
     MAXITER = 2,
     DIVERGED = 3,
     ZERO_RHS = 4,
-    FAULT = 6,     // a bounded device-side wait ran out (tile loads did not arrive)
+    FAULT = 6,     // a bounded device-side wait ran out (tile loads or another block's partial sum did not arrive)
 };
 
 // Tensor maps of a job's arrays (TMA descriptors), by array.
@@ -100,7 +100,8 @@ struct Scalars {
     int32_t cg_fused;       // 1: MIXED CG runs as one sweep per iteration (OpCGF)
     int32_t oob;            // bounds-check builds: first failing access site (0 = none)
     int32_t test_withhold;  // test-hook builds: withhold one tile load of the next sweep (see tau_sweep.cuh)
-    int32_t test_oob;       // test-hook builds: one failing bounds check in the resident kernel (tau_resident.cuh)
+    int32_t test_resident;  // test-hook builds, resident kernel (tau_resident.cuh): 1 = a failing bounds check,
+                            // 2 = a block that does not publish one of its partial sums
     // reductions for tau and porosity
     double flux_sum;    // sum over voxels of the tau flux term
     uint64_t pores;     // number of zero (pore) voxels

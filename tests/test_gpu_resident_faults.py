@@ -1,7 +1,10 @@
-"""What goes wrong inside the one-kernel CG comes out of the call: a failed
-bounds check of its blocks (a bounds-checked build with test hooks, where one
-block checks an index of an empty array, so nothing is accessed) fails the
-call as one in the sweeps does, and the call after it is as before."""
+"""What goes wrong inside the one-kernel CG comes out of the call, in builds
+with test hooks: a failed bounds check of its blocks (one checks an index of
+an empty array, so nothing is accessed) fails the call as one in the sweeps
+does; a block whose partial sum does not come (it publishes none in the third
+iteration) makes the blocks that wait for it give up after the time limit, 50
+ms here, and the call returns FAST_TIMEOUT.  Other right-hand sides of the
+launch and the call after it are as before."""
 import json
 import os
 import subprocess
@@ -14,7 +17,7 @@ ROOT = os.path.dirname(HERE)
 
 pytestmark = pytest.mark.gpu
 
-OK, CUDA_ERROR = 0, 6
+OK, CUDA_ERROR, TIMEOUT = 0, 6, 7
 
 PRELUDE = r"""
 import ctypes as C, json, os, sys
@@ -76,4 +79,23 @@ def test_bounds_record_survives(gpu, tmp_path):
         assert before[2] < sweeps[2]  # one kernel ran the iterations
         assert armed[0] == CUDA_ERROR and "bounds check" in armed[3]
         assert [r[0] for r in armed[1]] == [OK, CUDA_ERROR, OK] and armed[1][1][1] == 0.0
+        assert armed[1][0] == before[1][0] and armed[1][2] == before[1][2]
+
+
+SILENT = r"""
+out = {}
+for prec in (ft.Precision.F64, ft.Precision.F32):
+    out[prec.name] = [solve([0, 2, 4], prec), solve([0, 2, 4], prec, "FAST_TAU_TEST_SILENT", 3),
+                      solve([0, 2, 4], prec), solve([0, 2, 4], prec, profile=True)]
+print(json.dumps(out))
+"""
+
+
+def test_missing_partial_sum_times_out(gpu, tmp_path):
+    lib = _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1 -DFAST_TAU_WAIT_LIMIT_NS=50000000ull")
+    for before, armed, after, sweeps in _run(lib, SILENT).values():
+        assert before[0] == after[0] == OK and before[1] == after[1]
+        assert before[2] < sweeps[2]  # one kernel ran the iterations
+        assert armed[0] == TIMEOUT and "wait ran out" in armed[3] and "tile" not in armed[3]
+        assert [r[0] for r in armed[1]] == [OK, TIMEOUT, OK] and armed[1][1][1] == 0.0
         assert armed[1][0] == before[1][0] and armed[1][2] == before[1][2]
