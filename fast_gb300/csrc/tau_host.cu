@@ -431,7 +431,12 @@ int iterate_resident(Engine &E, const Launch &L, int njobs, Scalars *d_sc, bool 
     const uint64_t max_launches = max_iter / kIters + 4;
     int status = FAST_OK;
     for (uint64_t k = 0; k < max_launches; k++) {
+#if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
+        // test builds: FAST_TAU_TEST_REFUSE=1 stands in for a refused launch
+        cerr = env_int("FAST_TAU_TEST_REFUSE", 0) ? cudaErrorCooperativeLaunchTooLarge : launch(L, zc, kIters, st);
+#else
         cerr = launch(L, zc, kIters, st);
+#endif
         if (cerr != cudaSuccess && k == 0) {
             cudaGetLastError();
             launched = false;
@@ -593,7 +598,22 @@ constexpr DepthModel kDepthModel[3] = {
     {4, 7.9, 5.3, 0.75, {1.16, 1.44, 1.80, 2.18}},               // F32
     {6, 11.5, 0.0, 4.1, {1.31, 1.54, 1.85, 2.06, 2.37, 2.37}},   // MIXED
 };
-constexpr int kSms = 152;
+constexpr int kSms = 152;  // of the GPU that the models were fitted on
+
+// The SMs that a launch of this process has (kSms without a GPU).
+int device_sms()
+{
+    int dev = 0, sms = 0;
+#if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
+    sms = env_int("FAST_TAU_TEST_SMS", 0);  // test builds: a GPU with so many SMs
+    if (sms > 0) return sms;
+#endif
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+        return sms;
+    cudaGetLastError();
+    return kSms;
+}
 
 double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims, int width, int d)
 {
@@ -644,7 +664,8 @@ int modelled_depth(int prec, const std::vector<const int64_t *> &dims, int width
 }
 
 // CG in one kernel (tau_resident.cuh): the depth for right-hand sides with
-// dimensions dims, 0 where their blocks do not all fit on the GPU or the model
+// dimensions dims, 0 where their blocks do not all fit on the GPU (its SMs, not
+// the model's) or the model
 // puts the sweeps within 5 %.  us per iteration with b blocks on the fullest
 // SM: base[b] + d plane[b], fits to 18 launches (28 x 24 x 20 to 100^3, 1 to 12
 // right-hand sides) at all their depths.  Steps -> best resident depth: F64 CG
@@ -664,6 +685,7 @@ int resident_depth(int prec, const std::vector<const int64_t *> &dims, int width
     if (prec == FAST_PREC_MIXED) return 0;
     const bool f32 = prec == FAST_PREC_F32;
     const ResidentModel &M = kResidentModel[f32];
+    const int sms = device_sms();
     int64_t nz = 1;
     for (const int64_t *v : dims) nz = std::max(nz, v[2]);
     int64_t depth = 0;
@@ -673,8 +695,8 @@ int resident_depth(int prec, const std::vector<const int64_t *> &dims, int width
         d = (nz + n - 1) / n;  // even slabs
         int64_t blocks = 0;
         for (const int64_t *v : dims) blocks += make_geometry(v[0], v[1], v[2], (int)d, width).ntiles;
-        if (blocks > kResidentBlocks) break;
-        const int b = blocks > kSms;
+        if (blocks > std::min(kResidentBlocks, 2 * sms)) break;
+        const int b = blocks > sms;
         if ((width == TX ? Kernels<TX>::resident_per_sm : Kernels<kNarrowTX>::resident_per_sm)(f32, (int)d) < b + 1) continue;
         const double us = M.base[b] + (double)d * M.plane[b];
         if (us < best) {
@@ -903,8 +925,9 @@ int build_job(Job &J, Scalars &S, const uint8_t *d_mask, int64_t nx, int64_t ny,
 // `vols`) together: one launch per solver step covers all of them, each
 // block working for one (job, tile); converged right-hand sides drop out of
 // the launches at block entry.  conc_out: only with a single job.
+// one_kernel = false: small CG solves run the sweeps, at the same depth.
 int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<JobSpec> &jobs,
-               const fast_tau_params &P, fast_tau_result *res, void *conc_out)
+               const fast_tau_params &P, fast_tau_result *res, void *conc_out, bool one_kernel = true)
 {
     cudaStream_t st = E.stream;
     t_prof.reset((P.flags & FAST_FLAG_PROFILE) != 0);
@@ -923,7 +946,7 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
     // steps).
     bool resident = false;
     const int zc = tuned_depth(prec, solver, dims, &resident), width = launch_width(dims, solver);
-    resident = resident && !t_prof.on && env_int("FAST_TAU_TRACE", 0) < 2;
+    resident = resident && one_kernel && !t_prof.on && env_int("FAST_TAU_TRACE", 0) < 2;
     size_t need = solve_bytes(vols, jobs, prec, solver, zc, width, false);
     if (resident) need += align_up(kResidentBlocks * kResidentSlotBytes, 256);
     size_t free_b = 0, total_b = 0;
@@ -1041,9 +1064,19 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
         std::vector<Step> steps;
         if (solver == FAST_SOLVER_CG) steps = {Step::CG1, store_q ? Step::CG2_Q : Step::CG2};
         else steps = {Step::BI_RESTART, Step::BI1, Step::BI2, Step::BI3};
-        // (A context whose SMs are limited can refuse the cooperative launch.)
-        if (resident) status = iterate_resident(E, L, nj, d_sc, prec == FAST_PREC_F32, zc, width, P.max_iter, resident);
-        if (!resident) status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
+        if (resident) {
+            bool launched = true;
+            status = iterate_resident(E, L, nj, d_sc, prec == FAST_PREC_F32, zc, width, P.max_iter, launched);
+            if (!launched) {
+                // A context whose share of the SMs is limited can refuse the
+                // cooperative launch: plan again for the sweeps, with q.
+                CU(cudaFreeAsync(A.base, st));
+                CU(cudaStreamSynchronize(st));
+                return solve_jobs(E, vols, jobs, P, res, conc_out, false);
+            }
+        } else {
+            status = iterate(E, L, nj, d_sc, steps, fn, P.max_iter);
+        }
     } else {
         // FP32 iterations with in-graph FP64 residual replacement: the
         // replacement slot leads every iteration and is a no-op launch unless

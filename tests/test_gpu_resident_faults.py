@@ -4,7 +4,9 @@ an empty array, so nothing is accessed) fails the call as one in the sweeps
 does; a block whose partial sum does not come (it publishes none in the third
 iteration) makes the blocks that wait for it give up after the time limit, 50
 ms here, and the call returns FAST_TIMEOUT.  Other right-hand sides of the
-launch and the call after it are as before."""
+launch and the call after it are as before.  Where the cooperative launch is
+refused, or the GPU has too few SMs for the blocks, the sweeps run instead:
+the same bits, with the stored product that sweeps have."""
 import json
 import os
 import subprocess
@@ -99,3 +101,38 @@ def test_missing_partial_sum_times_out(gpu, tmp_path):
         assert armed[0] == TIMEOUT and "wait ran out" in armed[3] and "tile" not in armed[3]
         assert [r[0] for r in armed[1]] == [OK, TIMEOUT, OK] and armed[1][1][1] == 0.0
         assert armed[1][0] == before[1][0] and armed[1][2] == before[1][2]
+
+
+REFUSED = r"""
+def used_high(reset=False):  # bytes at most in use from the device's default memory pool
+    cu, dev, pool, v = C.CDLL("libcuda.so.1"), C.c_int(), C.c_void_p(), C.c_uint64(0)
+    assert cu.cuInit(0) == 0 and cu.cuDeviceGet(C.byref(dev), 0) == 0
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), dev) == 0
+    if reset:
+        assert cu.cuMemPoolSetAttribute(pool, 8, C.byref(v)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    assert cu.cuMemPoolGetAttribute(pool, 8, C.byref(v)) == 0
+    return v.value
+
+out = {}
+for prec, n in ((ft.Precision.F64, 80), (ft.Precision.F32, 100)):
+    m = volumes.spheres((n, n, n), seed=8, r_min=3.0, solid_fraction=0.5)
+    nz, ny, nx = m.shape
+    rows = []
+    for kw in ({}, {"hook": "FAST_TAU_TEST_REFUSE", "arm": 1}, {"hook": "FAST_TAU_TEST_SMS", "arm": 8},
+               {"profile": True}, {}):
+        used_high(reset=True)
+        rows.append(solve([2], prec, **kw) + [used_high()])
+    out[prec.name] = rows
+print(json.dumps(out))
+"""
+
+
+def test_refused_launch_runs_the_sweeps(gpu, tmp_path):
+    lib = _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1")
+    for kernel, refused, few_sms, sweeps, after in _run(lib, REFUSED).values():
+        assert all(r[0] == OK for r in (kernel, refused, few_sms, sweeps, after))
+        assert kernel[1] == refused[1] == after[1]
+        assert refused[1] == sweeps[1]
+        assert abs(few_sms[1][0][1] - kernel[1][0][1]) <= 1e-4 * kernel[1][0][1]  # another depth: other sums
+        assert kernel[2] == after[2] < min(refused[2], few_sms[2], sweeps[2])
+        assert refused[4] == sweeps[4] >= kernel[4] + (2 << 20)  # q: 4 MB
