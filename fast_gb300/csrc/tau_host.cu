@@ -56,7 +56,14 @@ int ft_fail(int status, const char *fmt, ...)
     return status;
 }
 
-void ft_clear_error() { g_last_error.clear(); }
+// At the start of a call: neither its message nor a CUDA error that an earlier
+// call of the thread met and reported (an allocation that did not fit) is this
+// call's.
+void ft_clear_error()
+{
+    g_last_error.clear();
+    cudaGetLastError();
+}
 
 void ft_retain_pool_memory(int device)
 {
@@ -1306,7 +1313,7 @@ FAST_API int fast_tau_solve_dirs_device(const uint8_t *d_mask, int64_t nx, int64
                                         const fast_tau_params *p, int32_t ndirs, const int32_t *dirs,
                                         fast_tau_result *results, void *stream)
 {
-    g_last_error.clear();
+    ft_clear_error();
     int st = check_args(d_mask, nx, ny, nz, p, ndirs, dirs);
     if (st != FAST_OK) return st;
     if (!results) return fail(FAST_BAD_ARG, "results is NULL");
@@ -1323,7 +1330,7 @@ FAST_API int fast_tau_solve_dirs_device(const uint8_t *d_mask, int64_t nx, int64
 FAST_API int fast_tau_solve_batch_device(const fast_tau_volume *vols, int32_t nvols, const fast_tau_params *p,
                                          fast_tau_result *results, void *stream)
 {
-    g_last_error.clear();
+    ft_clear_error();
     int st = check_batch(vols, nvols, p, results);
     if (st != FAST_OK) return st;
     Engine *E = nullptr;
@@ -1345,7 +1352,7 @@ FAST_API int fast_tau_solve_batch_device(const fast_tau_volume *vols, int32_t nv
 FAST_API int fast_tau_solve_batch(const fast_tau_volume *vols, int32_t nvols, const fast_tau_params *p,
                                   fast_tau_result *results)
 {
-    g_last_error.clear();
+    ft_clear_error();
     int st = check_batch(vols, nvols, p, results);
     if (st != FAST_OK) return st;
     Engine *E = nullptr;
@@ -1376,7 +1383,7 @@ FAST_API int fast_tau_solve_batch(const fast_tau_volume *vols, int32_t nvols, co
 static int solve_host(const uint8_t *mask, int64_t nx, int64_t ny, int64_t nz, const fast_tau_params *p,
                       int32_t ndirs, const int32_t *dirs, fast_tau_result *results, void *conc_out)
 {
-    g_last_error.clear();
+    ft_clear_error();
     int st = check_args(mask, nx, ny, nz, p, ndirs, dirs);
     if (st != FAST_OK) return st;
     Engine *E = nullptr;
@@ -1422,7 +1429,7 @@ FAST_API int fast_tau_solve(const uint8_t *mask, int64_t nx, int64_t ny, int64_t
 FAST_API int fast_porosity(const uint8_t *mask, int64_t nx, int64_t ny, int64_t nz, double *porosity,
                            uint64_t *pore_count)
 {
-    g_last_error.clear();
+    ft_clear_error();
     if (!mask) return fail(FAST_NO_HOST_DATA, "mask must be allocated");
     if (nx <= 0 || ny <= 0 || nz <= 0) return fail(FAST_BAD_ARG, "dimensions must be positive");
     Engine *E = nullptr;
