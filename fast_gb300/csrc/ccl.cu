@@ -602,8 +602,10 @@ int check_dims(int64_t nx, int64_t ny, int64_t nz)
 
 // Geometry and scratch plan of a labelling; `base` null: sizes only.
 // Returns the scratch bytes: 8 + 2 x slots + 4 per 64-voxel word, one bit per
-// voxel and one count per chunk (1.2 bytes per voxel of a wide volume).
-size_t plan(Ccl &A, char *base)
+// voxel and one count per chunk (1.2 bytes per voxel of a wide volume), and
+// with `copy` (the mask lies in the labels' memory, which pass 1 writes while
+// other blocks still read the mask) the mask.
+size_t plan(Ccl &A, char *base, bool copy)
 {
     const size_t words = (size_t)A.wx * A.ny * A.nz;
     const size_t n = (size_t)A.nx * A.ny * A.nz;
@@ -621,6 +623,7 @@ size_t plan(Ccl &A, char *base)
     A.cnt = (uint32_t *)take((nchunks + 1) * 4);
     A.root_bits = (uint32_t *)take(nchunks * (kChunk / 32) * 4);
     A.zero_words = (int64_t)((off - zero_off) / 4);
+    if (copy) A.mask = (uint8_t *)take(n);
     return off;
 }
 
@@ -687,12 +690,20 @@ int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint
     A.bg = bg;
     A.mask = d_mask;
     A.par = d_labels;
-    const size_t need = plan(A, nullptr);
+    const size_t n = (size_t)(nx * ny * nz);
+    const uintptr_t m0 = (uintptr_t)d_mask, l0 = (uintptr_t)d_labels;
+    const bool copy = m0 < l0 + 4 * n && l0 < m0 + n;
+    const size_t need = plan(A, nullptr, copy);
     char *scratch = nullptr;
     cudaError_t e = cudaMallocAsync((void **)&scratch, need, st);
     if (e != cudaSuccess) return ft_fail(FAST_NOMEM, "labelling scratch: %s", cudaGetErrorString(e));
-    plan(A, scratch);
-    int s = label_device(A, num_labels, st);
+    plan(A, scratch, copy);
+    int s = FAST_OK;
+    if (copy) {
+        e = cudaMemcpyAsync((void *)A.mask, d_mask, n, cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) s = ft_fail(FAST_CUDA_ERROR, "labelling mask: %s", cudaGetErrorString(e));
+    }
+    if (s == FAST_OK) s = label_device(A, num_labels, st);
     cudaFreeAsync(scratch, st);
     if (s == FAST_OK && boundary) {
         if (boundary_cap < (uint64_t)7 * *num_labels)
