@@ -40,8 +40,14 @@
 // are inside a brick, where shared memory answers in a few dozen cycles, and
 // about one in five is left for pass 2.  768 x 700 x 720 spheres: 5.92 ms of
 // kernels -> 1.30 (pass 1 0.57, issue bound; pass 2 0.25; pass 6 0.37, 4.2 TB/s
-// of labels); 1024^3 17.3 -> 3.7 ms.  Scratch is 1.2 bytes per voxel (4.1
-// with a parent per voxel) for volumes at least 64 voxels wide.
+// of labels); 1024^3 17.3 -> 3.7 ms.  Scratch is 76 bytes per 64-voxel word of
+// a row plus a bit per voxel: 1.3 bytes per voxel at multiples of 64, at most
+// 2.5 above 64 (a parent per voxel: 4.1).  A row of less than 64 voxels keeps
+// 12 + 2 ceil(nx / 2) bytes: 1.3 per voxel at 63, 2.0 at 14, 5.5 and 7.1 at 3
+// and 2.  A volume one voxel wide is labelled as its y-z plane (the same
+// indices and neighbours): 1 x 6000 x 5000 takes 1.1 ms instead of 4.3, and 1.3
+// bytes per voxel instead of 14.  30 M voxels 2, 3, 8 and 33 wide: 2.1, 1.6,
+// 0.93 and 0.45 ms (5.8, 4.6, 3.0 and 1.5 with a parent per voxel).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -680,13 +686,13 @@ int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint
     CK(cudaGetDevice(&dev));
     ft_retain_pool_memory(dev);
     Ccl A = {};
-    A.nx = (int)nx;
-    A.ny = (int)ny;
-    A.nz = (int)nz;
-    A.wx = (int)((nx + 63) / 64);
-    A.by = (int)((ny + RY - 1) / RY);
-    A.bz = (int)((nz + RZ - 1) / RZ);
-    A.slots = nx >= 64 ? kSlots : (int)((nx + 1) / 2);
+    A.nx = (int)(nx > 1 ? nx : ny);
+    A.ny = (int)(nx > 1 ? ny : nz);
+    A.nz = (int)(nx > 1 ? nz : 1);
+    A.wx = (A.nx + 63) / 64;
+    A.by = (A.ny + RY - 1) / RY;
+    A.bz = (A.nz + RZ - 1) / RZ;
+    A.slots = A.nx >= 64 ? kSlots : (A.nx + 1) / 2;
     A.bg = bg;
     A.mask = d_mask;
     A.par = d_labels;
