@@ -336,22 +336,44 @@ int rebuild(Ctx &C)
     return FAST_OK;
 }
 
-int launch_chunk(Ctx &C)
+void sync_groups(Ctx &C)
 {
-    const int b = (C.head + C.inflight) & 1;
-    // The groups share nothing but the slot array (one entry per solve): their
-    // chunks run side by side, behind everything queued on the context's stream
-    // and before anything queued on it from here on.  One after the other, each
-    // group's sweeps left the GPU part idle in their last wave of blocks: a
-    // burst of 24 requests of both solvers took 157 ms, side by side 138 ms
-    // (132 with the narrow tiles' group).
+    for (Group &G : C.groups)
+        if (G.st) cudaStreamSynchronize(G.st);
+}
+
+// The groups share nothing but the slot array (one entry per solve): their
+// chunks run side by side, behind everything queued on the context's stream
+// and before anything queued on it from here on.  One after the other, each
+// group's sweeps left the GPU part idle in their last wave of blocks: a
+// burst of 24 requests of both solvers took 157 ms, side by side 138 ms
+// (132 with the narrow tiles' group).
+int fork_groups(Ctx &C)
+{
     SV(cudaEventRecord(C.ev_fork, C.st));
     for (Group &G : C.groups) {
         if (!G.exec) continue;
         SV(cudaStreamWaitEvent(G.st, C.ev_fork, 0));
         SV(cudaGraphLaunch(G.exec, G.st));
+#if defined(FAST_TAU_TEST_HOOKS) && FAST_TAU_TEST_HOOKS
+        // test builds: FAST_TAU_TEST_FORK=1 stands in for a failing call here
+        if (env_int("FAST_TAU_TEST_FORK", 0)) return ft_fail(FAST_CUDA_ERROR, "FAST_TAU_TEST_FORK");
+#endif
         SV(cudaEventRecord(G.done, G.st));
         SV(cudaStreamWaitEvent(C.st, G.done, 0));
+    }
+    return FAST_OK;
+}
+
+int launch_chunk(Ctx &C)
+{
+    const int b = (C.head + C.inflight) & 1;
+    const int s = fork_groups(C);
+    if (s != FAST_OK) {
+        // A graph that was launched may not be joined: nothing may be queued
+        // on the context's stream, or freed, while it runs.
+        sync_groups(C);
+        return s;
     }
     int hi = 0;
     for (const Active &A : C.active) hi = std::max(hi, A.slot + 1);
@@ -404,6 +426,7 @@ void destroy(Ctx *C)
 {
     if (!C) return;
     if (C->st) cudaStreamSynchronize(C->st);
+    sync_groups(*C);
     for (Active &A : C->active) cudaFreeAsync(A.arena, C->st);
     for (Group &G : C->groups) {
         if (G.exec) cudaGraphExecDestroy(G.exec);
