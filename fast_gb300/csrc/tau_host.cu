@@ -722,15 +722,21 @@ int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims, 
     const int env = env_int("FAST_TAU_ZC", 0);
     if (env > 0) return env;
     int64_t W = 0;
+    double planes = 0.0;
     for (const int64_t *d : dims) {
         const Geometry G = make_geometry(d[0], d[1], d[2], 1);
         W += (int64_t)G.tx * G.ty * d[2];
+        planes += std::ceil((double)d[0] / TX) * std::ceil((double)d[1] / TY) * (double)d[2];
     }
     if (prec >= 0 && prec < 3 && solver >= 0 && solver < 2) {
         slab_init();
         const int t = g_slab[prec][solver][slab_class(W)].load(std::memory_order_relaxed);
         if (t > 0) {
-            if (solver != FAST_SOLVER_CG || g_slab_set[prec][solver].load(std::memory_order_relaxed)) return t;
+            // (The models count blocks in integers: a launch of more tile-planes
+            // than this fits no GPU, and gets the table's depth.)
+            if (solver != FAST_SOLVER_CG || g_slab_set[prec][solver].load(std::memory_order_relaxed) ||
+                planes > (double)INT32_MAX)
+                return t;
             const int width = launch_width(dims, solver);
             const int r = resident_depth(prec, dims, width, t);
             if (resident) *resident = r > 0;
