@@ -13,10 +13,16 @@ cubic volume and a number of right-hand sides) and each candidate depth it
 times two solves of a fixed number of iterations (tolerance far below
 reach, so every solve runs its iteration budget) and takes the difference,
 so allocation, the stencil-code pass, graph capture and the tau pass
-cancel and the per-iteration time remains.  Cases of one class are pooled
+cancel and the per-iteration time remains.  A candidate is timed as a table
+with that depth in every class runs, tiles included.  Cases of one class are pooled
 (time per voxel-iteration summed over the cases); a class without a case
 takes the depth of the nearest measured class.  A solve that stops before
 its budget (a diverging FP32 BiCGSTAB) leaves that depth unmeasured.
+
+With the built-in table a CG launch may take another depth, or all its
+iterations in one kernel (small F64 and F32 solves); an installed table turns
+both off for its precision and solver, so installing pays for BiCGSTAB, and
+for CG only where its depths beat the library's own choice.
 
     python -m fast_gb300.autotune             # measure and print the table
     python -m fast_gb300.autotune --install   # ... and use it in this process
@@ -25,6 +31,7 @@ its budget (a diverging FP32 BiCGSTAB) leaves that depth unmeasured.
 from __future__ import annotations
 
 import argparse
+import contextlib
 import ctypes as C
 import json
 import os
@@ -86,6 +93,20 @@ def rule_depth(shape, nrhs: int, precision: Precision, solver: DiffusionSolverTy
             os.environ["FAST_TAU_ZC"] = old
 
 
+@contextlib.contextmanager
+def _depth_everywhere(precision: Precision, solver: DiffusionSolverType, depth: int):
+    """Launches of this precision and solver at one depth; the built-in table
+    afterwards."""
+    old = os.environ.pop("FAST_TAU_ZC", None)
+    set_slab_table(precision, solver, [depth] * NUM_CLASSES)
+    try:
+        yield
+    finally:
+        set_slab_table(precision, solver, None)
+        if old is not None:
+            os.environ["FAST_TAU_ZC"] = old
+
+
 def _volume(edge: int, seed: int):
     from . import volumes
     return volumes.spheres((edge,) * 3, seed=seed, r_min=3.0, r_max=6.0, solid_fraction=0.5)
@@ -108,9 +129,7 @@ def _per_iteration_device(mask, dirs, prec, solver, depth, iters, repeats) -> Op
     long enough that the event bracketing of every launch costs nothing
     measurable while the allocation of their state would swamp a wall-clock
     difference."""
-    old = os.environ.get("FAST_TAU_ZC")
-    os.environ["FAST_TAU_ZC"] = str(depth)
-    try:
+    with _depth_everywhere(prec, solver, depth):
         p = TortuosityParams(tolerance=1e-30, max_iter=iters, precision=prec, profile=True)
         best = None
         for _ in range(repeats + 1):  # the first solve warms up
@@ -121,19 +140,12 @@ def _per_iteration_device(mask, dirs, prec, solver, depth, iters, repeats) -> Op
             v = sum(k["ms"] for name, k in ks.items() if name not in _SETUP_KERNELS) / 1e3 / iters
             best = v if best is None else min(best, v)
         return best
-    finally:
-        if old is None:
-            os.environ.pop("FAST_TAU_ZC", None)
-        else:
-            os.environ["FAST_TAU_ZC"] = old
 
 
 def _per_iteration(mask, dirs, prec, solver, depth, base_iters, span, repeats) -> Optional[float]:
     """Seconds per iteration of the launch at this depth (None if a solve
     stopped early)."""
-    old = os.environ.get("FAST_TAU_ZC")
-    os.environ["FAST_TAU_ZC"] = str(depth)
-    try:
+    with _depth_everywhere(prec, solver, depth):
         _timed(mask, dirs, prec, solver, base_iters)  # warm-up (pool, graph shapes)
         best = None
         for _ in range(repeats):
@@ -144,18 +156,14 @@ def _per_iteration(mask, dirs, prec, solver, depth, base_iters, span, repeats) -
             v = (t2 - t1) / span
             best = v if best is None else min(best, v)
         return best
-    finally:
-        if old is None:
-            os.environ.pop("FAST_TAU_ZC", None)
-        else:
-            os.environ["FAST_TAU_ZC"] = old
 
 
 def measure(cases: Sequence[Tuple[int, int]] = DEFAULT_CASES, precisions: Sequence[Precision] = PRECISIONS,
             solvers: Sequence[DiffusionSolverType] = SOLVERS, candidates: Sequence[int] = CANDIDATES,
             repeats: int = 2, target_s: float = 0.03, log=None) -> List[dict]:
     """Per-iteration times of every case, precision, solver and candidate
-    depth (depths above the volume's planes are skipped).  The iteration
+    depth (depths above the volume's planes are skipped).  Leaves the
+    built-in tables installed.  The iteration
     span of a case is sized so that it runs about target_s seconds.  Where
     an iteration takes more than DEVICE_TIMED_S the time is the kernels'
     own (CUDA events), else the wall-clock difference of two solves."""

@@ -88,7 +88,9 @@ typedef struct fast_tau_params {
 } fast_tau_params;
 
 /* fast_tau_params.flags: time every kernel launch of the solve with CUDA
- * events (launches are serialised and not graph-replayed while profiling). */
+ * events (launches are serialised and not graph-replayed while profiling; a
+ * small F64 or F32 CG, whose iterations otherwise run in one kernel, runs the
+ * two kernels of an iteration, with the same results). */
 #define FAST_FLAG_PROFILE 1
 /* MIXED only: keep the iterate as a float-float pair per voxel and evaluate
  * the replacement's b - A x with error-free FP32 transformations (about 48
@@ -245,7 +247,9 @@ FAST_API int fast_tau_last_stats(fast_tau_stats *out);
  * has fewer than 608 blocks); depth_by_class NULL restores the built-in
  * table, which fast_gb300/autotune.py writes from GB300 timings.  With the
  * built-in table a CG launch may take another depth than its class's, by a
- * model of how its blocks fill the GPU; an installed table is followed. */
+ * model of how its blocks fill the GPU, and a small F64 or F32 one runs all
+ * iterations in one kernel; an installed table is followed, and its launches
+ * run kernel by kernel (the tile's width stays the library's choice). */
 FAST_API int fast_tau_slab_depth(int64_t nx, int64_t ny, int64_t nz, int32_t nrhs, int32_t precision,
                                  int32_t solver, int32_t *depth, int32_t *size_class /* nullable */);
 FAST_API int fast_tau_set_slab_table(int32_t precision, int32_t solver, const int32_t *depth_by_class,
