@@ -127,9 +127,9 @@ static void dispatch(Step s, const Launch &L, cudaStream_t st)
         case Step::CG2_Q: pointwise_kernel<PwCG2<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
 #if FAST_TAU_TX == 64
         case Step::INIT_BI: go<OpInit<T, ST, true>>(L, st); break;
-        case Step::BI_RESTART: go<OpBiRestart<T, ST>>(L, st); break;
-        case Step::BI1: go<OpBi1<T, ST>>(L, st); break;
-        case Step::BI2: go<OpBi2<T, ST>>(L, st); break;
+        case Step::BI_RESTART: go<OpBiRestart<T>>(L, st); break;
+        case Step::BI1: go<OpBi1<T>>(L, st); break;
+        case Step::BI2: go<OpBi2<T>>(L, st); break;
         case Step::BI3: pointwise_kernel<PwBi3<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
 #endif
         default: break;
@@ -148,9 +148,9 @@ static cudaError_t configure()
     if constexpr (std::is_same<ST, float>::value) {
 #if FAST_TAU_TX == 64
         if ((r = cfg<OpInit<T, ST, true>>()) != cudaSuccess) e = r;
-        if ((r = cfg<OpBiRestart<T, ST>>()) != cudaSuccess) e = r;
-        if ((r = cfg<OpBi1<T, ST>>()) != cudaSuccess) e = r;
-        if ((r = cfg<OpBi2<T, ST>>()) != cudaSuccess) e = r;
+        if ((r = cfg<OpBiRestart<T>>()) != cudaSuccess) e = r;
+        if ((r = cfg<OpBi1<T>>()) != cudaSuccess) e = r;
+        if ((r = cfg<OpBi2<T>>()) != cudaSuccess) e = r;
 #endif
     }
     return e;

@@ -40,9 +40,9 @@ void Kernels<TX>::pure_f64(Step s, const Launch &L, cudaStream_t st)
     case Step::CG2_Q: pointwise_kernel<PwCG2<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
 #if FAST_TAU_TX == 64
     case Step::INIT_BI: go<OpInit<T, T, true>>(L, st); break;
-    case Step::BI_RESTART: go<OpBiRestart<T, T>>(L, st); break;
-    case Step::BI1: go<OpBi1<T, T>>(L, st); break;
-    case Step::BI2: go<OpBi2<T, T>>(L, st); break;
+    case Step::BI_RESTART: go<OpBiRestart<T>>(L, st); break;
+    case Step::BI1: go<OpBi1<T>>(L, st); break;
+    case Step::BI2: go<OpBi2<T>>(L, st); break;
     case Step::BI3: pointwise_kernel<PwBi3<T>, kPlanes><<<(unsigned)L.nblocks, NTHREADS, 0, st>>>(L); break;
 #endif
     default: break;  // replacement steps are MIXED-only (kern_misc.cu)
@@ -65,9 +65,9 @@ cudaError_t Kernels<TX>::configure_f64()
     if ((r = cfg<OpCG2<T, T>>()) != cudaSuccess) e = r;
 #if FAST_TAU_TX == 64
     if ((r = cfg<OpInit<T, T, true>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBiRestart<T, T>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi1<T, T>>()) != cudaSuccess) e = r;
-    if ((r = cfg<OpBi2<T, T>>()) != cudaSuccess) e = r;
+    if ((r = cfg<OpBiRestart<T>>()) != cudaSuccess) e = r;
+    if ((r = cfg<OpBi1<T>>()) != cudaSuccess) e = r;
+    if ((r = cfg<OpBi2<T>>()) != cudaSuccess) e = r;
 #endif
     if ((r = configure_resident<T>()) != cudaSuccess) e = r;
     return e;

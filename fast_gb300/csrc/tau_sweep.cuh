@@ -893,29 +893,6 @@ __device__ __forceinline__ void mixed_cg_finish(Scalars &sc, double rsq, double 
     mixed_request(sc, rsq);
 }
 
-__device__ __forceinline__ void mixed_bicg_finish(Scalars &sc, double r0r, double rsq)
-{
-    sc.rsq = rsq;
-    sc.iter += 1;
-    if (!(rsq <= sc.div_thresh)) {
-        sc.restarts += 1;
-        sc.replace = 2;
-        return;
-    }
-    const double rho_old = sc.rho;
-    sc.rho_old = rho_old;
-    sc.rho = r0r;
-    // The shadow residual r0 has become (numerically) orthogonal to r: in
-    // FP32, r0.r is noise well before |rho| reaches eps^2 |r0|^2.
-    if (fabs(r0r) < sc.eps2 * sc.r0_sq || r0r * r0r < sc.cos2_min * sc.r0_sq * rsq) {
-        sc.restarts += 1;
-        sc.replace = 2;
-        return;
-    }
-    sc.beta = (r0r / rho_old) * (sc.alpha / sc.omega);
-    mixed_request(sc, rsq);
-}
-
 // ===========================================================================
 // CG step 1: p <- z + beta p (z = r/diag on the fly), q = A p, dot p.q.
 // CG.cu:113-135 (z, beta, p update of the previous iteration) + :70-81.
@@ -1117,10 +1094,10 @@ struct OpCG2 {
 // residual is recomputed from x and becomes the new shadow residual.  Runs
 // as a no-op kernel unless a restart is pending.  Streams: x, code.
 // ===========================================================================
-template <typename TT, typename ST>
+template <typename TT>
 struct OpBiRestart {
     using T = TT;
-    static constexpr bool FB = sizeof(TT) == 4 && sizeof(ST) == 8;  // MIXED FP32 iterations
+    using ST = TT;
     using SL = Streams<sizeof(TT), 1>;
     static constexpr int NV = 1;
     static constexpr bool rare = true;
@@ -1159,7 +1136,7 @@ struct OpBiRestart {
     __device__ Out apply(const Geo &g, const Coef<T> &C, Shared &, const Own &o, const Pos &ps, T fc,
                          T fxp, T fxm, T fyp, T fym, T fzp, T fzm)
     {
-        const T d = diag_of<T, FB>(C, g, o.code, ps);
+        const T d = diag_of<T, false>(C, g, o.code, ps);
         const T ax = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
         const T res = rhs_at<T>(C, g, o.code, ps.x, ps.y, ps.z) - ax;
         rr.add_prod(res, res);
@@ -1187,10 +1164,10 @@ struct OpBiRestart {
 // BiCGSTAB step 1: p <- r + beta (p - w v), y = p/diag, v = A y, dot r0.v.
 // BICGSTAB.cu:112-147.  Streams: r, p_old, v_old, r0, code.
 // ===========================================================================
-template <typename TT, typename ST>
+template <typename TT>
 struct OpBi1 {
     using T = TT;
-    static constexpr bool FB = sizeof(TT) == 4 && sizeof(ST) == 8;  // MIXED FP32 iterations
+    using ST = TT;
     using SL = Streams<sizeof(TT), sizeof(TT), sizeof(TT), sizeof(TT), 1>;
     static constexpr uint32_t maps = map_bits(TM_R, TM_R + 1, TM_P, TM_P + 1, TM_V, TM_V + 1, TM_R0, TM_CODE);
     static constexpr int NV = 1;
@@ -1201,7 +1178,6 @@ struct OpBi1 {
     const CUtensorMap *tmap[SL::N];
     Faces<T> F;
     T *pnew, *vnew;
-    T *ezero;  // MIXED: e to zero after a residual replacement, else null
     T beta, nw;
     Acc<T> r0v;
 
@@ -1233,7 +1209,6 @@ struct OpBi1 {
         tmap[4] = &J.tm[TM_CODE];
         pnew = (T *)J.p[par ^ 1];
         vnew = (T *)J.v[par ^ 1];
-        ezero = J.sc->e_reset ? (T *)J.x : nullptr;
         beta = (T)J.sc->beta;
         nw = (T)(-J.sc->omega);
     }
@@ -1241,18 +1216,18 @@ struct OpBi1 {
     __device__ __forceinline__ T pval(const Vals &v) const { return beta * (v.p + nw * v.v) + v.r; }
     __device__ T field(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps) const
     {
-        return pval(v) * inv_of<T, FB>(C, g, v.code, ps);
+        return pval(v) * inv_of<T, false>(C, g, v.code, ps);
     }
     __device__ Own own(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps, T &f) const
     {
         const T pn = pval(v);
-        f = pn * inv_of<T, FB>(C, g, v.code, ps);
+        f = pn * inv_of<T, false>(C, g, v.code, ps);
         return Own{v.code, pn, v.r0};
     }
     __device__ Out apply(const Geo &g, const Coef<T> &C, Shared &, const Own &o, const Pos &ps, T fc,
                          T fxp, T fxm, T fyp, T fym, T fzp, T fzm)
     {
-        const T d = diag_of<T, FB>(C, g, o.code, ps);
+        const T d = diag_of<T, false>(C, g, o.code, ps);
         const T vn = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
         r0v.add_prod(o.r0, vn);
         return Out{o.p, vn};
@@ -1261,13 +1236,11 @@ struct OpBi1 {
     {
         store2<T>(pnew, i, a.p, b.p, v0, v1);
         store2<T>(vnew, i, a.v, b.v, v0, v1);
-        if (ezero) store2<T>(ezero, i, T(0), T(0), v0, v1);
     }
     __device__ void partials(T (&v)[NV]) const { v[0] = r0v.hi(); }
     __device__ static void finish(Scalars &sc, const double (&t)[NV])
     {
         sc.alpha = (double)((ST)sc.rho / (ST)t[0]);  // BICGSTAB.cu:147
-        sc.e_reset = 0;
     }
 };
 
@@ -1276,10 +1249,10 @@ struct OpBi1 {
 // t.t.  BICGSTAB.cu:149-183.  Streams: r, v_new, code.  Step 3 is pointwise
 // (tau_pointwise.cuh).
 // ===========================================================================
-template <typename TT, typename ST>
+template <typename TT>
 struct OpBi2 {
     using T = TT;
-    static constexpr bool FB = sizeof(TT) == 4 && sizeof(ST) == 8;  // MIXED FP32 iterations
+    using ST = TT;
     using SL = Streams<sizeof(TT), sizeof(TT), 1>;
     static constexpr uint32_t maps = map_bits(TM_R, TM_R + 1, TM_V, TM_V + 1, TM_CODE);
     static constexpr int NV = 2;
@@ -1320,18 +1293,18 @@ struct OpBi2 {
     __device__ __forceinline__ T sval(const Vals &v) const { return v.r + nalpha * v.v; }  // s = r + (-alpha) v
     __device__ T field(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps) const
     {
-        return sval(v) * inv_of<T, FB>(C, g, v.code, ps);
+        return sval(v) * inv_of<T, false>(C, g, v.code, ps);
     }
     __device__ Own own(const Geo &g, const Coef<T> &C, Shared &, const Vals &v, const Pos &ps, T &f) const
     {
         const T s = sval(v);
-        f = s * inv_of<T, FB>(C, g, v.code, ps);
+        f = s * inv_of<T, false>(C, g, v.code, ps);
         return Own{v.code, s};
     }
     __device__ Out apply(const Geo &g, const Coef<T> &C, Shared &, const Own &o, const Pos &ps, T fc,
                          T fxp, T fxm, T fyp, T fym, T fzp, T fzm)
     {
-        const T d = diag_of<T, FB>(C, g, o.code, ps);
+        const T d = diag_of<T, false>(C, g, o.code, ps);
         const T t = stencil7<T>(F, o.code, fc, fxp, fxm, fyp, fym, fzp, fzm, d);
         ts.add_prod(t, o.s);
         tt.add_prod(t, t);
