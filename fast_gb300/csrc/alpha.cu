@@ -56,7 +56,6 @@
 
 #include "ccl_faces.h"
 #include "fasttau.h"
-#include "fp_convert.h"
 #include "tau_errors.h"
 
 namespace {
@@ -342,8 +341,8 @@ constexpr int QCAP = 4096;  // cells in the queue at once
 // fixed order.  A cell's triangles are fans: a thread keeps the fan's first
 // and last vertex and makes one new vertex per triangle.  Areas add in double
 // at every level: about two FP64 additions per cut cell beside some hundreds of
-// other instructions (512^3, seven fields, with the labelling: 1.88 ms, and
-// 1.87 with float pairs instead).
+// other instructions (512^3, seven fields, with the labelling: 1.86 ms, and 1.87
+// with float pairs, or with the conversion done in integer instructions).
 //
 // Bound by instruction issue (384^3: 74 % of the slots busy, DRAM 6 %); most
 // of it is the cut cells' vertices and areas.  Against summing every cell's
@@ -541,7 +540,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
                     }
                     const float3 v1 = v2;
                     v2 = vertex(C, s_t, s_edge, e);
-                    acc += ft::widen_f(triangle_area(v0, v1, v2));
+                    acc += (double)triangle_area(v0, v1, v2);
                 }
             }
             __syncthreads();
