@@ -689,9 +689,9 @@ int label_common(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint
     A.nx = (int)(nx > 1 ? nx : ny);
     A.ny = (int)(nx > 1 ? ny : nz);
     A.nz = (int)(nx > 1 ? nz : 1);
-    A.wx = (A.nx + 63) / 64;
-    A.by = (A.ny + RY - 1) / RY;
-    A.bz = (A.nz + RZ - 1) / RZ;
+    A.wx = (int)(((int64_t)A.nx + 63) / 64);
+    A.by = (int)(((int64_t)A.ny + RY - 1) / RY);
+    A.bz = (int)(((int64_t)A.nz + RZ - 1) / RZ);
     A.slots = A.nx >= 64 ? kSlots : (A.nx + 1) / 2;
     A.bg = bg;
     A.mask = d_mask;
