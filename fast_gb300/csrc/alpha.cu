@@ -383,7 +383,11 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
     // Voxel rows as bits: one warp per row, bit b = the voxel at x = i0 - 1 + b
     // (clamped to the volume, as y and z).
     const int rows = VY * (nzc + 2);
-    const int x0 = min(max(i0 - 1 + lane, 0), A.nx - 1), x1 = min(i0 + 31 + lane, A.nx - 1);
+    // Coordinates before the clamp go past 2^31 on the longest axes: unsigned.
+    auto clamped = [](int at, int plus, int n) {  // at - 1 + plus in [0, n)
+        return (int)min(max((unsigned)at + (unsigned)plus, 1u) - 1u, (unsigned)(n - 1));
+    };
+    const int x0 = clamped(i0, lane, A.nx), x1 = clamped(i0, 32 + lane, A.nx);
     bool bad = false;
     constexpr int U = LABELS ? 3 : 6;  // rows in flight per warp
     for (int r0 = warp; r0 < rows; r0 += (NT / 32) * U) {
@@ -392,7 +396,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
         for (int u = 0; u < U; u++) {
             const int r = min(r0 + u * (NT / 32), rows - 1);
             const int zz = r / VY, yy = r - zz * VY;
-            const int gz = min(max(k0 - 1 + zz, 0), A.nz - 1), gy = min(max(j0 - 1 + yy, 0), A.ny - 1);
+            const int gz = clamped(k0, zz, A.nz), gy = clamped(j0, yy, A.ny);
             const int64_t base = ((int64_t)gz * A.ny + gy) * A.nx;
             m[u][0] = __ldg(A.mask + base + x0);
             m[u][1] = __ldg(A.mask + base + x1);
@@ -471,7 +475,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
         // One row of cells per thread: those with corners on both sides.
         const int k = tid / BY, j = tid - k * BY;
         uint64_t cut = 0;
-        if (k < nzc && j0 + j < A.ny) {
+        if (k < nzc && j < A.ny - j0) {
             const int nc = min(BX, A.nx - i0);
             uint64_t any = 0, all = ~0ull;
 #pragma unroll
