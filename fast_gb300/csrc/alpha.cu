@@ -349,9 +349,11 @@ constexpr int QCAP = 4096;  // cells in the queue at once
 // corners as one 4-bit lane per field and queueing triangles: 512^3 spheres
 // 7.40 -> 1.03 ms for the seven fields, 1024^3 58.6 -> 8.3; 200 x 181 x 190
 // one field 146 -> 69 us.  U rows in flight hide the loads; more cost
-// registers and so blocks per SM.
+// registers and so blocks per SM: five fit by their shared memory, and the
+// bound keeps the registers of the seven-field pass to 46 (it took 57, and
+// 4 % more time at 512^3, when left to the compiler).
 template <bool LABELS>
-__global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
+__global__ void __launch_bounds__(NT, 5) alpha_kernel(AlphaArgs A)
 {
     constexpr int NF = LABELS ? kFields : 1;
     __shared__ uint64_t s_v[NF][VROWS];
@@ -383,11 +385,10 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
     // Voxel rows as bits: one warp per row, bit b = the voxel at x = i0 - 1 + b
     // (clamped to the volume, as y and z).
     const int rows = VY * (nzc + 2);
-    // Coordinates before the clamp go past 2^31 on the longest axes: unsigned.
-    auto clamped = [](int at, int plus, int n) {  // at - 1 + plus in [0, n)
-        return (int)min(max((unsigned)at + (unsigned)plus, 1u) - 1u, (unsigned)(n - 1));
-    };
-    const int x0 = clamped(i0, lane, A.nx), x1 = clamped(i0, 32 + lane, A.nx);
+    // The clamps are on the offset from the voxel before the brick: on the
+    // longest axes the coordinate itself leaves 32 bits before a clamp.
+    auto clamped = [](int plus, int at, int n) { return min(max(plus, at == 0 ? 1 : 0), n - at); };
+    const int x0 = i0 - 1 + clamped(lane, i0, A.nx), x1 = i0 - 1 + clamped(32 + lane, i0, A.nx);
     bool bad = false;
     constexpr int U = LABELS ? 3 : 6;  // rows in flight per warp
     for (int r0 = warp; r0 < rows; r0 += (NT / 32) * U) {
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(NT) alpha_kernel(AlphaArgs A)
         for (int u = 0; u < U; u++) {
             const int r = min(r0 + u * (NT / 32), rows - 1);
             const int zz = r / VY, yy = r - zz * VY;
-            const int gz = clamped(k0, zz, A.nz), gy = clamped(j0, yy, A.ny);
+            const int gz = k0 - 1 + clamped(zz, k0, A.nz), gy = j0 - 1 + clamped(yy, j0, A.ny);
             const int64_t base = ((int64_t)gz * A.ny + gy) * A.nx;
             m[u][0] = __ldg(A.mask + base + x0);
             m[u][1] = __ldg(A.mask + base + x1);
