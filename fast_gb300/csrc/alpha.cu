@@ -340,11 +340,11 @@ constexpr int QCAP = 4096;  // cells in the queue at once
 // block-wide scan and item q is done by thread q mod NT, so every sum has a
 // fixed order.  A cell's triangles are fans: a thread keeps the fan's first
 // and last vertex and makes one new vertex per triangle.  Areas add in double
-// at every level: about two FP64 additions per cut cell beside some hundreds of
-// other instructions (512^3, seven fields, with the labelling: 1.86 ms, and 1.87
-// with float pairs, or with the conversion done in integer instructions).
+// at every level, which keeps the FP64 pipe half busy beside the other
+// instructions (512^3, seven fields, with the labelling: 1.86 ms, and 1.87 with
+// float pairs, or with the conversion done in integer instructions).
 //
-// Bound by instruction issue (384^3: 74 % of the slots busy, DRAM 6 %); most
+// Bound by instruction issue (384^3: 80 % of the slots busy, DRAM 7 %); most
 // of it is the cut cells' vertices and areas.  Against summing every cell's
 // corners as one 4-bit lane per field and queueing triangles: 512^3 spheres
 // 7.40 -> 1.03 ms for the seven fields, 1024^3 58.6 -> 8.3; 200 x 181 x 190
@@ -608,8 +608,11 @@ int area_device(const uint8_t *d_mask, const uint32_t *d_labels, const uint8_t *
     A.tiles_x = (int)((nx + BX - 1) / BX);
     A.tiles_y = (int)((ny + BY - 1) / BY);
     // Bricks 16 cells deep, halved while the grid has fewer than 6 blocks per
-    // SM: 200 x 181 x 190 92 us at 6, 99 at 8 (half as deep), 104 at 3 (twice);
-    // the other sizes from 64^3 to 512^3 differ by 2 %.
+    // SM.  Of 2, 3, 4, 6, 8 and 12 at eleven sizes from 48^3 to 256^3, one field
+    // and the tensor call, each of the others is 10 % or more behind somewhere
+    // (2: 239 against 210 us at 97 x 300 x 150; 3 and 4: 283 against 252 at 190 x
+    // 181 x 200, both tensors; 8 and 12: 79 against 70 at 160^3, one field), 6 at
+    // 128^3 with one field alone (67 against 60 at 3).
     int sms = 152, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t xy = (int64_t)A.tiles_x * A.tiles_y;

@@ -642,7 +642,7 @@ double modelled_us(const DepthModel &M, const std::vector<const int64_t *> &dims
 // Without the margin the means are a little higher and the worst 0.91x: near
 // equal predictions are not worth following.
 //
-// One right-hand side of a MIXED solve is what the serving context runs
+// One right-hand side of a MIXED solve is what the serving context mostly runs
 // beside others, at the depth it has alone: there it takes no less than three
 // quarters of the table's depth, since shallow slabs that fill an idle GPU
 // only read more halo planes on a busy one.  (No MIXED launch takes a single
@@ -716,6 +716,15 @@ int resident_depth(int prec, const std::vector<const int64_t *> &dims, int width
 
 // The depth of a launch of right-hand sides with dimensions dims; resident =
 // it is that of a solve in one kernel.
+//
+// The serving context takes the depth of each request alone, the one-kernel
+// solve's included although it runs the sweeps: the depth sets the order of the
+// sums, and a served result equals the request alone.  Depths that fill an idle
+// GPU cost a full one halo planes: 256 requests of 24^3 in F64 take 124 ms at the
+// one plane they have alone and 84 at the table's two (212 with the sweeps
+// before the face tables), 32 of 128^3 in F32 191 at 7 planes and 146 at 16 (202 before).
+// Alone the table's depths are what is slower: 128^3 F32 8.9 against 7.8 ms, 160^3
+// 16.9 against 13.2.
 int tuned_depth(int prec, int solver, const std::vector<const int64_t *> &dims, bool *resident = nullptr)
 {
     if (resident) *resident = false;
