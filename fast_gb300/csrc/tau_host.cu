@@ -998,12 +998,14 @@ int solve_jobs(Engine &E, const std::vector<VolSpec> &vols, const std::vector<Jo
 
     // F64 / F32 CG keeps q = A p between its steps where the extra vector
     // fits beside everything else; a volume that fills the GPU evaluates the
-    // product twice instead (the same results).
+    // product twice instead (the same results).  Where a second solve of this
+    // size fits (another thread's), q leaves room for it.
     Arena A;
     bool store_q = !mixed && solver == FAST_SOLVER_CG && !resident;
     if (store_q) {
         const size_t more = solve_bytes(vols, jobs, prec, solver, zc, width, true);
-        store_q = more <= avail && cudaMallocAsync((void **)&A.base, more, st) == cudaSuccess;
+        store_q = more <= avail && (more + need <= avail || need > avail - need) &&
+                  cudaMallocAsync((void **)&A.base, more, st) == cudaSuccess;
         if (store_q) need = more;
         else cudaGetLastError();
     }

@@ -95,6 +95,28 @@ def test_stored_product_against_evaluated_again(gpu, tmp_path):
         assert (stored["tau"], stored["iters"]) == (again["tau"], again["iters"]), shape
 
 
+BESIDE = r"""
+shape = (72, 70, 130)
+m = mask(shape)
+nz, ny, nx = shape
+voxels = (nx + 15) // 16 * 16 * ny * nz
+need = voxels * 33  # four vectors and the codes, and 4 % for all else
+q = voxels * 8
+out = [q]
+for free in (1.04 * need + q, 2.08 * need + q / 2, 2.08 * need + 1.1 * q):
+    out.append(solve(m, ft.Dir.Y_POS, ft.Precision.F64, {"FAST_TAU_TEST_FREE_BYTES": str(int(free))}))
+print(json.dumps(out))
+"""
+
+
+def test_stored_product_leaves_room_for_a_second_solve(gpu, tmp_path):
+    """No second solve of the size fits; one fits beside the plain plan alone;
+    one fits beside q too."""
+    q, filled, beside, roomy = _run(BESIDE, _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1"))
+    assert filled["memory"] == roomy["memory"] >= beside["memory"] + q
+    assert filled["tau"] == beside["tau"] == roomy["tau"]
+
+
 TILES = r"""
 out = []
 for shape in NARROW:
