@@ -291,8 +291,9 @@ FAST_API int fast_ccl_label(const uint8_t *mask, int64_t nx, int64_t ny, int64_t
                             uint32_t *labels, uint32_t *num_labels, uint8_t *boundary, uint64_t boundary_cap);
 
 /* The same on a DEVICE mask, labels written to DEVICE memory d_labels
- * (nx*ny*nz uint32); boundary stays a host buffer.  stream: a cudaStream_t
- * as void*, NULL = the legacy default stream; the call synchronises it. */
+ * (nx*ny*nz uint32; the mask may lie inside that memory); boundary stays a
+ * host buffer.  stream: a cudaStream_t as void*, NULL = the legacy default
+ * stream; the call synchronises it. */
 FAST_API int fast_ccl_label_device(const uint8_t *d_mask, int64_t nx, int64_t ny, int64_t nz, uint8_t background,
                                    uint32_t *d_labels, uint32_t *num_labels, uint8_t *boundary,
                                    uint64_t boundary_cap, void *stream);

@@ -93,9 +93,14 @@ print(json.dumps(out))
 """
 
 
-def test_missing_partial_sum_times_out(gpu, tmp_path):
-    lib = _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1 -DFAST_TAU_WAIT_LIMIT_NS=50000000ull")
-    for before, armed, after, sweeps in _run(lib, SILENT).values():
+@pytest.fixture(scope="module")
+def hooked_lib(tmp_path_factory):
+    return _build(str(tmp_path_factory.mktemp("hooks")),
+                  "-DFAST_TAU_TEST_HOOKS=1 -DFAST_TAU_WAIT_LIMIT_NS=50000000ull")
+
+
+def test_missing_partial_sum_times_out(gpu, hooked_lib):
+    for before, armed, after, sweeps in _run(hooked_lib, SILENT).values():
         assert before[0] == after[0] == OK and before[1] == after[1]
         assert before[2] < sweeps[2]  # one kernel ran the iterations
         assert armed[0] == TIMEOUT and "wait ran out" in armed[3] and "tile" not in armed[3]
@@ -127,9 +132,8 @@ print(json.dumps(out))
 """
 
 
-def test_refused_launch_runs_the_sweeps(gpu, tmp_path):
-    lib = _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1")
-    for kernel, refused, few_sms, sweeps, after in _run(lib, REFUSED).values():
+def test_refused_launch_runs_the_sweeps(gpu, hooked_lib):
+    for kernel, refused, few_sms, sweeps, after in _run(hooked_lib, REFUSED).values():
         assert all(r[0] == OK for r in (kernel, refused, few_sms, sweeps, after))
         assert kernel[1] == refused[1] == after[1]
         assert refused[1] == sweeps[1]

@@ -72,6 +72,11 @@ def _run(body, lib=None):
     return json.loads(r.stdout.strip().splitlines()[-1])
 
 
+@pytest.fixture(scope="module")
+def hooked_lib(tmp_path_factory):
+    return _build(str(tmp_path_factory.mktemp("hooks")), "-DFAST_TAU_TEST_HOOKS=1")
+
+
 STORED = r"""
 out = []
 for shape in NARROW + WIDE:
@@ -87,8 +92,8 @@ print(json.dumps(out))
 """
 
 
-def test_stored_product_against_evaluated_again(gpu, tmp_path):
-    for shape, q, stored, again in _run(STORED, _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1")):
+def test_stored_product_against_evaluated_again(gpu, hooked_lib):
+    for shape, q, stored, again in _run(STORED, hooked_lib):
         assert stored["status"] == again["status"] == 0
         assert stored["cg1"] >= stored["iters"] and stored["cg2"] >= stored["iters"]  # sweeps
         assert stored["memory"] - again["memory"] >= q  # q was there, and was not
@@ -109,10 +114,10 @@ print(json.dumps(out))
 """
 
 
-def test_stored_product_leaves_room_for_a_second_solve(gpu, tmp_path):
+def test_stored_product_leaves_room_for_a_second_solve(gpu, hooked_lib):
     """No second solve of the size fits; one fits beside the plain plan alone;
     one fits beside q too."""
-    q, filled, beside, roomy = _run(BESIDE, _build(str(tmp_path), "-DFAST_TAU_TEST_HOOKS=1"))
+    q, filled, beside, roomy = _run(BESIDE, hooked_lib)
     assert filled["memory"] == roomy["memory"] >= beside["memory"] + q
     assert filled["tau"] == beside["tau"] == roomy["tau"]
 
